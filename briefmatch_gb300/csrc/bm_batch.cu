@@ -159,7 +159,8 @@ __global__ void __launch_bounds__(256) k_b_upsample(BatchDev bd, int which)
         upsample_px<uint8_t>(P.frame[which], P.up, P.sx_in, P.sy_in, P.sx, P.lx, P.ix, P.ly, P.iy, x, y);
 }
 
-// Tile `tile` of the up-sampled grids, visited in reverse order when rev is set.
+// Pair and pixel of this thread in tile `tile` of the up-sampled grids; false where
+// the pixel lies outside its pair's grid (the pair is the block's all the same).
 __device__ __forceinline__ bool up_tile(const BatchDev& bd, unsigned int tile, int& i, int& x, int& y)
 {
     i = find_pair(bd.pre_up, bd.lo, bd.hi, tile);
@@ -187,11 +188,11 @@ __global__ void __launch_bounds__(256) k_b_jump(BatchDev bd, int cur, int p, int
     const unsigned int base = bd.pre_up[bd.lo], total = bd.pre_up[bd.hi] - base;
     const unsigned int tile = base + (rev ? total - 1 - blockIdx.x : blockIdx.x);
     int i, x, y;
-    if (!up_tile(bd, tile, i, x, y)) return;
+    up_tile(bd, tile, i, x, y);
     const PairDev& P = bd.pairs[i];
     RsArgs r = rs;
     r.dist = P.dist;
-    jump_px<NSP, RS>(P.F[0], P.F[1], P.flow[cur], P.flow[cur ^ 1], P.cost, P.sx, P.sy, p, pd, doubleProp, r, x, y);
+    jump_level_px<NSP, RS>(P.F[0], P.F[1], P.flow[cur], P.flow[cur ^ 1], P.cost, P.sx, P.sy, p, pd, doubleProp, r, x, y);
 }
 
 struct MatchPlan {
@@ -235,15 +236,15 @@ __global__ void __launch_bounds__(256) k_b_match_persistent(BatchDev bd, MatchPl
             for (unsigned int k = blockIdx.x; k < total; k += gridDim.x) {
                 const unsigned int tile = base + (rev ? total - 1 - k : k);
                 int i, x, y;
-                if (!up_tile(bd, tile, i, x, y)) continue;
+                up_tile(bd, tile, i, x, y);
                 const PairDev& P = bd.pairs[i];
                 rs.dist = P.dist;
                 if (last)
-                    jump_px<NSP, true, true>(P.F[0], P.F[1], P.flow[cur], P.flow[cur ^ 1], P.cost, P.sx, P.sy, s, pd,
-                                             plan.doubleProp, rs, x, y);
+                    jump_level_px<NSP, true, true>(P.F[0], P.F[1], P.flow[cur], P.flow[cur ^ 1], P.cost, P.sx, P.sy, s,
+                                                   pd, plan.doubleProp, rs, x, y);
                 else
-                    jump_px<NSP, false, true>(P.F[0], P.F[1], P.flow[cur], P.flow[cur ^ 1], P.cost, P.sx, P.sy, s,
-                                              pd, plan.doubleProp, rs, x, y);
+                    jump_level_px<NSP, false, true>(P.F[0], P.F[1], P.flow[cur], P.flow[cur ^ 1], P.cost, P.sx, P.sy, s,
+                                                    pd, plan.doubleProp, rs, x, y);
             }
             cur ^= 1;
             if (!grid_sync(gs, gridDim.x, plan.spin_limit, ++phase)) return;

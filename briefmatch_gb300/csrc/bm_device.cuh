@@ -77,17 +77,23 @@ __device__ __forceinline__ void rs_normals(const RsArgs& rs, unsigned int id, fl
         n2 = v.y;
     } else {
         // The reference state: curand_init(id, 0, 0) (briefmatch_cuda.cu:57) advanced by
-        // two uniforms per earlier call (two curand_normal per call, :240-241).
-        curandStateXORWOW_t st;
-        curand_init((unsigned long long)id, 0ull, 0ull, &st);
-        unsigned long long skip = 2ull * rs.call;
+        // two uniforms per earlier call (two curand_normal per call, :240-241).  Each
+        // branch has a state of its own: skipahead takes its state's address, which
+        // would keep a shared one in local memory through every step of the loop.
+        const unsigned long long skip = 2ull * rs.call;
         if (skip <= 512ull) {
-            for (unsigned long long k = 0; k < skip; k++) (void)curand(&st);
+            curandStateXORWOW_t st;
+            curand_init((unsigned long long)id, 0ull, 0ull, &st);
+            for (unsigned int k = 0; k < (unsigned int)skip; k++) (void)curand(&st);
+            n1 = curand_normal(&st);
+            n2 = curand_normal(&st);
         } else {
+            curandStateXORWOW_t st;
+            curand_init((unsigned long long)id, 0ull, 0ull, &st);
             skipahead(skip, &st);
+            n1 = curand_normal(&st);
+            n2 = curand_normal(&st);
         }
-        n1 = curand_normal(&st);
-        n2 = curand_normal(&st);
     }
 }
 
@@ -393,31 +399,73 @@ __device__ __forceinline__ uint32_t field_load(const uint32_t* p)
         return __ldg(p);
 }
 
-template <int NSP, bool RS, bool INLAUNCH = false>
-__device__ __forceinline__ void jump_px(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
-                                        const uint32_t* flow_in, uint32_t* flow_out, uint16_t* cost, int sx, int sy,
-                                        int p, int pd, int doubleProp, const RsArgs& rs, int x, int y)
+// Linear offsets of a level's neighbours, down a column (v) and along a row (h), for
+// d = +1 (d = -1 negates them).  An offset of n = sx * sy or more leaves the plane
+// from every pixel; it is held at n, so that pixel + offset fits 32 bits
+// (n <= 32767^2).
+struct JumpStep {
+    int v, h;
+};
+__device__ __forceinline__ JumpStep jump_step(int sx, int sy, int p, int pd)
+{
+    const long n = (long)sx * sy;
+    const long h = (long)pd * p, v = h * sx;
+    return {(int)max(-n, min(n, v)), (int)max(-n, min(n, h))};
+}
+
+// A register with no defined value and no instruction to define it: the words of a
+// gather whose predicate is off are never looked at.
+__device__ __forceinline__ uint32_t undefined_word()
+{
+    uint32_t r;
+    asm("" : "=r"(r));
+    return r;
+}
+
+// 16 bytes of a descriptor, read only when `pred` holds (undefined words otherwise).
+__device__ __forceinline__ uint4 gather16_pred(const uint32_t* __restrict__ src, bool pred)
+{
+    uint4 w = make_uint4(undefined_word(), undefined_word(), undefined_word(), undefined_word());
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t@p ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%5];\n\t}"
+        : "+r"(w.x), "+r"(w.y), "+r"(w.z), "+r"(w.w)
+        : "r"(pred ? 1 : 0), "l"(src));
+    return w;
+}
+
+// The same for data read once (evict-first), as load_desc_stream.
+__device__ __forceinline__ uint4 stream16_pred(const uint32_t* __restrict__ src, bool pred)
+{
+    uint4 w = make_uint4(undefined_word(), undefined_word(), undefined_word(), undefined_word());
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t@p ld.global.cs.v4.u32 {%0, %1, %2, %3}, [%5];\n\t}"
+        : "+r"(w.x), "+r"(w.y), "+r"(w.z), "+r"(w.w)
+        : "r"(pred ? 1 : 0), "l"(src));
+    return w;
+}
+
+__device__ __forceinline__ int hamming16(const uint4& a, const uint4& b)
+{
+    return __popc(a.x ^ b.x) + __popc(a.y ^ b.y) + __popc(a.z ^ b.z) + __popc(a.w ^ b.w);
+}
+
+// Candidates of a level for one pixel: the four neighbours' vectors (0 outside the
+// plane), clamped into the image two components at a time (16-bit pairs), and the
+// random-search candidate.  A candidate equal to `own` or to an earlier one is not
+// live; with doubleProp off the d = -1 neighbours become `own`.
+template <bool RS, bool INLAUNCH>
+__device__ __forceinline__ void jump_candidates(const uint32_t* flow_in, uint32_t own, int sx, int sy, JumpStep js,
+                                                int doubleProp, const RsArgs& rs, int x, int y, int pix,
+                                                uint32_t (&cand)[RS ? 5 : 4], bool (&live)[RS ? 5 : 4])
 {
     constexpr int NC = RS ? 5 : 4;
-    const long n = (long)sx * sy;
-    const long pix = x + (long)y * sx;
-    const uint32_t own = field_load<INLAUNCH>(flow_in + pix);
-    const int h0 = INLAUNCH ? (int)__ldcg(cost + pix) : (int)cost[pix];
-
-    uint32_t cand[NC];
-    bool live[NC];
+    const unsigned int n = (unsigned int)(sx * sy);
+    const uint32_t lo = pack_flow(-x, -y), hi = pack_flow(sx - x - 1, sy - y - 1);
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-        const int d = (c < 2) ? -1 : 1;
-        const int xy = c & 1;
-        const bool active = d > 0 || doubleProp;
-        const long doff = xy ? (long)pd * p * d : (long)sx * pd * p * d;
-        const long q = pix + doff;
-        const uint32_t nb = (active && q >= 0 && q < n) ? field_load<INLAUNCH>(flow_in + q) : 0u;
-        const int nx = min(max(lo16(nb), -x), sx - x - 1);
-        const int ny = min(max(hi16(nb), -y), sy - y - 1);
-        cand[c] = pack_flow(nx, ny);
-        live[c] = active;
+        const int off = (c & 1) ? js.h : js.v;
+        const int q = pix + (c < 2 ? -off : off);
+        const bool active = c >= 2 || doubleProp;
+        const uint32_t nb = (active && (unsigned int)q < n) ? field_load<INLAUNCH>(flow_in + q) : 0u;
+        cand[c] = active ? __vmaxs2(__vmins2(nb, hi), lo) : own;
     }
     if constexpr (RS) {
         float n1, n2;
@@ -425,43 +473,185 @@ __device__ __forceinline__ void jump_px(const uint32_t* __restrict__ F1, const u
         const int nx = min(max((int)round(rs.dist * n1), -x), sx - x - 1);
         const int ny = min(max((int)round(rs.dist * n2), -y), sy - y - 1);
         cand[NC - 1] = pack_flow(nx, ny);
-        live[NC - 1] = true;
     }
 #pragma unroll
     for (int c = 0; c < NC; c++) {
         bool dup = cand[c] == own;
 #pragma unroll
-        for (int k = 0; k < c; k++) dup = dup || (live[k] && cand[k] == cand[c]);
-        live[c] = live[c] && !dup;
+        for (int k = 0; k < c; k++) dup = dup || cand[k] == cand[c];
+        live[c] = !dup;
     }
+}
 
-    uint32_t f1[NSP];
-    load_desc_stream<NSP>(f1, F1 + pix * NSP);
-    // predicated gathers, all in flight at once
-    uint32_t g[NC][NSP];
+// Descriptors of up to 16 bytes: one thread reads its pixel's descriptor and its
+// candidates' whole; a thread without a live candidate reads none.  The level is bound
+// by the L1 data pipe (a gather of 32 scattered 16-byte vectors takes ~18 wavefronts)
+// with the integer pipe next to it: 32-bit indices, clamps on 16-bit pairs and gathers
+// without zero-fill took the integer pipe from 74 % to 52 % and a level at 1024x436
+// u2.9 N128 from 42.0 to 36.8 us (67.1 to 56.9 with the random search, whose state
+// now stays in registers).
+template <int NSP, bool RS, bool INLAUNCH = false>
+__device__ __forceinline__ void jump_px(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
+                                        const uint32_t* flow_in, uint32_t* flow_out, uint16_t* cost, int sx, int sy,
+                                        JumpStep js, int doubleProp, const RsArgs& rs, int x, int y)
+{
+    static_assert(NSP <= 4, "longer descriptors go through jump_row");
+    constexpr int NC = RS ? 5 : 4;
+    const int pix = x + y * sx;
+    const uint32_t own = field_load<INLAUNCH>(flow_in + pix);
+    uint32_t cand[NC];
+    bool live[NC];
+    jump_candidates<RS, INLAUNCH>(flow_in, own, sx, sy, js, doubleProp, rs, x, y, pix, cand, live);
+    bool any = live[0];
 #pragma unroll
-    for (int c = 0; c < NC; c++) {
-        const long t = pix + lo16(cand[c]) + (long)hi16(cand[c]) * sx;
-        gather_desc_pred<NSP>(g[c], F2 + t * NSP, live[c]);
-    }
-    int hc[NC];
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-        int acc = 0;
-#pragma unroll
-        for (int k = 0; k < NSP; k++) acc += __popc(f1[k] ^ g[c][k]);
-        hc[c] = live[c] ? acc : 0x7fffffff;
-    }
-    int h = h0;
+    for (int c = 1; c < NC; c++) any = any || live[c];
     uint32_t best = own;
+    if (any) {
+        const int h0 = INLAUNCH ? (int)__ldcg(cost + pix) : (int)cost[pix];
+        uint32_t f1[NSP];
+        load_desc_stream<NSP>(f1, F1 + (size_t)(unsigned int)pix * NSP);
+        // predicated gathers, all in flight at once
+        uint32_t g[NC][NSP];
 #pragma unroll
-    for (int c = 0; c < NC; c++)
-        if (hc[c] < h) {
-            h = hc[c];
-            best = cand[c];
+        for (int c = 0; c < NC; c++) {
+            const int t = pix + lo16(cand[c]) + hi16(cand[c]) * sx;
+            gather_desc_pred<NSP>(g[c], F2 + (size_t)(unsigned int)t * NSP, live[c]);
         }
+        int h = h0;
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            int acc = 0;
+#pragma unroll
+            for (int k = 0; k < NSP; k++) acc += __popc(f1[k] ^ g[c][k]);
+            if (live[c] && acc < h) {
+                h = acc;
+                best = cand[c];
+            }
+        }
+        if (h != h0) cost[pix] = (uint16_t)h;
+    }
     flow_out[pix] = best;
-    if (h != h0) cost[pix] = (uint16_t)h;
+}
+
+// Descriptors of 32 or 64 bytes: a warp takes 32 consecutive pixels of a row (lane =
+// pixel for the candidates and the decision) and reads descriptors L = NSP / 4 lanes
+// to one, 16 bytes each, so that one load instruction covers 32 / L whole descriptors
+// in consecutive sectors.  One lane reading a 64-byte descriptor alone touches a line
+// of its own with every 16-byte load: at N = 512 that kept the L1 data pipe 91 % busy
+// with HBM at 52 % (3136x1764 pixels, 249 us under ncu); this form is bound by HBM
+// (the same level in the engine: 132 us, 116 us at the measured copy bandwidth for its
+// 140 bytes per pixel; the whole 1920x1080 u4.9 N512 pair 56.8 -> 47.2 ms).  Step s serves pixels s * (32 / L) ...; each lane's partial distances
+// of the L steps are summed over the L lanes by a reduce-scatter that leaves step k's
+// sums with the group's lane k, and one shuffle hands them to the pixel's lane.  All
+// 32 lanes take part; `valid` says which pixels lie in the image (x, y are then theirs).
+template <int NSP, bool RS, bool INLAUNCH = false>
+__device__ __forceinline__ void jump_row(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
+                                         const uint32_t* flow_in, uint32_t* flow_out, uint16_t* cost, int sx, int sy,
+                                         JumpStep js, int doubleProp, const RsArgs& rs, int x, int y, bool valid)
+{
+    static_assert(NSP == 8 || NSP == 16, "two or four lanes per descriptor");
+    constexpr int NC = RS ? 5 : 4;
+    constexpr int L = NSP / 4;      // lanes per descriptor
+    constexpr int PPS = 32 / L;     // pixels per step
+    constexpr int NP = (NC + 1) / 2;  // packed pairs of distances (each at most 512)
+    const unsigned int FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int pix = x + y * sx;
+    uint32_t own = 0, cand[NC];
+    int h0 = 0;
+    int t[NC];   // target pixel of a live candidate, else -1
+    bool any = false;
+#pragma unroll
+    for (int c = 0; c < NC; c++) t[c] = -1;
+    if (valid) {
+        bool live[NC];
+        own = field_load<INLAUNCH>(flow_in + pix);
+        h0 = INLAUNCH ? (int)__ldcg(cost + pix) : (int)cost[pix];
+        jump_candidates<RS, INLAUNCH>(flow_in, own, sx, sy, js, doubleProp, rs, x, y, pix, cand, live);
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            if (live[c]) t[c] = pix + lo16(cand[c]) + hi16(cand[c]) * sx;
+            any = any || live[c];
+        }
+    }
+    uint32_t best = own;
+    if (__any_sync(FULL, any)) {
+        const int part = lane & (L - 1), slot = lane / L;
+        const int pix0 = __shfl_sync(FULL, pix, 0);   // lane 0's pixel; the row's others follow
+        uint32_t sum[L][NP];
+        constexpr int G = NSP == 8 ? 2 : 1;   // steps in flight together (measured; 64 bytes spill with two)
+#pragma unroll
+        for (int s0 = 0; s0 < L; s0 += G) {
+            uint4 f1[G], g[G][NC];
+#pragma unroll
+            for (int i = 0; i < G; i++) {
+                const int j = (s0 + i) * PPS + slot;
+                int tj[NC];
+                bool aj = false;
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    tj[c] = __shfl_sync(FULL, t[c], j);
+                    aj = aj || tj[c] >= 0;
+                }
+                f1[i] = stream16_pred(F1 + (size_t)(unsigned int)(pix0 + j) * NSP + part * 4, aj);
+#pragma unroll
+                for (int c = 0; c < NC; c++)
+                    g[i][c] = gather16_pred(F2 + (size_t)(unsigned int)tj[c] * NSP + part * 4, tj[c] >= 0);
+            }
+#pragma unroll
+            for (int i = 0; i < G; i++)
+#pragma unroll
+                for (int k = 0; k < NP; k++) {
+                    sum[s0 + i][k] = (uint32_t)hamming16(f1[i], g[i][2 * k]);
+                    if (2 * k + 1 < NC) sum[s0 + i][k] |= (uint32_t)hamming16(f1[i], g[i][2 * k + 1]) << 16;
+                }
+        }
+        uint32_t mine[NP];
+#pragma unroll
+        for (int k = 0; k < NP; k++) {
+            uint32_t v[L];
+#pragma unroll
+            for (int s = 0; s < L; s++) v[s] = sum[s][k];
+            // halve the steps held per lane until one is left: step == part
+#pragma unroll
+            for (int w = L / 2; w > 0; w /= 2) {
+                const bool up = (part & w) != 0;
+#pragma unroll
+                for (int s = 0; s < w; s++) {
+                    const uint32_t give = up ? v[s] : v[s + w];
+                    const uint32_t keep = up ? v[s + w] : v[s];
+                    v[s] = keep + __shfl_xor_sync(FULL, give, w);
+                }
+            }
+            // lane slot * L + part now holds pixel part * PPS + slot
+            mine[k] = __shfl_sync(FULL, v[0], (lane % PPS) * L + lane / PPS);
+        }
+        int h = h0;
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            const int hc = (int)((c & 1) ? mine[c / 2] >> 16 : mine[c / 2] & 0xffffu);
+            if (t[c] >= 0 && hc < h) {
+                h = hc;
+                best = cand[c];
+            }
+        }
+        if (h != h0) cost[pix] = (uint16_t)h;
+    }
+    if (valid) flow_out[pix] = best;
+}
+
+// One level for the warp's 32 pixels, by descriptor length.
+template <int NSP, bool RS, bool INLAUNCH = false>
+__device__ __forceinline__ void jump_level_px(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
+                                              const uint32_t* flow_in, uint32_t* flow_out, uint16_t* cost, int sx,
+                                              int sy, int p, int pd, int doubleProp, const RsArgs& rs, int x, int y)
+{
+    const JumpStep js = jump_step(sx, sy, p, pd);
+    const bool valid = x < sx && y < sy;
+    if constexpr (NSP >= 8)
+        jump_row<NSP, RS, INLAUNCH>(F1, F2, flow_in, flow_out, cost, sx, sy, js, doubleProp, rs, x, y, valid);
+    else if (valid)
+        jump_px<NSP, RS, INLAUNCH>(F1, F2, flow_in, flow_out, cost, sx, sy, js, doubleProp, rs, x, y);
 }
 
 // Local refinement step of the seeded schedule (no reference counterpart): the

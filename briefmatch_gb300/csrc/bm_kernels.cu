@@ -206,16 +206,21 @@ __global__ void __launch_bounds__(256) k_seed(const uint32_t* __restrict__ F1, c
                  logit_min);
 }
 
+// Blocks per SM the level is compiled for (its time falls with the loads in flight up
+// to the line where registers spill into them): 5 for 32- and 64-byte descriptors (at
+// N512, 3136x1764: 156 us uncapped at 100 registers, 132 at 5 blocks, 156 at 6), 6 with
+// the random search (229 us at 5 blocks, 217 at 6).
 template <int NSP, bool RS>
-__global__ void __launch_bounds__(256) k_jump_level(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
+__host__ __device__ constexpr int jump_blocks() { return NSP <= 4 ? (RS ? 6 : 8) : (NSP == 16 && RS ? 6 : 5); }
+template <int NSP, bool RS>
+__global__ void __launch_bounds__(256, (jump_blocks<NSP, RS>())) k_jump_level(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
                                                     const uint32_t* __restrict__ flow_in, uint32_t* __restrict__ flow_out,
                                                     uint16_t* __restrict__ cost, int sx, int sy,
                                                     int p, int pd, int doubleProp, RsArgs rs, int rev)
 {
     const int2 t0 = block_tile(rev);
     const int x = t0.x + threadIdx.x, y = t0.y + threadIdx.y;
-    if (x >= sx || y >= sy) return;
-    jump_px<NSP, RS>(F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, x, y);
+    jump_level_px<NSP, RS>(F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, x, y);
 }
 
 template <int NSP>
