@@ -68,12 +68,16 @@ struct bm_ctx {
     int prev_frame() const { return (cur_frame + 2) % 3; }
     float* d_up = nullptr;   // dense up-sampled image (BM_BUF_UP), filled on request
     // working up-sampled image with an edge-replicated margin of up_margin pixels on
-    // every side (at least the pattern's largest offset), row pitch up_pitch()
+    // every side (at least the pattern's largest offset), row pitch up_pitch(), followed
+    // by its key image (upad_keys())
     float* d_upad = nullptr;
     int up_margin = 0;
     bool upad_valid = false;   // d_upad holds the current frame
+    bool upad_use = false;     // frames are re-sampled and the pattern fits the key image
     int up_pitch() const { return (int)prm.sx + 2 * up_margin; }
+    size_t upad_count(size_t m) const { return (prm.sx + 2 * m) * (prm.sy + 2 * m); }
     float* upad_origin() const { return d_upad + (size_t)up_margin * up_pitch() + up_margin; }
+    uint32_t* upad_keys() const { return reinterpret_cast<uint32_t*>(d_upad + upad_count(up_margin)); }
     uint32_t* d_feat[2] = {nullptr, nullptr};
     int feat1 = 0;                           // d_feat[feat1] is FEAT1, d_feat[feat1^1] FEAT2
     uint32_t* d_flow[2] = {nullptr, nullptr};
@@ -96,7 +100,7 @@ struct bm_ctx {
     int4* d_pattern = nullptr;
     int pattern_rmax = 0;
     bmk::PatternOffsets pattern_off;       // linear offsets for width sx
-    bmk::PatternOffsets pattern_off_pad;   // linear offsets for pitch up_pitch()
+    bmk::KeyOffsets pattern_off_pad;       // byte offsets for pitch up_pitch() and its margin
     float* d_taps = nullptr;
     float* d_lx = nullptr;
     int* d_ix = nullptr;
@@ -276,8 +280,8 @@ bm_status features_into(bm_ctx* c, const float* d_up, uint32_t* F, bool padded =
 {
     const bm_params& p = c->prm;
     if (padded) {
-        BM_LAUNCH(c, "features", bmk::features_pad(d_up, c->up_pitch(), F, (int)p.sx, (int)p.sy, (int)c->nsp,
-                                                   c->pattern_off_pad, next_order(c), c->stream));
+        BM_LAUNCH(c, "features", bmk::features_keys(c->upad_keys(), c->d_upad, c->up_pitch(), F, (int)p.sx, (int)p.sy,
+                                                    (int)c->nsp, c->pattern_off_pad, next_order(c), c->stream));
         return BM_OK;
     }
     BM_LAUNCH(c, "features", bmk::features(d_up, F, (int)p.sx, (int)p.sy, (int)p.N, (int)c->nsp, c->d_pattern, c->pattern_rmax,
@@ -424,11 +428,13 @@ bm_status set_pattern_impl(bm_ctx* c, const float* h_pattern)
     }
     // the working up-sampled image's margin must cover the largest offset
     const bm_params& p = c->prm;
+    const bool use = (p.sx != p.sx_in || p.sy != p.sy_in) &&
+                     bmk::key_image_fits(std::max(rmax, c->up_margin), (int)p.sx + 2 * std::max(rmax, c->up_margin));
     // (the new image is allocated first: if that fails, the previous pattern and
     // working image stay in effect)
-    if ((p.sx != p.sx_in || p.sy != p.sy_in) && (!c->d_upad || rmax > c->up_margin)) {
+    if (use && (!c->d_upad || rmax > c->up_margin)) {
         float* fresh = nullptr;
-        const bm_status st = dev_alloc(&fresh, (p.sx + 2 * (size_t)rmax) * (p.sy + 2 * (size_t)rmax));
+        const bm_status st = dev_alloc(&fresh, 2 * c->upad_count(rmax));
         if (st != BM_OK) return st;
         const cudaError_t e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) {
@@ -441,12 +447,11 @@ bm_status set_pattern_impl(bm_ctx* c, const float* h_pattern)
         c->upad_valid = false;
     }
     std::memset(&c->pattern_off, 0, sizeof(c->pattern_off));
-    std::memset(&c->pattern_off_pad, 0, sizeof(c->pattern_off_pad));
-    const int sx = (int)p.sx, pitch = c->up_pitch();
-    for (uint32_t s = 0; s < N; s++) {
+    const int sx = (int)p.sx;
+    for (uint32_t s = 0; s < N; s++)
         c->pattern_off.off[s] = make_int2(pat[s].x + pat[s].y * sx, pat[s].z + pat[s].w * sx);
-        c->pattern_off_pad.off[s] = make_int2(pat[s].x + pat[s].y * pitch, pat[s].z + pat[s].w * pitch);
-    }
+    if (use) bmk::key_offsets(c->pattern_off_pad, pat.data(), (int)N, c->up_margin, c->up_pitch());
+    c->upad_use = use;
     BM_CUDA(cudaMemcpyAsync(c->d_pattern, pat.data(), N * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
     BM_CUDA(cudaStreamSynchronize(c->stream));
     c->pattern_rmax = rmax;
@@ -1054,13 +1059,18 @@ bm_status bm_frame(bm_ctx* c, const uint8_t* frame, int frame_on_device, float* 
     BM_LAUNCH(c, "u8_to_f32", bmk::u8_to_f32(d_u8, cur, ni, c->stream));
     // of_pipeline.cpp:301-310
     const float* up = cur;
-    const bool padded = p.sx != p.sx_in || p.sy != p.sy_in;
+    const bool padded = c->upad_use;
     if (padded) {
-        BM_LAUNCH(c, "upsample_u8", bmk::upsample_u8_pad(d_u8, c->d_upad, c->up_pitch(), c->up_margin, (int)p.sx_in,
-                                                         (int)p.sy_in, (int)p.sx, (int)p.sy, c->d_lx, c->d_ix, c->d_ly,
-                                                         c->d_iy, c->stream));
+        BM_LAUNCH(c, "upsample_u8", bmk::upsample_u8_pad(d_u8, c->d_upad, c->upad_keys(), c->up_pitch(), c->up_margin,
+                                                         (int)p.sx_in, (int)p.sy_in, (int)p.sx, (int)p.sy, c->d_lx,
+                                                         c->d_ix, c->d_ly, c->d_iy, c->stream));
         up = c->upad_origin();
         c->upad_valid = true;
+    } else if (p.sx != p.sx_in || p.sy != p.sy_in) {
+        BM_LAUNCH(c, "upsample_u8", bmk::upsample_u8(d_u8, c->d_up, (int)p.sx_in, (int)p.sy_in, (int)p.sx, (int)p.sy,
+                                                     c->d_lx, c->d_ix, c->d_ly, c->d_iy, c->stream));
+        up = c->d_up;
+        c->upad_valid = false;
     }
     bm_status st;
     bool refine_async = false;

@@ -42,7 +42,7 @@ struct PairDev {
     const uint8_t* frame[2];
     float* guide;          // frame 0 as float (the trilateral guide)
     float* up;             // up-sampled frame: dense sx*sy, or edge-replicated (below)
-    int up_margin;         // margin the up buffer has room for: (sx+2m)*(sy+2m) floats
+    int up_margin;         // margin the up buffer has room for: (sx+2m)*(sy+2m) floats, then as many key words
     uint32_t* F[2];
     uint32_t* flow[2];
     uint16_t* cost;
@@ -303,7 +303,7 @@ struct bm_batch {
     std::vector<uint32_t> pos;     // caller's pair index -> internal index
     std::vector<size_t> ws;        // working set of each pair (internal order), bytes
     std::vector<PatternOffsets> pattern_off;  // per pair (internal order), for the per-pair descriptor launches
-    std::vector<PatternOffsets> pattern_off_pad;  // the same for the edge-replicated up-sampled image
+    std::vector<KeyOffsets> pattern_off_pad;  // the same for the edge-replicated up-sampled image
     int max_fsize = 1, max_tri_s = 0;
     size_t tri_smem = 0;
     int coop_blocks_per_sm = 0, num_sms = 0;
@@ -423,14 +423,15 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
     int rev = 0;
     // descriptors from the edge-replicated up-sampled image while the pair's pattern
     // fits the margin its buffer was laid out with; from the dense image otherwise
-    const bool padded = resample && d.rmax <= d.up_margin;
     const int pitch = d.sx + 2 * d.up_margin;
+    const bool padded = resample && d.rmax <= d.up_margin && key_image_fits(d.up_margin, pitch);
     for (int which = 0; which < 2; which++) {
         if (padded) {
-            BB_CUDA(upsample_u8_pad(d.frame[which], d.up, pitch, d.up_margin, d.sx_in, d.sy_in, d.sx, d.sy, d.lx, d.ix,
-                                    d.ly, d.iy, st));
-            BB_CUDA(features_pad(d.up + (size_t)d.up_margin * pitch + d.up_margin, pitch, d.F[which], d.sx, d.sy,
-                                 (int)b->nsp, b->pattern_off_pad[j], rev, st));
+            uint32_t* keys = reinterpret_cast<uint32_t*>(d.up + (size_t)pitch * (d.sy + 2 * d.up_margin));
+            BB_CUDA(upsample_u8_pad(d.frame[which], d.up, keys, pitch, d.up_margin, d.sx_in, d.sy_in, d.sx, d.sy, d.lx,
+                                    d.ix, d.ly, d.iy, st));
+            BB_CUDA(features_keys(keys, d.up, pitch, d.F[which], d.sx, d.sy, (int)b->nsp, b->pattern_off_pad[j], rev,
+                                  st));
         } else {
             if (resample)
                 BB_CUDA(upsample_u8(d.frame[which], d.up, d.sx_in, d.sy_in, d.sx, d.sy, d.lx, d.ix, d.ly, d.iy, st));
@@ -882,7 +883,7 @@ bm_status bm_batch_create(const bm_params* pairs, uint32_t count, bm_batch** out
         const size_t n = (size_t)p.sx * p.sy, ni = (size_t)p.sx_in * p.sy_in;
         Off& o = offs[i];
         o.guide = take(ni * 4);
-        o.up = take((p.sx + 2 * (size_t)margin[i]) * (p.sy + 2 * (size_t)margin[i]) * 4);
+        o.up = take(2 * (p.sx + 2 * (size_t)margin[i]) * (p.sy + 2 * (size_t)margin[i]) * 4);
         o.F[0] = take(n * b->nsp * 4);
         o.F[1] = take(n * b->nsp * 4);
         o.flow[0] = take(n * 4);
@@ -1069,7 +1070,7 @@ bm_status bm_batch_set_pattern(bm_batch* b, uint32_t pair, const float* h_patter
     if (!b || !h_pattern || pair >= b->count) return bfail(BM_ERR_INVALID, "bm_batch_set_pattern: bad argument");
     if (count != 4 * b->N) return bfail(BM_ERR_INVALID, "bm_batch_set_pattern: expected 4*N values");
     std::vector<int4> pat(b->N);
-    std::vector<int2> off(BM_PATCH_MAX / 4, make_int2(0, 0)), off_pad(BM_PATCH_MAX / 4, make_int2(0, 0));
+    std::vector<int2> off(BM_PATCH_MAX / 4, make_int2(0, 0));
     int rmax = 0;
     const uint32_t j = b->pos[pair];
     PairDev& d = b->pairs[j];
@@ -1082,13 +1083,12 @@ bm_status bm_batch_set_pattern(bm_batch* b, uint32_t pair, const float* h_patter
         }
         pat[s] = make_int4(v[0], v[1], v[2], v[3]);
         off[s] = make_int2(v[0] + v[1] * sx, v[2] + v[3] * sx);
-        off_pad[s] = make_int2(v[0] + v[1] * pitch, v[2] + v[3] * pitch);
     }
     d.rmax = rmax;
     if (b->pattern_off.size() != b->count) b->pattern_off.resize(b->count);
     if (b->pattern_off_pad.size() != b->count) b->pattern_off_pad.resize(b->count);
     std::memcpy(b->pattern_off[j].off, off.data(), sizeof(b->pattern_off[j].off));
-    std::memcpy(b->pattern_off_pad[j].off, off_pad.data(), sizeof(b->pattern_off_pad[j].off));
+    if (rmax <= d.up_margin) key_offsets(b->pattern_off_pad[j], pat.data(), (int)b->N, d.up_margin, pitch);
     BB_CUDA(cudaMemcpyAsync((void*)d.pat, pat.data(), b->N * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
     BB_CUDA(cudaMemcpyAsync((void*)d.off, off.data(), off.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
     if (b->d_pairs)

@@ -204,6 +204,47 @@ __device__ __forceinline__ void upsample_px(const T* __restrict__ in, float* __r
 }
 
 // ---------------------------------------------------------------------------
+// 16-bit keys of image samples: a monotone map of the float value to a half-precision
+// bit pattern, so that keys compare two at a time; different keys order as their floats
+// do, equal keys leave the order open.  The 63487 finite halves from -0x7bff to 0x7bff
+// cover 128 +- 158.7 grey levels (Lanczos overshoot included) in steps of 1/200;
+// values beyond share the end keys.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t sample_key(float v)
+{
+    const int i = __float2int_rn(fminf(fmaxf(__fmaf_rn(v, 200.0f, -25600.0f), -31743.0f), 31743.0f));
+    return i < 0 ? 0x8000u | (uint32_t)(-i) : (uint32_t)i;
+}
+// 1.0 or 0.0 per half
+__device__ __forceinline__ uint32_t half2_gt(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("set.gt.f16x2.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t half2_eq(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("set.eq.f16x2.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// 2 * acc + bit per half
+__device__ __forceinline__ uint32_t half2_shift_in(uint32_t acc, uint32_t bit)
+{
+    uint32_t r;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(acc), "r"(0x40004000u), "r"(bit));
+    return r;
+}
+// Four accumulators that hold 1024 + byte in each half (0x6400 | byte): the words of the
+// low and of the high halves' bytes.
+__device__ __forceinline__ void half2_bytes(const uint32_t (&a)[4], uint32_t& lo, uint32_t& hi)
+{
+    const uint32_t p = __byte_perm(a[0], a[1], 0x6240), q = __byte_perm(a[2], a[3], 0x6240);
+    lo = __byte_perm(p, q, 0x5410);
+    hi = __byte_perm(p, q, 0x7632);
+}
+
+// ---------------------------------------------------------------------------
 // BRIEF descriptors (briefmatch_cuda.cu:82-124).
 // Interior pixels (at least rmax from every border, rmax = the largest |offset|)
 // read the image at the precomputed linear offsets `off` with no clamping -- the
@@ -230,44 +271,6 @@ __device__ __forceinline__ void features_interior_px(const float* __restrict__ I
         word[wd] = acc;
     }
     store_desc<NSP>(F + ((size_t)y * sx + x) * NSP, word);
-}
-
-// A strip of PX pixels at x, x+TX, ..., x+(PX-1)*TX of one row, in an image whose
-// every sample point of those pixels is addressable (an edge-replicated margin at
-// least as wide as the largest offset: the reads then equal the reference's
-// per-coordinate clamped reads).  `base` points at pixel x, `room` = sx - x; the
-// strip's pixels share each offset's address arithmetic (the others are immediate
-// displacements of TX pixels).
-template <int NSP, int PX, typename OffArray>
-__device__ __forceinline__ void features_strip_px(const float* __restrict__ base, uint32_t* __restrict__ F, int room,
-                                                  const OffArray& off)
-{
-    uint32_t word[PX][NSP];
-#pragma unroll
-    for (int wd = 0; wd < NSP; wd++) {
-        uint32_t acc[PX];
-#pragma unroll
-        for (int k = 0; k < PX; k++) acc[k] = 0;
-#pragma unroll
-        for (int b = 0; b < 32; b++) {
-            const int2 o = off[wd * 32 + b];
-            const float* p1 = base + o.x;
-            const float* p2 = base + o.y;
-#pragma unroll
-            for (int k = 0; k < PX; k++) {
-                if (k == 0 || k * TX < room) {
-                    const float i1 = __ldg(p1 + k * TX);
-                    const float i2 = __ldg(p2 + k * TX);
-                    if (i1 > i2) acc[k] |= 1u << b;
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < PX; k++) word[k][wd] = acc[k];
-    }
-#pragma unroll
-    for (int k = 0; k < PX; k++)
-        if (k == 0 || k * TX < room) store_desc<NSP>(F + (size_t)k * TX * NSP, word[k]);
 }
 
 template <int NSP>

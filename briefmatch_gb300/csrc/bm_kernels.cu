@@ -13,6 +13,7 @@
 //   cost         uint16 per pixel, the Hamming distance of the current candidate
 //                (the reference's D is cost/N)
 #include <climits>
+#include <cstring>
 #include <mutex>
 
 #include "bm_device.cuh"
@@ -81,9 +82,15 @@ __global__ void __launch_bounds__(256) k_upsample(const T* __restrict__ in, floa
 // reference's order (util_cuda.cu:140-152: over source columns, then rows;
 // v += (in * Lx) * Ly as one rounded product and an FMA, w += Lx * Ly as an FMA), so
 // every value equals upsample_val's bit for bit.
+//
+// Beside the float image the kernel writes the key image the descriptors read: a word
+// per pixel with the 16-bit key (sample_key) of the pixel in its low half and of the
+// pixel below it in its high half.  A thread pairs the keys of its own rows; the word
+// that spans two threads' rows is written as two halves.
 constexpr int UP_R = 8;
 __global__ void __launch_bounds__(TX * TY) k_upsample_pad_rows(const uint8_t* __restrict__ in, float* __restrict__ out,
-                                                               int pitch, int m, int sxi, int syi, int sxo, int syo,
+                                                               uint32_t* __restrict__ keys, int pitch, int m, int sxi,
+                                                               int syi, int sxo, int syo,
                                                                const float* __restrict__ lx, const int* __restrict__ ix,
                                                                const float* __restrict__ ly, const int* __restrict__ iy)
 {
@@ -101,6 +108,7 @@ __global__ void __launch_bounds__(TX * TY) k_upsample_pad_rows(const uint8_t* __
     }
     float P[6][6];  // P[a][b] = in[row b of the window][col a] * Lx[a]
     int win = INT_MIN;
+    uint32_t key_above = 0;
 #pragma unroll
     for (int r = 0; r < UP_R; r++) {
         const int Y = Y0 + r;
@@ -127,7 +135,16 @@ __global__ void __launch_bounds__(TX * TY) k_upsample_pad_rows(const uint8_t* __
                 w = __fmaf_rn(Lx[a], Ly[b], w);
                 v = __fmaf_rn(P[a][b], Ly[b], v);
             }
-        out[X + (size_t)Y * pitch] = v / w;
+        const float val = v / w;
+        const size_t o = X + (size_t)Y * pitch;
+        out[o] = val;
+        const uint32_t key = sample_key(val);
+        if (r > 0)
+            keys[o - pitch] = key_above | (key << 16);
+        else if (Y > 0)
+            reinterpret_cast<uint16_t*>(keys + (o - pitch))[1] = (uint16_t)key;
+        if (r == UP_R - 1 || Y == syo + 2 * m - 1) reinterpret_cast<uint16_t*>(keys + o)[0] = (uint16_t)key;
+        key_above = key;
     }
 }
 
@@ -160,26 +177,122 @@ __global__ void __launch_bounds__(256) k_features(const float* __restrict__ I, u
     }
 }
 
-// BRIEF descriptors from an edge-replicated image (k_upsample_pad_rows) whose margin is
-// at least the pattern's largest offset: every pixel reads at the linear offsets
-// (no clamping, no border tiles); each thread computes feat_px<NSP>() pixels TX apart
-// (two up to 128-bit descriptors, where sharing each offset's address arithmetic
-// pays; one for longer ones, whose descriptor words would cost occupancy).
+// BRIEF descriptors from the key image of an edge-replicated frame (k_upsample_pad_rows)
+// whose margin is at least the pattern's largest offset: every pixel reads at the
+// linear offsets (no clamping, no border tiles).  A thread takes the pixels (x, y) and
+// (x, y + 1): one key word per sample serves both.
+//
+// Per sample pair, four half-precision instructions: `set.gt` and `set.eq` (1.0 or 0.0
+// per half) and an FMA each that shifts the result into an accumulator
+// (acc = 2 acc + bit; from 4.0, eight results leave 1024 + their byte, exact in a
+// half).  Equal keys do not say which sample is larger: those pairs (and only those)
+// are compared again on the float image, so every bit is the float comparison's.
+// Samples whose two points coincide (and the padding past N) are equal by construction;
+// their bits are masked out of that by the pattern (po.differ).  On textured frames one
+// pair in a thousand ties and each lane repairs its own; saturated or flat parts tie
+// throughout, and there (a lane with more than MANY_TIES) the warp goes sample by
+// sample, and past FLAT_TIES samples of a word reads the next words of the chunk from
+// the float image outright.
+//
+// Reading two keys per 4 bytes halves the load requests that bound the float form
+// (70 % of the load unit's rate, and 13 % of its instructions branches around the
+// strip's end): 144 -> 98 us at 2969x1264 N128, 280 -> 194 at N256, 980 -> 572 at
+// 3136x1764 N512.  What bounds it now is issue; without the ties' repair and detection
+// it would be 68 us at N128.  Measured beside it: four pixels per thread (32 columns
+// on, sharing the addresses) 101, 203 and 606 us, its code twice as long for the
+// instruction cache; all sixteen words of N512 unrolled 17 % slower; a repair that
+// always goes sample by sample 102 and 575.  Six blocks per SM (40 registers) measured
+// 1-3 % better than five, seven or eight.
+constexpr int FLAT_TIES = 12, MANY_TIES = 12;
 template <int NSP>
-__host__ __device__ constexpr int feat_px() { return NSP <= 4 ? 2 : 1; }
-template <int NSP>
-__global__ void __launch_bounds__(256) k_features_pad(const float* __restrict__ I, uint32_t* __restrict__ F,
-                                                      int pitch, int sx, int sy,
-                                                      const __grid_constant__ PatternOffsets po, int rev)
+__global__ void __launch_bounds__(256, 6) k_features_keys(const uint32_t* __restrict__ W, const float* __restrict__ I,
+                                                          int pitch, uint32_t* __restrict__ F, int sx, int sy,
+                                                          const __grid_constant__ KeyOffsets po, int rev)
 {
     int bx = blockIdx.x, by = blockIdx.y;
     if (rev) {
         bx = gridDim.x - 1 - bx;
         by = gridDim.y - 1 - by;
     }
-    const int x = bx * (TX * feat_px<NSP>()) + threadIdx.x, y = by * TY + threadIdx.y;
-    if (x >= sx || y >= sy) return;
-    features_strip_px<NSP, feat_px<NSP>()>(I + (size_t)y * pitch + x, F + ((size_t)y * sx + x) * NSP, sx - x, po.off);
+    const int x = bx * TX + threadIdx.x;
+    const int y = 2 * (by * TY + threadIdx.y);
+    const bool inside = x < sx && y < sy;
+    const unsigned int warp = __ballot_sync(0xffffffffu, inside);
+    if (!inside) return;
+    // the pixel less the margin; each sample adds an unsigned 32-bit byte offset
+    const size_t origin = (size_t)y * pitch + x;
+    const char* base = reinterpret_cast<const char*>(W + origin);
+    const char* fbase = reinterpret_cast<const char*>(I + origin);
+    const size_t down = (size_t)pitch * sizeof(float);
+    const bool second = y + 1 < sy;
+    // sample b of word w of pixel v on the float image
+    auto larger = [&](uint2 o, int v) {
+        const char* f = fbase + v * down;
+        return __ldg(reinterpret_cast<const float*>(f + o.x)) > __ldg(reinterpret_cast<const float*>(f + o.y));
+    };
+    auto compare = [&](int w, int b, const uint32_t (&ask)[2], uint32_t (&bits)[2]) {
+        const uint2 o = po.off[w * 32 + b];
+#pragma unroll
+        for (int v = 0; v < 2; v++)
+            if ((ask[v] >> b & 1u) && larger(o, v)) bits[v] |= 1u << b;
+    };
+    constexpr int CW = NSP < 4 ? NSP : 4;   // words formed before they are stored
+#pragma unroll 1
+    for (int c = 0; c < NSP / CW; c++) {
+        uint32_t word[2][CW];
+        bool flat = false;
+#pragma unroll
+        for (int wd = 0; wd < CW; wd++) {
+            const int w = c * CW + wd;
+            uint32_t bits[2], ask[2];
+            if (flat) {
+                bits[0] = bits[1] = 0;
+                ask[0] = 0xffffffffu;
+                ask[1] = second ? 0xffffffffu : 0;
+#pragma unroll 4
+                for (int b = 0; b < 32; b++) compare(w, b, ask, bits);
+            } else {
+                uint32_t gt[4], eq[4];
+#pragma unroll
+                for (int g = 0; g < 4; g++) {
+                    gt[g] = eq[g] = 0x44004400u;     // 4.0, 4.0
+#pragma unroll
+                    for (int b = 7; b >= 0; b--) {   // the byte's low bit is its first sample
+                        const uint2 o = po.off[w * 32 + g * 8 + b];
+                        const uint32_t k1 = __ldg(reinterpret_cast<const uint32_t*>(base + o.x));
+                        const uint32_t k2 = __ldg(reinterpret_cast<const uint32_t*>(base + o.y));
+                        gt[g] = half2_shift_in(gt[g], half2_gt(k1, k2));
+                        eq[g] = half2_shift_in(eq[g], half2_eq(k1, k2));
+                    }
+                }
+                half2_bytes(gt, bits[0], bits[1]);
+                half2_bytes(eq, ask[0], ask[1]);
+                ask[0] &= po.differ[w];
+                ask[1] = second ? ask[1] & po.differ[w] : 0;
+                if (__any_sync(warp, max(__popc(ask[0]), __popc(ask[1])) > MANY_TIES)) {
+                    uint32_t any = __reduce_or_sync(warp, ask[0] | ask[1]);
+                    flat = __popc(any) > FLAT_TIES;
+                    while (any) {
+                        const int b = __ffs(any) - 1;
+                        any &= any - 1;
+                        compare(w, b, ask, bits);
+                    }
+                } else {
+#pragma unroll
+                    for (int v = 0; v < 2; v++)
+                        while (ask[v]) {
+                            const int b = __ffs(ask[v]) - 1;
+                            ask[v] &= ask[v] - 1;
+                            if (larger(po.off[w * 32 + b], v)) bits[v] |= 1u << b;
+                        }
+                }
+            }
+            word[0][wd] = bits[0];
+            word[1][wd] = bits[1];
+        }
+        store_desc<CW>(F + ((size_t)y * sx + x) * NSP + c * CW, word[0]);
+        if (second) store_desc<CW>(F + ((size_t)(y + 1) * sx + x) * NSP + c * CW, word[1]);
+    }
 }
 
 template <int NSP>
@@ -420,12 +533,12 @@ cudaError_t upsample_u8(const uint8_t* in, float* out, int sxi, int syi, int sxo
     return cudaGetLastError();
 }
 
-cudaError_t upsample_u8_pad(const uint8_t* in, float* out, int pitch, int m, int sxi, int syi, int sxo, int syo,
-                            const float* lx, const int* ix, const float* ly, const int* iy, cudaStream_t st)
+cudaError_t upsample_u8_pad(const uint8_t* in, float* out, uint32_t* keys, int pitch, int m, int sxi, int syi, int sxo,
+                            int syo, const float* lx, const int* ix, const float* ly, const int* iy, cudaStream_t st)
 {
     if (m < 0 || pitch < sxo + 2 * m) return cudaErrorInvalidValue;
     const dim3 g((sxo + 2 * m + TX - 1) / TX, (syo + 2 * m + TY * UP_R - 1) / (TY * UP_R));
-    k_upsample_pad_rows<<<g, dim3(TX, TY), 0, st>>>(in, out, pitch, m, sxi, syi, sxo, syo, lx, ix, ly, iy);
+    k_upsample_pad_rows<<<g, dim3(TX, TY), 0, st>>>(in, out, keys, pitch, m, sxi, syi, sxo, syo, lx, ix, ly, iy);
     return cudaGetLastError();
 }
 
@@ -452,14 +565,24 @@ cudaError_t features(const float* up, uint32_t* F, int sx, int sy, int N, int ns
     return cudaGetLastError();
 }
 
-cudaError_t features_pad(const float* up, int pitch, uint32_t* F, int sx, int sy, int nsp,
-                         const PatternOffsets& po, int rev, cudaStream_t st)
+bool key_image_fits(int m, int pitch) { return (2 * (size_t)m + 1) * (size_t)pitch < ((size_t)1 << 30); }
+
+void key_offsets(KeyOffsets& ko, const int4* pat, int N, int m, int pitch)
 {
-    BM_DISPATCH_NSP(nsp, {
-        const int w = TX * feat_px<NSP>();
-        k_features_pad<NSP><<<dim3((sx + w - 1) / w, (sy + TY - 1) / TY), dim3(TX, TY), 0, st>>>(up, F, pitch, sx, sy,
-                                                                                                 po, rev);
-    });
+    std::memset(&ko, 0, sizeof(ko));
+    auto at = [&](int dx, int dy) { return (uint32_t)((size_t)(dy + m) * pitch + (dx + m)) * 4u; };
+    for (int s = 0; s < BM_PATCH_MAX / 4; s++) {
+        const int4 q = s < N ? pat[s] : make_int4(0, 0, 0, 0);
+        ko.off[s] = make_uint2(at(q.x, q.y), at(q.z, q.w));
+        if (ko.off[s].x != ko.off[s].y) ko.differ[s / 32] |= 1u << (s % 32);
+    }
+}
+
+cudaError_t features_keys(const uint32_t* keys, const float* up, int pitch, uint32_t* F, int sx, int sy, int nsp,
+                          const KeyOffsets& ko, int rev, cudaStream_t st)
+{
+    const dim3 g((sx + TX - 1) / TX, (sy + 2 * TY - 1) / (2 * TY));
+    BM_DISPATCH_NSP(nsp, (k_features_keys<NSP><<<g, dim3(TX, TY), 0, st>>>(keys, up, pitch, F, sx, sy, ko, rev)));
     return cudaGetLastError();
 }
 
