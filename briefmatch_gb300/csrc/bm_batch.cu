@@ -38,7 +38,6 @@ struct PairDev {
     float dist, mx, my, cE, cI, cS;
     int first_up_tile_x;   // tiles per row on the up-sampled grid
     int first_in_tile_x;   // tiles per row at input resolution (32x8)
-    int first_tri_tile_x;  // tiles per row for the trilateral filter (TX x TRI_BY)
     const uint8_t* frame[2];
     float* guide;          // frame 0 as float (the trilateral guide)
     float* up;             // up-sampled frame: dense sx*sy, or edge-replicated (below)
@@ -66,7 +65,6 @@ struct BatchDev {
     const PairDev* pairs;
     const unsigned int* pre_up;   // [count+1] exclusive prefix of up-sampled-grid tiles
     const unsigned int* pre_in;   // input-resolution 32x8 tiles
-    const unsigned int* pre_tri;  // trilateral TX x TRI_BY tiles
     int lo, hi;
     int N;
 };
@@ -293,8 +291,8 @@ struct bm_batch {
     size_t arena_bytes = 0;
     std::vector<PairDev> pairs;   // host copy (device addresses)
     PairDev* d_pairs = nullptr;
-    unsigned int* d_pre = nullptr;   // 3 prefix arrays of count+1
-    std::vector<unsigned int> pre_up, pre_in, pre_tri;
+    unsigned int* d_pre = nullptr;   // 2 prefix arrays of count+1
+    std::vector<unsigned int> pre_up, pre_in;
     GridSync* d_sync = nullptr;
     size_t frames_offset = 0, frames_bytes = 0;   // packed input frames inside the arena
     size_t flows_offset = 0, flows_bytes = 0;     // packed refined flows (U,V per pair)
@@ -305,7 +303,6 @@ struct bm_batch {
     std::vector<PatternOffsets> pattern_off;  // per pair (internal order), for the per-pair descriptor launches
     std::vector<KeyOffsets> pattern_off_pad;  // the same for the edge-replicated up-sampled image
     int max_fsize = 1, max_tri_s = 0;
-    size_t tri_smem = 0;
     int coop_blocks_per_sm = 0, num_sms = 0;
     bm_batch_schedule sched{};
     cudaGraphExec_t graph_exec = nullptr;
@@ -354,7 +351,6 @@ BatchDev batch_dev(const bm_batch* b, int lo, int hi)
     bd.pairs = b->d_pairs;
     bd.pre_up = b->d_pre;
     bd.pre_in = b->d_pre + (b->count + 1);
-    bd.pre_tri = b->d_pre + 2 * (b->count + 1);
     bd.lo = lo;
     bd.hi = hi;
     bd.N = (int)b->N;
@@ -925,7 +921,6 @@ bm_status bm_batch_create(const bm_params* pairs, uint32_t count, bm_batch** out
     b->pairs.resize(count);
     b->pre_up.assign(count + 1, 0);
     b->pre_in.assign(count + 1, 0);
-    b->pre_tri.assign(count + 1, 0);
     std::vector<float> pattern(4 * (size_t)b->N);
     for (uint32_t j = 0; j < count; j++) {
         const uint32_t i = b->order[j];  // caller's index of internal pair j
@@ -951,10 +946,8 @@ bm_status bm_batch_create(const bm_params* pairs, uint32_t count, bm_batch** out
         d.cS = tc.cS;
         d.first_up_tile_x = (d.sx + TX - 1) / TX;
         d.first_in_tile_x = (d.sx_in + TX - 1) / TX;
-        d.first_tri_tile_x = (d.sx_in + TX - 1) / TX;
         b->pre_up[j + 1] = b->pre_up[j] + (unsigned)(d.first_up_tile_x * ((d.sy + TY - 1) / TY));
         b->pre_in[j + 1] = b->pre_in[j] + (unsigned)(d.first_in_tile_x * ((d.sy_in + TY - 1) / TY));
-        b->pre_tri[j + 1] = b->pre_tri[j] + (unsigned)(d.first_tri_tile_x * ((d.sy_in + TRI_BY - 1) / TRI_BY));
         char* A = b->arena;
         d.frame[0] = reinterpret_cast<const uint8_t*>(A + b->frames_offset + b->frame_off[2 * i]);
         d.frame[1] = reinterpret_cast<const uint8_t*>(A + b->frames_offset + b->frame_off[2 * i + 1]);
@@ -991,18 +984,16 @@ bm_status bm_batch_create(const bm_params* pairs, uint32_t count, bm_batch** out
         bm_status st = bm_batch_set_pattern(b, i, pattern.data(), 4 * b->N);
         if (st != BM_OK) return fail_clean(st);
     }
-    b->tri_smem = tri_smem_bytes(b->max_tri_s);
-    if (b->filter && b->tri_smem > 220 * 1024)
+    if (b->filter && b->max_tri_s > TRI_MAX_S)
         return fail_clean(bfail(BM_ERR_LIMIT, "bm_batch_create: spatial window %d too large for the batched filter",
                                 b->max_tri_s));
     if (bmk::device_malloc((void**)&b->d_pairs, count * sizeof(PairDev)) != cudaSuccess ||
-        bmk::device_malloc((void**)&b->d_pre, 3 * (count + 1) * sizeof(unsigned int)) != cudaSuccess ||
+        bmk::device_malloc((void**)&b->d_pre, 2 * (count + 1) * sizeof(unsigned int)) != cudaSuccess ||
         bmk::device_malloc((void**)&b->d_sync, sizeof(GridSync)) != cudaSuccess)
         return fail_clean(bfail(BM_ERR_NOMEM, "bm_batch_create: descriptor allocation failed"));
     std::vector<unsigned int> pre;
     pre.insert(pre.end(), b->pre_up.begin(), b->pre_up.end());
     pre.insert(pre.end(), b->pre_in.begin(), b->pre_in.end());
-    pre.insert(pre.end(), b->pre_tri.begin(), b->pre_tri.end());
     if (cudaMemcpyAsync(b->d_pairs, b->pairs.data(), count * sizeof(PairDev), cudaMemcpyHostToDevice, b->stream) !=
             cudaSuccess ||
         cudaMemcpyAsync(b->d_pre, pre.data(), pre.size() * sizeof(unsigned int), cudaMemcpyHostToDevice, b->stream) !=

@@ -152,15 +152,12 @@ __device__ __forceinline__ f2x pk2(float a, float b) { f2x r; asm("mov.b64 %0, {
 __device__ __forceinline__ float lo2(f2x v) { return __uint_as_float((unsigned int)(v & 0xffffffffull)); }
 __device__ __forceinline__ float hi2(f2x v) { return __uint_as_float((unsigned int)(v >> 32)); }
 __device__ __forceinline__ f2x add2(f2x a, f2x b) { f2x d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2x sub2(f2x a, f2x b) { f2x d; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f2x mul2(f2x a, f2x b) { f2x d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ f2x fma2(f2x a, f2x b, f2x c)
 {
     f2x d;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-__device__ __forceinline__ f2x ex2_2(f2x a) { return pk2(exp2f(lo2(a)), exp2f(hi2(a))); }
 
 
 // ---------------------------------------------------------------------------
@@ -796,166 +793,230 @@ __device__ __forceinline__ void median2_px(const float* __restrict__ in, float* 
 }
 
 // ---------------------------------------------------------------------------
-// Cross-trilateral filter (briefmatch_cuda.cu:248-297), one block of TX x TRI_TY
-// threads filtering the TX x TRI_BY outputs whose top-left pixel is (bx0, by0).
-// Each thread owns four vertically adjacent outputs, held as two pairs in packed
-// f32x2 registers, so every neighbourhood sample it reads from shared memory is
-// used four times and every arithmetic instruction serves two outputs.  The
-// (2s + TX) x (2s + TRI_BY) neighbourhood is staged in shared memory with
-// clamp-to-edge addressing.  The three Gaussians are one exp2 of the summed
-// exponents cE*(du^2 + dv^2) + cI*dI^2 + cS*j^2 = r*(du'^2 + dv'^2 + dI'^2 + j^2*cS/r)
-// with du' = kE*u - kE*uc: kE is the power of two nearest sqrt(cE) (so kE*uc is
-// exact and du' is the scaled difference rounded once -- a rounded centre would
-// tilt every weight of the window the same way), r = cE/kE^2, kI = sqrt(cI/r).
-// Each scaled difference is one FMA against the centre's negated scaled value, the
-// squared terms accumulate by FMA onto the row term, one multiply by r, one exp2:
-// seven FP32 operations per tap and output before the three accumulations.  The
-// column factor exp2(-cS*i^2) is applied once per column (the inner loop runs down
-// a column); row terms outside the window are +inf (weight 0).
-// `smem` must hold tri_smem_bytes(s).
+// Cross-trilateral filter (briefmatch_cuda.cu:248-297): one block filters the TX x
+// 4 TY outputs whose top-left pixel is (bx0, by0).  Each thread owns four vertically
+// adjacent outputs and walks the window column by column, two source rows at a time:
+// packed f32x2 registers hold the two rows, so a sample pair is used as it is read from
+// shared memory (the tile is stored column by column) and serves all four outputs.
+// TRI_G = 2 groups of TX x TY threads share a tile, each taking half of the window's
+// columns; their sums meet in shared memory.  The neighbourhood is staged with
+// clamp-to-edge addressing, `smem` must hold tri_smem_bytes(s, TY).
+//
+// The three Gaussians are one exp2 of the summed exponents:
+// q = du^2 + dv^2 + dI^2 + j^2 cS over scaled differences (kE = sqrt(cE), kI = sqrt(cI)).
+// Samples are staged as kE (u - ru) with one reference flow per block (a nearby median
+// value): scaling and subtraction round relative to the small difference, the sums are
+// of small numbers, and the reference is added back to the quotient, which leaves a
+// fifth of the error of sums over the flow itself (1920x1080: 3.9e-8 of the field's norm
+// against 64 bits, 2.1e-7 before).  The column factor exp2(-cS i^2) is applied once per
+// column.  Nine FP32 lane operations per tap and output.
+//
+// What bounds it is the FP32 pipe's operand reads: a packed FMA with three different
+// 64-bit operands takes three cycles, with two it takes two (measured).  So differences
+// are additions, squares read one register twice, and only the two weighted sums need
+// three operands: 20 cycles per pair of taps, 18 by operation count.  1920x1080 with a
+// 94 x 94 window: 7.16 -> 5.66 ms; 1024x436 (48 x 48): 400 -> 344 us.
+//
+// Row pairs: source row m lies in output r's window when 0 <= m - r < 2s.  Outputs 0
+// and 2 take whole pairs; outputs 1 and 3 have a single row in their first and last
+// pair, whose other half is taken as zero with an infinite row term, so no sample
+// outside a window is touched.
 // ---------------------------------------------------------------------------
-constexpr int TRI_R = 4;                // outputs per thread (two f32x2 pairs)
-constexpr int TRI_TY = 8;               // thread rows per block
-constexpr int TRI_BY = TRI_TY * TRI_R;  // output rows per block (32x32 outputs)
+constexpr int TRI_R = 4;       // outputs per thread
+constexpr int TRI_UNROLL = 8;  // row pairs per turn of the column walk (measured: 1, 2, 4, 8, 16)
+constexpr int TRI_MAX_S = 52;  // largest half window whose tile fits an SM's shared memory (226 KB)
+constexpr int TRI_G = 2;       // thread groups per block, each taking half of the window's columns
 
-__host__ __device__ inline size_t tri_smem_bytes(int s)
+// Rows of a tile of TY thread rows, and floats per tile column: the rows, padded to 2
+// modulo 4 so that the 16 lanes of a 64-bit read phase fall on 32 different banks.
+__host__ __device__ constexpr int tri_rows(int ty) { return ty * TRI_R; }
+__host__ __device__ inline int tri_pitch(int s, int ty) { return tri_rows(ty) + 2 * s + ((s & 1) ? 0 : 2); }
+
+__host__ __device__ inline size_t tri_smem_bytes(int s, int ty)
 {
-    return (size_t)(2 * s + TRI_R - 1) * sizeof(float4) + (size_t)(TX + 2 * s) * (TRI_BY + 2 * s) * 3 * sizeof(float);
+    const size_t tile = (size_t)(TX + 2 * s) * tri_pitch(s, ty) * 3;
+    const size_t sums = (size_t)(TRI_G - 1) * TX * ty * TRI_R * 3;   // the groups' partial sums reuse the tile
+    return (size_t)(s + 1) * sizeof(float4) + (tile > sums ? tile : sums) * sizeof(float);
 }
 
-__device__ __forceinline__ f2x ex2n_2(f2x a) { return pk2(exp2f(-lo2(a)), exp2f(-hi2(a))); }
+// A common flow (or intensity) that the samples of a block are taken relative to: a
+// nearby value where that is an ordinary one, else 0.
+__device__ __forceinline__ float tri_reference(float v) { return fabsf(v) <= 1024.0f ? v : 0.0f; }
 
+// 2^-x per half.  The negation is spelled without .ftz, which makes it a modifier of the
+// exponential's operand: under -use_fast_math a C++ minus is neg.ftz, an addition of its
+// own on the FP32 pipe (two of them per pair of taps were 19 % of that pipe's work).
+__device__ __forceinline__ float ex2n(float x)
+{
+    float r;
+    asm("{\n\t.reg .f32 t;\n\tneg.f32 t, %1;\n\tex2.approx.ftz.f32 %0, t;\n\t}" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ f2x ex2n_2(f2x a) { return pk2(ex2n(lo2(a)), ex2n(hi2(a))); }
+
+template <int TY>
 __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, const float* __restrict__ V,
                                                  const float* __restrict__ Um, const float* __restrict__ Vm,
                                                  const float* __restrict__ I, float* __restrict__ Uo,
-                                                 float* __restrict__ Vo, int sx, int sy, int s, float cE, float cI,
+                                                 float* __restrict__ Vo, int sx, int sy, int s, float kE, float kI,
                                                  float cS, int bx0, int by0, float4* smem4)
 {
-    const int TW = TX + 2 * s, TH = TRI_BY + 2 * s;
-    const int NR = 2 * s + TRI_R - 1;        // source rows a thread walks per column
-    float4* rowf = smem4;                    // [NR] row terms j^2*cS for outputs r=0..3
-    float2* suv = reinterpret_cast<float2*>(smem4 + NR);
-    float* sI = reinterpret_cast<float*>(suv + TW * TH);
+    const int TW = TX + 2 * s, TH = tri_rows(TY) + 2 * s, P = tri_pitch(s, TY);
+    // row terms of pair p: outputs 0 (.x .y: rows 2p, 2p + 1) and 1 (.z .w: rows 2p - 1,
+    // 2p); outputs 2 and 3 use pair p - 1's
+    float4* rowf = smem4;                                     // [s + 1]
+    float* sU = reinterpret_cast<float*>(smem4 + s + 1);      // [TW][P], column by column
+    float* sV = sU + TW * P;
+    float* sI = sV + TW * P;
     const int x0 = bx0 - s, y0 = by0 - s;
-    const int tid = threadIdx.y * TX + threadIdx.x;
-    // kE: the power of two nearest sqrt(cE) (exact scaling), r_ the remaining factor
-    const float kE = exp2f(rintf(0.5f * __log2f(cE))), r_ = cE / (kE * kE);
-    const float kI = sqrtf(cI / r_), cS_r = cS / r_;
-    for (int k = tid; k < TW * TH; k += TX * TRI_TY) {
-        const int r = k / TW, c = k - r * TW;
-        const int gx = min(sx - 1, max(0, x0 + c)), gy = min(sy - 1, max(0, y0 + r));
-        const size_t g = (size_t)gx + (size_t)gy * sx;
-        suv[k] = make_float2(__ldg(U + g), __ldg(V + g));
-        sI[k] = __ldg(I + g);
-    }
-    for (int m = tid; m < NR; m += TX * TRI_TY) {
-        float t[TRI_R];
-#pragma unroll
-        for (int r = 0; r < TRI_R; r++) {
-            const int j = m - r - s;  // vertical offset of this source row for output r
-            t[r] = (j >= -s && j < s) ? (float)(j * j) * cS_r : __int_as_float(0x7f800000);
+    // the block's reference flow and intensity
+    const size_t mid = (size_t)min(sx - 1, bx0 + TX / 2) + (size_t)min(sy - 1, by0 + tri_rows(TY) / 2) * sx;
+    const float ru = tri_reference(__ldg(Um + mid)), rv = tri_reference(__ldg(Vm + mid)), ri = tri_reference(__ldg(I + mid));
+    for (int r = threadIdx.z * TY + threadIdx.y; r < TH; r += TY * TRI_G) {
+        const size_t row = (size_t)min(sy - 1, max(0, y0 + r)) * sx;
+        for (int c = threadIdx.x; c < TW; c += TX) {
+            const size_t g = row + min(sx - 1, max(0, x0 + c));
+            sU[c * P + r] = __fmul_rn(kE, __fsub_rn(__ldg(U + g), ru));
+            sV[c * P + r] = __fmul_rn(kE, __fsub_rn(__ldg(V + g), rv));
+            sI[c * P + r] = __fmul_rn(kI, __fsub_rn(__ldg(I + g), ri));
         }
-        rowf[m] = make_float4(t[0], t[1], t[2], t[3]);
+    }
+    for (int p = threadIdx.y * TX + threadIdx.x; p <= s; p += TX * TY) {
+        auto term = [&](int n) {
+            return n >= 0 && n < 2 * s ? (float)((n - s) * (n - s)) * cS : __int_as_float(0x7f800000);
+        };
+        rowf[p] = make_float4(term(2 * p), term(2 * p + 1), term(2 * p - 1), term(2 * p));
     }
     __syncthreads();
 
     const int x = bx0 + threadIdx.x;
     const int yb = by0 + threadIdx.y * TRI_R;
-    if (x >= sx || yb >= sy) return;
-    float umc[TRI_R], vmc[TRI_R], Ic[TRI_R];
+    // (pixels outside the image compute on clamped centres and store nothing)
+    f2x um[TRI_R], vm[TRI_R], ic[TRI_R];   // negated scaled centres, twice
 #pragma unroll
     for (int r = 0; r < TRI_R; r++) {
-        const int yy = min(sy - 1, yb + r);
-        const size_t o = (size_t)x + (size_t)yy * sx;
-        umc[r] = -kE * __ldg(Um + o);
-        vmc[r] = -kE * __ldg(Vm + o);
-        Ic[r] = -kI * sI[(threadIdx.y * TRI_R + r + s) * TW + threadIdx.x + s];
+        const size_t o = (size_t)min(sx - 1, x) + (size_t)min(sy - 1, yb + r) * sx;
+        const float a = __fmul_rn(-kE, __fsub_rn(__ldg(Um + o), ru)), b = __fmul_rn(-kE, __fsub_rn(__ldg(Vm + o), rv));
+        const float i0 = -sI[(threadIdx.x + s) * P + threadIdx.y * TRI_R + r + s];
+        um[r] = pk2(a, a);
+        vm[r] = pk2(b, b);
+        ic[r] = pk2(i0, i0);
     }
-    const f2x umA = pk2(umc[0], umc[1]), umB = pk2(umc[2], umc[3]);
-    const f2x vmA = pk2(vmc[0], vmc[1]), vmB = pk2(vmc[2], vmc[3]);
-    const f2x IA = pk2(Ic[0], Ic[1]), IB = pk2(Ic[2], Ic[3]);
-    const f2x kEE = pk2(kE, kE), kII = pk2(kI, kI), rr = pk2(r_, r_);
-    f2x ufA = 0, ufB = 0, vfA = 0, vfB = 0, WA = 0, WB = 0;  // 0 bits = (0.0f, 0.0f)
-    const int row0 = threadIdx.y * TRI_R;
-    // NC source columns (i .. i + NC - 1) per step: NC times the independent
-    // accumulation chains of a one-column walk, to keep the FMA pipe fed between the
-    // exp2s (three columns with the row loop unrolled four times measured fastest;
-    // the last 2s mod 3 columns go one at a time)
-    auto columns = [&](int i, auto ncols) {
-        constexpr int NC = decltype(ncols)::value;
-        const float2* col = suv + row0 * TW + threadIdx.x + s + i;
-        const float* colI = sI + row0 * TW + threadIdx.x + s + i;
-        f2x cuA[NC], cuB[NC], cvA[NC], cvB[NC], cwA[NC], cwB[NC];
+    float su[TRI_R], sv[TRI_R], sw[TRI_R];
 #pragma unroll
-        for (int c = 0; c < NC; c++) cuA[c] = cuB[c] = cvA[c] = cvB[c] = cwA[c] = cwB[c] = 0;
-        // source row m lies in output r's window when 0 <= m - r < 2s: pair A (outputs
-        // 0, 1) has none of its rows past m = 2s, pair B (outputs 2, 3) none before
-        // m = 2; those evaluations would add exact zeros and are skipped
-        auto tap = [&](int m, int c, auto doA, auto doB) {
-            const float2 uv = col[m * TW + c];
-            const float i1 = colI[m * TW + c];
-            const float4 rf = rowf[m];
-            const f2x uu = pk2(uv.x, uv.x), vv = pk2(uv.y, uv.y), ii = pk2(i1, i1);
-            if constexpr (decltype(doA)::value) {
-                const f2x du = fma2(uu, kEE, umA), dv = fma2(vv, kEE, vmA), dI = fma2(ii, kII, IA);
-                const f2x q = fma2(dI, dI, fma2(dv, dv, fma2(du, du, pk2(rf.x, rf.y))));
-                const f2x w = ex2n_2(mul2(q, rr));
-                cuA[c] = fma2(w, uu, cuA[c]);
-                cvA[c] = fma2(w, vv, cvA[c]);
-                cwA[c] = add2(cwA[c], w);
-            }
-            if constexpr (decltype(doB)::value) {
-                const f2x du = fma2(uu, kEE, umB), dv = fma2(vv, kEE, vmB), dI = fma2(ii, kII, IB);
-                const f2x q = fma2(dI, dI, fma2(dv, dv, fma2(du, du, pk2(rf.z, rf.w))));
-                const f2x w = ex2n_2(mul2(q, rr));
-                cuB[c] = fma2(w, uu, cuB[c]);
-                cvB[c] = fma2(w, vv, cvB[c]);
-                cwB[c] = add2(cwB[c], w);
-            }
+    for (int r = 0; r < TRI_R; r++) su[r] = sv[r] = sw[r] = 0.0f;
+
+    struct Pair {
+        f2x u, v, i;
+    };
+    const ulonglong2* terms = reinterpret_cast<const ulonglong2*>(rowf);
+    auto column = [&](int i) {
+        const float* cu = sU + (threadIdx.x + s + i) * P + threadIdx.y * TRI_R;
+        const int plane = TW * P;
+        f2x au[TRI_R], av[TRI_R], aw[TRI_R];
+#pragma unroll
+        for (int r = 0; r < TRI_R; r++) au[r] = av[r] = aw[r] = 0;   // 0 bits = (0.0f, 0.0f)
+        auto load = [&](int p) {
+            Pair t;
+            t.u = *reinterpret_cast<const f2x*>(cu + 2 * p);
+            t.v = *reinterpret_cast<const f2x*>(cu + plane + 2 * p);
+            t.i = *reinterpret_cast<const f2x*>(cu + 2 * plane + 2 * p);
+            return t;
         };
-        static_assert(TRI_R == 4, "the row split below assumes two output pairs");
-        using yes = std::true_type;
-        using no = std::false_type;
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-            tap(0, c, yes{}, no{});
-            tap(1, c, yes{}, no{});
+        auto weight = [&](int r, const Pair& t, f2x row) {
+            const f2x du = add2(t.u, um[r]), dv = add2(t.v, vm[r]), dI = add2(t.i, ic[r]);
+            return ex2n_2(fma2(dI, dI, fma2(dv, dv, fma2(du, du, row))));
+        };
+        auto sums = [&](int r, const Pair& t, f2x w) {
+            au[r] = fma2(w, t.u, au[r]);
+            av[r] = fma2(w, t.v, av[r]);
+            aw[r] = add2(aw[r], w);
+        };
+        auto upper = [&](const Pair& t) { return Pair{pk2(0.0f, hi2(t.u)), pk2(0.0f, hi2(t.v)), pk2(0.0f, hi2(t.i))}; };
+        auto lower = [&](const Pair& t) { return Pair{pk2(lo2(t.u), 0.0f), pk2(lo2(t.v), 0.0f), pk2(lo2(t.i), 0.0f)}; };
+        ulonglong2 f = terms[0];
+        f2x e0 = f.x, e1 = f.y;                       // the previous pair's terms
+        Pair t = load(0);                             // rows 0, 1
+        sums(0, t, weight(0, t, e0));
+        Pair h = upper(t);
+        sums(1, h, weight(1, h, e1));
+        if (s > 1) {
+            f = terms[1];
+            t = load(1);                              // rows 2, 3
+            f2x t0 = f.x, t1 = f.y;
+            sums(0, t, weight(0, t, t0));
+            sums(1, t, weight(1, t, t1));
+            sums(2, t, weight(2, t, e0));
+            h = upper(t);
+            sums(3, h, weight(3, h, e1));
+#pragma unroll TRI_UNROLL
+            for (int p = 2; p < s; p++) {
+                f = terms[p];
+                t0 = f.x;
+                t1 = f.y;
+                f = terms[p - 1];   // reloaded, not carried over: a copy per step costs more
+                e0 = f.x;
+                e1 = f.y;
+                t = load(p);
+                sums(0, t, weight(0, t, t0));
+                sums(1, t, weight(1, t, t1));
+                sums(2, t, weight(2, t, e0));
+                sums(3, t, weight(3, t, e1));
+            }
+            f = terms[s - 1];
+            e0 = f.x;
+            e1 = f.y;
         }
-#pragma unroll 4
-        for (int m = 2; m <= 2 * s; m++) {
-#pragma unroll
-            for (int c = 0; c < NC; c++) tap(m, c, yes{}, yes{});
+        f = terms[s];
+        t = load(s);                                  // rows 2s, 2s + 1
+        const f2x last = f.y;
+        h = lower(t);
+        sums(1, h, weight(1, h, last));
+        sums(2, t, weight(2, t, e0));
+        if (s > 1) {
+            sums(3, t, weight(3, t, e1));
+        } else {
+            h = upper(t);
+            sums(3, h, weight(3, h, e1));
         }
+        t = load(s + 1);                              // row 2s + 2
+        h = lower(t);
+        sums(3, h, weight(3, h, last));
+        const float wi = exp2f(-(float)(i * i) * cS);
 #pragma unroll
-        for (int c = 0; c < NC; c++) {
-            tap(2 * s + 1, c, no{}, yes{});
-            tap(2 * s + 2, c, no{}, yes{});
-        }
-#pragma unroll
-        for (int c = 0; c < NC; c++) {
-            const float wi = exp2f(-(float)((i + c) * (i + c)) * cS);
-            const f2x wi2 = pk2(wi, wi);
-            ufA = fma2(wi2, cuA[c], ufA);
-            ufB = fma2(wi2, cuB[c], ufB);
-            vfA = fma2(wi2, cvA[c], vfA);
-            vfB = fma2(wi2, cvB[c], vfB);
-            WA = fma2(wi2, cwA[c], WA);
-            WB = fma2(wi2, cwB[c], WB);
+        for (int r = 0; r < TRI_R; r++) {
+            su[r] = __fmaf_rn(wi, lo2(au[r]) + hi2(au[r]), su[r]);
+            sv[r] = __fmaf_rn(wi, lo2(av[r]) + hi2(av[r]), sv[r]);
+            sw[r] = __fmaf_rn(wi, lo2(aw[r]) + hi2(aw[r]), sw[r]);
         }
     };
-    int i = -s;
-    for (; i + 3 <= s; i += 3) columns(i, std::integral_constant<int, 3>{});
-    for (; i < s; i++) columns(i, std::integral_constant<int, 1>{});
-    const float uf[TRI_R] = {lo2(ufA), hi2(ufA), lo2(ufB), hi2(ufB)};
-    const float vf[TRI_R] = {lo2(vfA), hi2(vfA), lo2(vfB), hi2(vfB)};
-    const float W[TRI_R] = {lo2(WA), hi2(WA), lo2(WB), hi2(WB)};
+    // group z: columns [-s, 0) or [0, s)
+    for (int k = 0; k < s; k++) column(threadIdx.z ? k : k - s);
+
+    __syncthreads();   // every group is done with the tile
+    float* part = sU;  // [3 * TRI_R][TY * TX]
+    const int tid = threadIdx.y * TX + threadIdx.x;
+    if (threadIdx.z) {
+#pragma unroll
+        for (int r = 0; r < TRI_R; r++) {
+            part[(3 * r + 0) * TX * TY + tid] = su[r];
+            part[(3 * r + 1) * TX * TY + tid] = sv[r];
+            part[(3 * r + 2) * TX * TY + tid] = sw[r];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.z || x >= sx || yb >= sy) return;
+    const float inv_k = __frcp_rn(kE);
 #pragma unroll
     for (int r = 0; r < TRI_R; r++) {
+        const float w = sw[r] + part[(3 * r + 2) * TX * TY + tid];
+        const float mu = (su[r] + part[(3 * r + 0) * TX * TY + tid]) * inv_k;
+        const float mv = (sv[r] + part[(3 * r + 1) * TX * TY + tid]) * inv_k;
         if (yb + r < sy) {
             const size_t o = (size_t)x + (size_t)(yb + r) * sx;
-            const float Wc = fmaxf(1e-5f, W[r]);
-            Uo[o] = uf[r] / Wc;
-            Vo[o] = vf[r] / Wc;
+            // sum of w u over max(1e-5, sum of w), with u = ru + the centred scaled sample / kE
+            Uo[o] = w < 1e-5f ? __fdiv_rn(__fmaf_rn(ru, w, mu), 1e-5f) : ru + __fdiv_rn(mu, w);
+            Vo[o] = w < 1e-5f ? __fdiv_rn(__fmaf_rn(rv, w, mv), 1e-5f) : rv + __fdiv_rn(mv, w);
         }
     }
 }
@@ -964,14 +1025,17 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
 // with intensities divided by 255 folded into cI.
 struct TriCoef {
     float cE, cI, cS;
+    float kE, kI;   // sqrt(cE), sqrt(cI)
 };
-__host__ __device__ inline TriCoef tri_coef(float sigmaEPE2, float sigmaI2, float sigmaS2)
+inline TriCoef tri_coef(float sigmaEPE2, float sigmaI2, float sigmaS2)
 {
     const float LOG2E = 1.4426950408889634f;
     TriCoef t;
     t.cE = LOG2E / (2.0f * sigmaEPE2);
     t.cI = LOG2E / (2.0f * sigmaI2 * 255.0f * 255.0f);
     t.cS = LOG2E / (2.0f * sigmaS2);
+    t.kE = (float)__builtin_sqrt((double)t.cE);
+    t.kI = (float)__builtin_sqrt((double)t.cI);
     return t;
 }
 

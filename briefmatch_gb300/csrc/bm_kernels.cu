@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256) k_features(const float* __restrict__ I, u
 //
 // Reading two keys per 4 bytes halves the load requests that bound the float form
 // (70 % of the load unit's rate, and 13 % of its instructions branches around the
-// strip's end): 144 -> 98 us at 2969x1264 N128, 280 -> 194 at N256, 980 -> 572 at
+// strip's end): 144 -> 99 us at 2969x1264 N128, 280 -> 191 at N256, 980 -> 557 at
 // 3136x1764 N512.  What bounds it now is issue; without the ties' repair and detection
 // it would be 68 us at N128.  Measured beside it: four pixels per thread (32 columns
 // on, sharing the addresses) 101, 203 and 606 us, its code twice as long for the
@@ -440,14 +440,18 @@ __global__ void __launch_bounds__(256) k_median_pass(const float* __restrict__ i
     }
 }
 
-__global__ void __launch_bounds__(TX * TRI_TY) k_trilateral_x2(const float* __restrict__ U, const float* __restrict__ V,
-                                                               const float* __restrict__ Um, const float* __restrict__ Vm,
-                                                               const float* __restrict__ I, float* __restrict__ Uo,
-                                                               float* __restrict__ Vo, int sx, int sy, int s,
-                                                               float cE, float cI, float cS)
+template <int TY>
+__global__ void __launch_bounds__(TX * TY * TRI_G, 8 / TY) k_trilateral(const float* __restrict__ U,
+                                                                       const float* __restrict__ V,
+                                                                       const float* __restrict__ Um,
+                                                                       const float* __restrict__ Vm,
+                                                                       const float* __restrict__ I,
+                                                                       float* __restrict__ Uo, float* __restrict__ Vo,
+                                                                       int sx, int sy, int s, float kE, float kI, float cS)
 {
     extern __shared__ float4 smem4[];
-    trilateral_block(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, cE, cI, cS, blockIdx.x * TX, blockIdx.y * TRI_BY, smem4);
+    trilateral_block<TY>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, kE, kI, cS, blockIdx.x * TX, blockIdx.y * tri_rows(TY),
+                         smem4);
 }
 
 __global__ void __launch_bounds__(256) k_trilateral_global(const float* __restrict__ U, const float* __restrict__ V,
@@ -688,12 +692,26 @@ cudaError_t ensure_trilateral_smem(int s)
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    const int need = (int)tri_smem_bytes(s);
+    const int need = (int)tri_smem_bytes(s, 8);
     std::lock_guard<std::mutex> lock(mu);
     if (need <= granted[dev]) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_trilateral_x2, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    e = cudaFuncSetAttribute(k_trilateral<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trilateral<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trilateral<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
     if (e == cudaSuccess) granted[dev] = need;
     return e;
+}
+
+// Thread rows per block.  A block of 8 (16 warps, an SM's registers) has the smallest
+// halo per output and is the fastest wherever the grid is several waves deep; below two
+// 32 x 32 tiles per SM the waves' rounding costs more than the halo, and smaller blocks,
+// as many per SM as fill it, take over while their tiles fit side by side (584x388:
+// 109 -> 101 us with the median, 777x333: 93 -> 88; but 1024x436, 2.9 tiles per SM: 358 -> 369).
+static int trilateral_rows(int sx, int sy, int s, int sms)
+{
+    const size_t per_sm = 224 * 1024;
+    if ((long)((sx + TX - 1) / TX) * ((sy + 31) / 32) >= 2L * sms) return 8;
+    return 4 * tri_smem_bytes(s, 2) <= per_sm ? 2 : 2 * tri_smem_bytes(s, 4) <= per_sm ? 4 : 8;
 }
 
 cudaError_t trilateral(const float* U, const float* V, const float* Um, const float* Vm,
@@ -702,12 +720,23 @@ cudaError_t trilateral(const float* U, const float* V, const float* Um, const fl
 {
     const TriCoef tc = tri_coef(sigmaEPE2, sigmaI2, sigmaS2);
     const float cE = tc.cE, cI = tc.cI, cS = tc.cS;
-    const size_t smem = tri_smem_bytes(s);
-    if (smem <= 220 * 1024) {
+    if (s <= TRI_MAX_S) {
         cudaError_t e = ensure_trilateral_smem(s);
         if (e != cudaSuccess) return e;
-        dim3 g((sx + TX - 1) / TX, (sy + TRI_BY - 1) / TRI_BY);
-        k_trilateral_x2<<<g, dim3(TX, TRI_TY), smem, st>>>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, cE, cI, cS);
+        auto launch = [&](auto kernel, int ty) {
+            dim3 g((sx + TX - 1) / TX, (sy + tri_rows(ty) - 1) / tri_rows(ty));
+            kernel<<<g, dim3(TX, ty, TRI_G), tri_smem_bytes(s, ty), st>>>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, tc.kE, tc.kI,
+                                                                         cS);
+        };
+        int dev = 0, sms = 0;
+        e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        switch (trilateral_rows(sx, sy, s, sms)) {
+        case 2: launch(k_trilateral<2>, 2); break;
+        case 4: launch(k_trilateral<4>, 4); break;
+        default: launch(k_trilateral<8>, 8); break;
+        }
     } else {
         k_trilateral_global<<<grid2d(sx, sy), dim3(TX, TY), 0, st>>>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, cE, cI, cS);
     }
