@@ -559,6 +559,31 @@ __host__ __device__ constexpr uint32_t umma_idesc(int m, int n)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// This warp's 32 TMEM lanes, N columns from `taddr`, one lane per thread.
+template <int N>
+__device__ __forceinline__ void umma_load(uint32_t (&r)[N], uint32_t taddr)
+{
+    if constexpr (N == 32) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
+              "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
+              "=r"(r[30]), "=r"(r[31])
+            : "r"(taddr));
+    } else {
+        static_assert(N == 16, "N is 16 or 32 columns");
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(taddr));
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
 template <int EPI, int N>
 __global__ void __launch_bounds__(128) k_conv_umma(const __grid_constant__ CUtensorMap tmX,
                                                    const __grid_constant__ CUtensorMap tmW,
@@ -648,27 +673,7 @@ __global__ void __launch_bounds__(128) k_conv_umma(const __grid_constant__ CUten
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (done && s_ok) {
         uint32_t r[N];
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-        if constexpr (N == 32) {
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-                "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-                  "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-                  "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                : "r"(taddr));
-        } else {
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-                "[%16];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-                  "=r"(r[15])
-                : "r"(taddr));
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        umma_load<N>(r, tmem + ((uint32_t)(warp * 32) << 16));
         const int x = x0 + warp * 32 + lane;
         if (x < w) {
             const size_t pix = (size_t)row * w + x;
@@ -712,6 +717,173 @@ __global__ void __launch_bounds__(128) k_conv_umma(const __grid_constant__ CUten
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem) : "memory");
 }
 
+// ---------------------------------------------------------------------------
+// tcgen05 weight gradient of a 3x3 layer:
+//   dW[co][tap][ci] += sum over cells p of dY[p][co] * X[p + shift(tap)][ci],
+//   db[co] += sum over p of dY[p][co].
+// The cells are the reduction: both operands are MN-major (channels contiguous), as TMA
+// lands them -- per 128 cells of an image row nine shifted X tiles of 128 x 32 channels
+// (zero outside the image: the map is 4-D, so a tap's row cannot run into the next
+// image) and one dY tile of 128 x NCH.  Four X tiles 8 KB apart make the M = 128 rows
+// (tap, ci) of one MMA, so three accumulators (taps 0-3, 4-7 and 8) of NCH columns each
+// stay in tensor memory over all of a CTA's tiles, 24 MMAs of K = 16 cells per tile.  A
+// tile of ones behind tap 8 gives the bias gradient as one more row; rows past it are
+// not read out.  Two stages: the copies of the next tile run under the MMAs of this one.
+// At the end each warp adds its accumulator lanes (one tap, 32 input channels) to the
+// FP32 gradient, 128 contiguous bytes per output channel.
+//
+// It replaces mma.sync tiles with transposed shared-memory staging and an atomic flush
+// per 128 cells, which kept the L1 60-80 % busy: per layer of 32 images of 128 x 96 cells
+// 133 us (dilation 1) to 233 us (dilation 8), now 35 us, 245 MB of copies from L2.
+// ---------------------------------------------------------------------------
+constexpr uint32_t WG_ONES = 9, WG_TILES = 10;   // tile 9 holds ones
+__host__ __device__ constexpr uint32_t wg_stage(int nch) { return WG_TILES * U_TAP_A + (uint32_t)(UM * nch * 2); }
+// two stages, and room for the last MMA's unused rows past them
+constexpr size_t wgrad_umma_smem(int nch) { return 1024 + 2 * (size_t)wg_stage(nch) + 2 * U_TAP_A; }
+
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
+                                            uint64_t* bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+        ::"r"(s_addr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(s_addr(bar))
+        : "memory");
+}
+// Shared-memory matrix descriptor, MN-major: rows (K) of `width` channels contiguous and
+// swizzled by their width, 8-row groups 8 rows apart, the next `width` of MN `lead` bytes on.
+template <int WIDTH>
+__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr, uint32_t lead)
+{
+    static_assert(WIDTH == 16 || WIDTH == 32, "32- or 64-byte swizzle");
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+    d |= (uint64_t)((lead >> 4) & 0x3FFF) << 16;      // leading byte offset: along MN
+    d |= (uint64_t)(WIDTH * 2 * 8 >> 4) << 32;        // stride byte offset: along K
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)(WIDTH == 32 ? 4 : 6) << 61;       // swizzle mode
+    return d;
+}
+
+template <int NCH>
+__global__ void __launch_bounds__(128) k_wgrad_umma(const __grid_constant__ CUtensorMap tmX,
+                                                    const __grid_constant__ CUtensorMap tmD, float* __restrict__ dW,
+                                                    float* __restrict__ db, int h, int w, int rows, int dil,
+                                                    int cout_real, int* __restrict__ err)
+{
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t full[2], empty[2], done;
+    __shared__ uint32_t s_tmem;
+    __shared__ volatile int s_fail;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tiles_x = (w + UM - 1) / UM;
+    const int tiles = tiles_x * rows;
+
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 2; k++) {
+            mbar_init(&full[k], 1);
+            mbar_init(&empty[k], 1);
+        }
+        mbar_init(&done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_fail = 0;
+    }
+    for (int k = 0; k < 2; k++) {   // the tiles of ones (the same under any swizzle)
+        uint32_t* ones = reinterpret_cast<uint32_t*>(sm + k * wg_stage(NCH) + WG_ONES * U_TAP_A);
+        for (uint32_t i = threadIdx.x; i < U_TAP_A / 4; i += 128) ones[i] = 0x3F803F80u;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(s_addr(&s_tmem))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+
+    if (threadIdx.x == 0) {
+        // producer
+        int k = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, k++) {
+            const int st = k & 1;
+            if (k >= 2 && !mbar_wait(&empty[st], (uint32_t)((k >> 1) - 1) & 1u, U_POLLS)) {
+                atomicExch(err, 2);
+                s_fail = 1;
+            }
+            if (s_fail) break;
+            const int row = tile / tiles_x, x0 = (tile - row * tiles_x) * UM;
+            const int b = row / h, y = row - b * h;
+            unsigned char* base = sm + st * wg_stage(NCH);
+            mbar_expect_tx(&full[st], 9 * U_TAP_A + UM * NCH * 2);
+            for (int t = 0; t < 9; t++)
+                tma_load_4d(base + t * U_TAP_A, &tmX, 0, x0 + (t % 3 - 1) * dil, y + (t / 3 - 1) * dil, b, &full[st]);
+            tma_load_3d(base + WG_TILES * U_TAP_A, &tmD, 0, x0, row, &full[st]);
+        }
+    } else if (threadIdx.x == 32) {
+        // MMA issuer
+        constexpr uint32_t idesc = umma_idesc(UM, NCH) | (1u << 15) | (1u << 16);   // both operands MN-major
+        int k = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, k++) {
+            const int st = k & 1;
+            if (!mbar_wait(&full[st], (uint32_t)(k >> 1) & 1u, U_POLLS)) {
+                // give this CTA's copies one more bounded wait, then let everybody go
+                atomicExch(err, 1);
+                s_fail = 1;
+                mbar_wait(&full[st], (uint32_t)(k >> 1) & 1u, U_POLLS);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t base = s_addr(sm + st * wg_stage(NCH)), dbase = base + WG_TILES * U_TAP_A;
+            for (int kk = 0; kk < UM / 16; kk++) {   // 16 cells per MMA
+                const uint64_t bd = umma_desc_mn<NCH>(dbase + kk * 16 * NCH * 2, UM * NCH * 2);
+#pragma unroll
+                for (int g = 0; g < 3; g++) {
+                    const uint64_t ad = umma_desc_mn<32>(base + g * 4 * U_TAP_A + kk * 16 * 64, U_TAP_A);
+                    asm volatile(
+                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                        ::"r"(tmem + 32 * g), "l"(ad), "l"(bd), "r"(idesc), "r"((k | kk) ? 1u : 0u)
+                        : "memory");
+                }
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                         ::"r"(s_addr(&empty[st])) : "memory");
+        }
+        // arrives once the MMAs issued so far are done, also after a wait that gave up
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                     ::"r"(s_addr(&done)) : "memory");
+    }
+    __syncwarp();
+    // tcgen05.ld is warp-collective: the block agrees on one outcome of the wait.  The
+    // limit covers all of the CTA's tiles.
+    const bool mine = mbar_wait(&done, 0, 4 * U_POLLS);
+    const bool ok = __syncthreads_and(mine ? 1 : 0) != 0 && !s_fail;
+    if (!ok && threadIdx.x == 0) atomicExch(err, 2);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (ok) {
+#pragma unroll 1
+        for (int g = 0; g < 3; g++) {
+            const int tap = 4 * g + warp;   // tap 9: the row of ones
+            if (tap > 9) continue;
+            uint32_t r[NCH];
+            umma_load<NCH>(r, tmem + ((uint32_t)(warp * 32) << 16) + 32 * g);
+#pragma unroll
+            for (int co = 0; co < NCH; co++) {
+                if (co >= cout_real) continue;
+                if (tap < 9)
+                    atomicAdd(dW + ((size_t)co * 9 + tap) * 32 + lane, __uint_as_float(r[co]));
+                else if (lane == 0)
+                    atomicAdd(db + co, __uint_as_float(r[co]));
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem) : "memory");
+}
+
 // cuTensorMapEncodeTiled, fetched through the runtime (the library does not link the
 // driver library itself).
 typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -751,6 +923,21 @@ bool encode_map(CUtensorMap* map, const void* base, uint64_t d1, uint64_t d2, ui
 bool act_map(CUtensorMap* map, const __nv_bfloat16* X, int B, int h, int w)
 {
     return encode_map(map, X, (uint64_t)w, (uint64_t)B * h, UM, 1);
+}
+// A BF16 tensor map for the weight gradient: dims {nch, w, h, b} (b omitted when 0), box
+// {nch, UM, 1, 1}, rows swizzled by their width (64 or 32 bytes), zero fill.
+bool wgrad_map(CUtensorMap* map, const void* base, int nch, uint64_t w, uint64_t h, uint64_t b)
+{
+    EncodeTiled enc = encoder();
+    if (!enc) return false;
+    const uint64_t px = (uint64_t)nch * 2;
+    const cuuint64_t dims[4] = {(cuuint64_t)nch, w, h, b};
+    const cuuint64_t strides[3] = {px, px * w, px * w * h};
+    const cuuint32_t box[4] = {(cuuint32_t)nch, UM, 1, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, b ? 4 : 3, const_cast<void*>(base), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, nch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 // Weights [9][n][32] as the B operand (all nine taps in one copy).
 bool weight_map(CUtensorMap* map, const __nv_bfloat16* W, int n) { return encode_map(map, W, (uint64_t)n, 9, n, 9); }
@@ -832,24 +1019,7 @@ __device__ __forceinline__ void umma_epilogue(uint32_t taddr, const float* __res
                                               size_t pix, bool in_image, int cout_real, int out_stride)
 {
     uint32_t r[N];
-    if constexpr (N == 32) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-              "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]),
-              "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]),
-              "=r"(r[30]), "=r"(r[31])
-            : "r"(taddr));
-    } else {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(taddr));
-    }
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    umma_load<N>(r, taddr);
     if (!in_image) return;
     if constexpr (EPI == EPI_LINEAR_F32) {
         float* o = reinterpret_cast<float*>(out) + pix * out_stride;
@@ -1020,6 +1190,8 @@ cudaError_t conv_smem_optin()
         set((const void*)k_conv_umma<EPI_MASK_BF16, 32>, umma_smem(32)),
         set((const void*)k_conv_umma<EPI_LINEAR_F32, 16>, umma_smem(16)),
         set((const void*)k_net_fused, umma_smem(32)),
+        set((const void*)k_wgrad_umma<32>, wgrad_umma_smem(32)),
+        set((const void*)k_wgrad_umma<16>, wgrad_umma_smem(16)),
     };
     for (cudaError_t x : es)
         if (x != cudaSuccess) return x;
@@ -1078,6 +1250,9 @@ struct bm_net {
     CUtensorMap map_in;
     CUtensorMap map_act[NL - 1];
     CUtensorMap map_dy[2];
+    CUtensorMap map_in4, map_act4[NL - 1];   // the layers' inputs, images apart (weight gradient)
+    CUtensorMap map_dy16;                    // the head's gradient, 16 channels
+    int num_sms = 1;
 };
 
 namespace {
@@ -1126,6 +1301,8 @@ bool ensure_act_maps(bm_net* n, uint32_t B, uint32_t h, uint32_t w)
     bool ok = act_map(&n->map_in, n->d_in, Bi, hi, wi);
     for (int l = 0; ok && l < NL - 1; l++) ok = act_map(&n->map_act[l], n->d_act[l], Bi, hi, wi);
     for (int k = 0; ok && k < 2; k++) ok = act_map(&n->map_dy[k], n->d_dy[k], Bi, hi, wi);
+    ok = ok && wgrad_map(&n->map_in4, n->d_in, 32, w, h, B) && wgrad_map(&n->map_dy16, n->d_dy[0], 16, w, (uint64_t)B * h, 0);
+    for (int l = 0; ok && l < NL - 1; l++) ok = wgrad_map(&n->map_act4[l], n->d_act[l], 32, w, h, B);
     if (!ok) return false;
     n->map_B = B;
     n->map_h = h;
@@ -1191,6 +1368,31 @@ bm_status forward(bm_net* n, uint32_t B, uint32_t h, uint32_t w, cudaStream_t st
     return BM_OK;
 }
 
+// Weight and bias gradient of layer l from its output gradient in d_dy[cur] (the head's:
+// 16 channels in d_dy[0]), added to the FP32 gradient vector.
+bm_status weight_grad(bm_net* n, int l, int cur, int B, int h, int w, cudaStream_t st)
+{
+    const __nv_bfloat16* X = l == 0 ? n->d_in : n->d_act[l - 1];
+    float* dW = n->d_grad + n->poff[l];
+    float* db = dW + layer_w_count(l);
+    if (n->umma) {
+        const CUtensorMap& mx = l == 0 ? n->map_in4 : n->map_act4[l - 1];
+        const int rows = B * h, tiles = ((w + UM - 1) / UM) * rows, grid = std::min(tiles, n->num_sms);
+        if (l == NL - 1)
+            k_wgrad_umma<16><<<grid, 128, wgrad_umma_smem(16), st>>>(mx, n->map_dy16, dW, db, h, w, rows, DIL[l], COUT_R[l],
+                                                                     n->d_err);
+        else
+            k_wgrad_umma<32><<<grid, 128, wgrad_umma_smem(32), st>>>(mx, n->map_dy[cur], dW, db, h, w, rows, DIL[l],
+                                                                     COUT_R[l], n->d_err);
+        BN_CUDA(cudaGetLastError());
+    } else if (l == NL - 1) {
+        BN_CUDA((launch_wgrad<32, 16, 1>(X, n->d_dy[0], 16, B, h, w, dW, db, 32, 3, st)));
+    } else {
+        BN_CUDA(conv_wgrad(l, X, n->d_dy[cur], B, h, w, dW, db, st));
+    }
+    return BM_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1252,6 +1454,7 @@ bm_status bm_net_create(uint32_t max_batch, uint32_t max_h4, uint32_t max_w4, bm
         if (coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_net_fused, 128, umma_smem(32)) == cudaSuccess)
             n->fused_grid_max = occ * sms;
         n->fused = false;
+        n->num_sms = std::max(1, sms);
     }
     cudaMemset(n->d_m, 0, off * 4);
     cudaMemset(n->d_v, 0, off * 4);
@@ -1462,14 +1665,14 @@ bm_status bm_net_train_step(bm_net* n, uint32_t B, uint32_t h, uint32_t w, const
     BN_CUDA(cudaGetLastError());
     // layer 5: dY (16 padded channels, 3 real) -> dW5, and dX into the ReLU mask of act[4]
     float* g = n->d_grad;
-    BN_CUDA((launch_wgrad<32, 16, 1>(n->d_act[4], n->d_dy[0], 16, Bi, hi, wi, g + n->poff[5],
-                                     g + n->poff[5] + layer_w_count(5), 32, 3, st)));
+    s = weight_grad(n, 5, 0, Bi, hi, wi, st);
+    if (s != BM_OK) return s;
     BN_CUDA((launch_conv<16, 32, EPI_MASK_BF16, 1>(n->d_dy[0], n->d_wb[5], nullptr, n->d_act[4], n->d_dy[1], Bi, hi, wi,
                                                    32, 32, st)));
     int cur = 1;
     for (int l = 4; l >= 1; l--) {
-        BN_CUDA(conv_wgrad(l, n->d_act[l - 1], n->d_dy[cur], Bi, hi, wi, g + n->poff[l], g + n->poff[l] + layer_w_count(l),
-                           st));
+        s = weight_grad(n, l, cur, Bi, hi, wi, st);
+        if (s != BM_OK) return s;
         if (n->umma)
             BN_CUDA((launch_conv_umma<EPI_MASK_BF16, 32>(n->map_dy[cur], n->map_wb[l], nullptr, n->d_act[l - 1],
                                                           n->d_dy[cur ^ 1], Bi, hi, wi, DIL[l], 32, 32, n->d_err, st)));
@@ -1477,7 +1680,8 @@ bm_status bm_net_train_step(bm_net* n, uint32_t B, uint32_t h, uint32_t w, const
             BN_CUDA(conv_bwd_data(l, n->d_dy[cur], n->d_wb[l], n->d_act[l - 1], n->d_dy[cur ^ 1], Bi, hi, wi, st));
         cur ^= 1;
     }
-    BN_CUDA(conv_wgrad(0, n->d_in, n->d_dy[cur], Bi, hi, wi, g + n->poff[0], g + n->poff[0] + layer_w_count(0), st));
+    s = weight_grad(n, 0, cur, Bi, hi, wi, st);
+    if (s != BM_OK) return s;
     if (d_grad_out) BN_CUDA(cudaMemcpyAsync(d_grad_out, g, n->nparam * 4, cudaMemcpyDeviceToDevice, st));
     if (lr > 0) {
         n->step++;
