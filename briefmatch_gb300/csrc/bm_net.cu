@@ -487,18 +487,14 @@ cudaError_t conv_wgrad(int l, const __nv_bfloat16* X, const __nv_bfloat16* dY, i
 }
 
 // ---------------------------------------------------------------------------
-// tcgen05 implicit-GEMM 3x3 convolution.  One CTA of 128 threads per run of UM = 128
-// consecutive cells of one image row: D[cell][co] = sum over taps t and input channels
-// ci of X[cell + shift(t)][ci] * W[t][co][ci].  Shared memory holds the nine taps'
-// A tiles (128 cells x 32 channels, 8 KB each) and the weights B (9 x N x 32); both
-// arrive by TMA with 64-byte swizzling, which is the canonical K-major layout the MMA
-// descriptors name (rows of 64 bytes, 8-row groups 512 bytes apart).  A tap whose
-// source row lies outside the image is neither loaded nor multiplied (its A tile would
-// be zeros); a tap shifted past the left or right edge reads TMA's zero fill.  Thread 0
-// issues the copies and the 18 MMAs (M=128, N, K=16) into a 32-column TMEM
-// accumulator; all four warps then read their 32 TMEM lanes (cells) and apply the
-// epilogue.  Every wait is bounded: a wait that gives up records an error word and the
-// CTA still frees its tensor memory before it returns.
+// tcgen05 implicit-GEMM 3x3 convolution.  The GEMM's rows are UM = 128 consecutive
+// cells of one image row: D[cell][co] = sum over taps t and input channels ci of
+// X[cell + shift(t)][ci] * W[t][co][ci].  Operands arrive by TMA with 64-byte swizzling,
+// the canonical K-major layout the MMA descriptors name (rows of 64 bytes, 8-row groups
+// 512 bytes apart); a source row outside the image is neither loaded nor multiplied (it
+// would be zeros), a tap shifted past the left or right edge reads TMA's zero fill.
+// Accumulation is FP32 in tensor memory.  Every wait is bounded: a wait that gives up
+// records an error word and the CTA still frees its tensor memory before it returns.
 // ---------------------------------------------------------------------------
 constexpr int UM = 128;                                 // cells per CTA (MMA M)
 constexpr uint32_t U_TAP_A = UM * 32 * 2;               // bytes of one tap's A tile
@@ -584,37 +580,66 @@ __device__ __forceinline__ void umma_load(uint32_t (&r)[N], uint32_t taddr)
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// One layer.  A persistent CTA walks its tiles with six warps: warp 4 copies (the three
+// source rows of a tile, 128 + 2 dil cells each: the three horizontal taps are the same
+// rows read from 0, dil and 2 dil cells on, 27 KB instead of nine 8 KB tiles), warp 5
+// issues the 18 MMAs (M = 128, N, K = 16), warps 0-3 read the accumulator's lanes and
+// write the outputs.  Three stages of copies and two accumulators keep the three at
+// work on different tiles; the weights are loaded once.  Two CTAs share an SM.
+//
+// With `chained` the launch may start while the layer before it is still running
+// (programmatic dependent launch): barriers, tensor memory and weights are set up
+// meanwhile, and the copies begin once that layer is complete.  The trigger comes after
+// the wait, so whatever ran before that layer -- the packing of the weights -- is
+// complete when this one starts.
+//
+// 32 images of 128 x 96 cells, 32 -> 32 channels: 45.5 us with one CTA per tile and nine
+// copies, one layer of one 256 x 109 image 7.6 us.
+constexpr int CV_STAGES = 3, CV_THREADS = 192;
+constexpr uint32_t CV_ROW = (UM + 16) * 64;      // a source row's cells, dilation up to 8
+constexpr uint32_t CV_STAGE = 3 * CV_ROW;
+constexpr size_t conv_umma_smem(int n) { return 1024 + CV_STAGES * (size_t)CV_STAGE + 9 * (size_t)n * 64; }
+
 template <int EPI, int N>
-__global__ void __launch_bounds__(128) k_conv_umma(const __grid_constant__ CUtensorMap tmX,
-                                                   const __grid_constant__ CUtensorMap tmW,
-                                                   const float* __restrict__ bias,
-                                                   const __nv_bfloat16* __restrict__ act, void* __restrict__ out,
-                                                   int h, int w, int dil, int cout_real, int out_stride,
-                                                   int* __restrict__ err)
+__global__ void __launch_bounds__(CV_THREADS) k_conv_umma(const __grid_constant__ CUtensorMap tmX,
+                                                          const __grid_constant__ CUtensorMap tmW,
+                                                          const float* __restrict__ bias,
+                                                          const __nv_bfloat16* __restrict__ act, void* __restrict__ out,
+                                                          int h, int w, int rows, int dil, int cout_real, int out_stride,
+                                                          int chained, int* __restrict__ err)
 {
     static_assert(N == 16 || N == 32, "N is 16 or 32 output channels");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* sA = sm;                     // 9 taps x 8 KB
-    unsigned char* sB = sm + 9 * U_TAP_A;       // 9 taps x N rows x 64 B
-    __shared__ __align__(8) uint64_t bar_load, bar_mma;
+    unsigned char* sB = sm + CV_STAGES * CV_STAGE;   // 9 taps x N rows x 64 B
+    __shared__ __align__(8) uint64_t full[CV_STAGES], empty[CV_STAGES], acc_full[2], acc_empty[2], bar_w, done;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_ok;
+    __shared__ volatile int s_fail;
 
-    const int tiles_x = (w + UM - 1) / UM;
-    const int row = blockIdx.x / tiles_x;               // image row over the batch, b * h + y
-    const int x0 = (blockIdx.x - row * tiles_x) * UM;
-    const int y = row % h;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tiles_x = (w + UM - 1) / UM;
+    const int tiles = tiles_x * rows;               // rows: image rows over the batch, b * h + y
+    auto fail = [&](int code) {
+        atomicExch(err, code);
+        s_fail = 1;
+    };
 
     if (threadIdx.x == 0) {
-        mbar_init(&bar_load, 1);
-        mbar_init(&bar_mma, 1);
+        for (int k = 0; k < CV_STAGES; k++) {
+            mbar_init(&full[k], 1);
+            mbar_init(&empty[k], 1);
+        }
+        for (int k = 0; k < 2; k++) {
+            mbar_init(&acc_full[k], 1);
+            mbar_init(&acc_empty[k], 4);
+        }
+        mbar_init(&bar_w, 1);
+        mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        s_ok = 1;
+        s_fail = 0;
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 32;" ::"r"(s_addr(&s_tmem))
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;" ::"r"(s_addr(&s_tmem))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -623,59 +648,99 @@ __global__ void __launch_bounds__(128) k_conv_umma(const __grid_constant__ CUten
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
 
-    if (threadIdx.x == 0) {
-        uint32_t taps = 0, bytes = 9u * N * 64;
-        for (int t = 0; t < 9; t++) {
-            const int r = y + (t / 3 - 1) * dil;
-            if (r >= 0 && r < h) {
-                taps |= 1u << t;
-                bytes += U_TAP_A;
+    if (warp == 4) {
+        if (lane == 0) {   // copies
+            auto weights = [&]() {
+                mbar_expect_tx(&bar_w, 9u * N * 64);
+                tma_load_3d(sB, &tmW, 0, 0, 0, &bar_w);
+            };
+            if (chained) weights();
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+            if (!chained) weights();
+            int k = 0;
+            for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, k++) {
+                const int st = k % CV_STAGES, use = k / CV_STAGES;
+                if (use > 0 && !mbar_wait(&empty[st], (uint32_t)(use - 1) & 1u, U_POLLS)) fail(2);
+                if (s_fail) break;
+                const int row = tile / tiles_x, x0 = (tile - row * tiles_x) * UM;
+                const int y = row % h;
+                uint32_t bytes = 0;
+                for (int v = -1; v <= 1; v++)
+                    if (y + v * dil >= 0 && y + v * dil < h) bytes += (uint32_t)(UM + 2 * dil) * 64;
+                mbar_expect_tx(&full[st], bytes);
+                for (int v = -1; v <= 1; v++)
+                    if (y + v * dil >= 0 && y + v * dil < h)
+                        tma_load_3d(sm + st * CV_STAGE + (v + 1) * CV_ROW, &tmX, 0, x0 - dil, row + v * dil, &full[st]);
             }
+            // this CTA's copies land before it leaves, whatever happened
+            mbar_wait(&bar_w, 0, U_POLLS);
+            for (int j = k > CV_STAGES ? k - CV_STAGES : 0; j < k; j++)
+                mbar_wait(&full[j % CV_STAGES], (uint32_t)(j / CV_STAGES) & 1u, U_POLLS);
         }
-        mbar_expect_tx(&bar_load, bytes);
-        tma_load_3d(sB, &tmW, 0, 0, 0, &bar_load);
-        for (int t = 0; t < 9; t++)
-            if (taps >> t & 1u)
-                tma_load_3d(sA + t * U_TAP_A, &tmX, 0, x0 + (t % 3 - 1) * dil, row + (t / 3 - 1) * dil, &bar_load);
-        if (mbar_wait(&bar_load, 0, U_POLLS)) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    } else if (warp == 5) {
+        if (lane == 0) {   // MMAs
             constexpr uint32_t idesc = umma_idesc(UM, N);
-            uint32_t acc = 0;
-            for (int t = 0; t < 9; t++) {
-                if (!(taps >> t & 1u)) continue;
-                const uint32_t a0 = s_addr(sA + t * U_TAP_A), b0 = s_addr(sB + t * N * 64);
-#pragma unroll
-                for (int kh = 0; kh < 2; kh++) {  // K = 16 channels (32 bytes) per MMA
-                    const uint64_t ad = umma_desc(a0 + kh * 32), bd = umma_desc(b0 + kh * 32);
-                    asm volatile(
-                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                        ::"r"(tmem), "l"(ad), "l"(bd), "r"(idesc), "r"(acc)
-                        : "memory");
-                    acc = 1;
+            asm volatile("griddepcontrol.wait;" ::: "memory");   // the bounded waits count from here
+            if (!mbar_wait(&bar_w, 0, U_POLLS)) fail(1);
+            int k = 0;
+            for (int tile = blockIdx.x; tile < tiles && !s_fail; tile += gridDim.x, k++) {
+                const int st = k % CV_STAGES, acc = k & 1;
+                if ((k >= 2 && !mbar_wait(&acc_empty[acc], (uint32_t)((k >> 1) - 1) & 1u, U_POLLS)) ||
+                    !mbar_wait(&full[st], (uint32_t)(k / CV_STAGES) & 1u, U_POLLS)) {
+                    fail(1);
+                    break;
                 }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int y = (tile / tiles_x) % h;
+                const uint32_t a0 = s_addr(sm + st * CV_STAGE), b0 = s_addr(sB);
+                uint32_t add = 0;
+                for (int v = 0; v < 3; v++) {
+                    if (y + (v - 1) * dil < 0 || y + (v - 1) * dil >= h) continue;
+#pragma unroll
+                    for (int u = 0; u < 3; u++) {
+#pragma unroll
+                        for (int kh = 0; kh < 2; kh++) {  // K = 16 channels (32 bytes) per MMA
+                            const uint64_t ad = umma_desc(a0 + v * CV_ROW + u * dil * 64 + kh * 32);
+                            const uint64_t bd = umma_desc(b0 + (v * 3 + u) * N * 64 + kh * 32);
+                            asm volatile(
+                                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                                ::"r"(tmem + 32 * acc), "l"(ad), "l"(bd), "r"(idesc), "r"(add)
+                                : "memory");
+                            add = 1;
+                        }
+                    }
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                             ::"r"(s_addr(&empty[st])) : "memory");
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                             ::"r"(s_addr(&acc_full[acc])) : "memory");
             }
+            // the MMAs issued are done before tensor memory is freed, whatever happened
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         ::"r"(s_addr(&bar_mma)) : "memory");
-        } else {
-            // the copies did not land in time: give them one more bounded wait (they
-            // write this CTA's shared memory) and release the others without an MMA
-            atomicExch(err, 1);
-            s_ok = 0;
-            mbar_wait(&bar_load, 0, U_POLLS);
-            mbar_arrive(&bar_mma);
+                         ::"r"(s_addr(&done)) : "memory");
+            if (!mbar_wait(&done, 0, U_POLLS)) fail(2);
         }
-    }
-    // tcgen05.ld is warp-collective: the block agrees on one outcome of the wait
-    const bool mine = mbar_wait(&bar_mma, 0, U_POLLS);
-    const bool done = __syncthreads_and(mine ? 1 : 0) != 0;
-    if (!done && threadIdx.x == 0) atomicExch(err, 2);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (done && s_ok) {
-        uint32_t r[N];
-        umma_load<N>(r, tmem + ((uint32_t)(warp * 32) << 16));
-        const int x = x0 + warp * 32 + lane;
-        if (x < w) {
+    } else {   // epilogue
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        int k = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, k++) {
+            const int acc = k & 1;
+            // tcgen05.ld is warp-collective: the warp agrees on one outcome of the wait
+            const bool got = mbar_wait(&acc_full[acc], (uint32_t)(k >> 1) & 1u, U_POLLS);
+            if (!__all_sync(0xffffffffu, got)) {
+                if (lane == 0) fail(2);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint32_t r[N];
+            umma_load<N>(r, tmem + ((uint32_t)(warp * 32) << 16) + 32 * acc);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[acc]);
+            const int row = tile / tiles_x, x = (tile - row * tiles_x) * UM + warp * 32 + lane;
+            if (x >= w) continue;
             const size_t pix = (size_t)row * w + x;
             if constexpr (EPI == EPI_LINEAR_F32) {
                 float* o = reinterpret_cast<float*>(out) + pix * out_stride;
@@ -691,9 +756,9 @@ __global__ void __launch_bounds__(128) k_conv_umma(const __grid_constant__ CUten
                         const uint4 mv = m4[q];
                         const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
 #pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            const int co = q * 8 + 2 * k;
-                            const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(&mw[k]);
+                        for (int j = 0; j < 4; j++) {
+                            const int co = q * 8 + 2 * j;
+                            const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(&mw[j]);
                             const float v0 = __bfloat162float(m.x) > 0.0f ? __uint_as_float(r[co]) : 0.0f;
                             const float v1 = __bfloat162float(m.y) > 0.0f ? __uint_as_float(r[co + 1]) : 0.0f;
                             packed[co / 2] = pack_bf16(v0, v1);
@@ -714,7 +779,7 @@ __global__ void __launch_bounds__(128) k_conv_umma(const __grid_constant__ CUten
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem) : "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;" ::"r"(tmem) : "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -942,15 +1007,31 @@ bool wgrad_map(CUtensorMap* map, const void* base, int nch, uint64_t w, uint64_t
 // Weights [9][n][32] as the B operand (all nine taps in one copy).
 bool weight_map(CUtensorMap* map, const __nv_bfloat16* W, int n) { return encode_map(map, W, (uint64_t)n, 9, n, 9); }
 
+// Activations [B*h][w][32] as a conv layer's source rows: UM cells and a dilation's more
+// on either side.
+bool row_map(CUtensorMap* map, const __nv_bfloat16* X, int B, int h, int w, int dil)
+{
+    return encode_map(map, X, (uint64_t)w, (uint64_t)B * h, (uint32_t)(UM + 2 * dil), 1);
+}
+
 template <int EPI, int N>
 cudaError_t launch_conv_umma(const CUtensorMap& mx, const CUtensorMap& mw, const float* bias, const __nv_bfloat16* act,
-                             void* out, int B, int h, int w, int dil, int cout_real, int out_stride, int* err,
-                             cudaStream_t st)
+                             void* out, int B, int h, int w, int dil, int cout_real, int out_stride, int sms,
+                             bool chained, int* err, cudaStream_t st)
 {
-    const unsigned tiles = (unsigned)(((w + UM - 1) / UM) * (size_t)B * h);
-    k_conv_umma<EPI, N><<<tiles, 128, umma_smem(N), st>>>(mx, mw, bias, act, out, h, w, dil, cout_real, out_stride,
-                                                           err);
-    return cudaGetLastError();
+    const size_t tiles = ((w + UM - 1) / UM) * (size_t)B * h;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min<size_t>(tiles, 2 * (size_t)sms));
+    cfg.blockDim = dim3(CV_THREADS);
+    cfg.dynamicSmemBytes = conv_umma_smem(N);
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_conv_umma<EPI, N>, mx, mw, bias, act, out, h, w, B * h, dil, cout_real, out_stride,
+                              chained ? 1 : 0, err);
 }
 
 // ---------------------------------------------------------------------------
@@ -1186,16 +1267,16 @@ cudaError_t conv_smem_optin()
         set((const void*)k_conv<32, 32, EPI_MASK_BF16, 8>, conv_smem(32, 32, 8)),
         set((const void*)k_conv_wgrad<32, 32, 4>, wgrad_smem(32, 32, 4)),
         set((const void*)k_conv_wgrad<32, 32, 8>, wgrad_smem(32, 32, 8)),
-        set((const void*)k_conv_umma<EPI_RELU_BF16, 32>, umma_smem(32)),
-        set((const void*)k_conv_umma<EPI_MASK_BF16, 32>, umma_smem(32)),
-        set((const void*)k_conv_umma<EPI_LINEAR_F32, 16>, umma_smem(16)),
+        set((const void*)k_conv_umma<EPI_RELU_BF16, 32>, conv_umma_smem(32)),
+        set((const void*)k_conv_umma<EPI_MASK_BF16, 32>, conv_umma_smem(32)),
+        set((const void*)k_conv_umma<EPI_LINEAR_F32, 16>, conv_umma_smem(16)),
         set((const void*)k_net_fused, umma_smem(32)),
         set((const void*)k_wgrad_umma<32>, wgrad_umma_smem(32)),
         set((const void*)k_wgrad_umma<16>, wgrad_umma_smem(16)),
     };
     for (cudaError_t x : es)
         if (x != cudaSuccess) return x;
-    // the tcgen05 kernels take 93 KB each: ask for the largest shared-memory carve-out
+    // the tcgen05 convolutions take 93-102 KB each: ask for the largest shared-memory carve-out
     // so that two CTAs share an SM (the fused launch then holds a 1024x436 frame's 218
     // tiles in one wave)
     const void* big[] = {(const void*)k_conv_umma<EPI_RELU_BF16, 32>, (const void*)k_conv_umma<EPI_MASK_BF16, 32>,
@@ -1250,6 +1331,7 @@ struct bm_net {
     CUtensorMap map_in;
     CUtensorMap map_act[NL - 1];
     CUtensorMap map_dy[2];
+    CUtensorMap map_fwd[NL], map_bwd[NL];    // source rows of each layer's forward and backward-data pass
     CUtensorMap map_in4, map_act4[NL - 1];   // the layers' inputs, images apart (weight gradient)
     CUtensorMap map_dy16;                    // the head's gradient, 16 channels
     int num_sms = 1;
@@ -1293,6 +1375,10 @@ bm_status check_dims(bm_net* n, uint32_t B, uint32_t h, uint32_t w)
     return BM_OK;
 }
 
+// The gradient buffer that holds layer l's output gradient: the head's is in 0, and the
+// backward pass alternates.
+constexpr int dy_slot(int l) { return (NL - 1 - l) & 1; }
+
 // Tensor maps of the activation buffers for a (B, h, w) call (host-side encoding only).
 bool ensure_act_maps(bm_net* n, uint32_t B, uint32_t h, uint32_t w)
 {
@@ -1301,6 +1387,8 @@ bool ensure_act_maps(bm_net* n, uint32_t B, uint32_t h, uint32_t w)
     bool ok = act_map(&n->map_in, n->d_in, Bi, hi, wi);
     for (int l = 0; ok && l < NL - 1; l++) ok = act_map(&n->map_act[l], n->d_act[l], Bi, hi, wi);
     for (int k = 0; ok && k < 2; k++) ok = act_map(&n->map_dy[k], n->d_dy[k], Bi, hi, wi);
+    for (int l = 0; ok && l < NL; l++) ok = row_map(&n->map_fwd[l], l ? n->d_act[l - 1] : n->d_in, Bi, hi, wi, DIL[l]);
+    for (int l = 1; ok && l < NL - 1; l++) ok = row_map(&n->map_bwd[l], n->d_dy[dy_slot(l)], Bi, hi, wi, DIL[l]);
     ok = ok && wgrad_map(&n->map_in4, n->d_in, 32, w, h, B) && wgrad_map(&n->map_dy16, n->d_dy[0], 16, w, (uint64_t)B * h, 0);
     for (int l = 0; ok && l < NL - 1; l++) ok = wgrad_map(&n->map_act4[l], n->d_act[l], 32, w, h, B);
     if (!ok) return false;
@@ -1352,12 +1440,13 @@ bm_status forward(bm_net* n, uint32_t B, uint32_t h, uint32_t w, cudaStream_t st
             return BM_OK;
         }
         for (int l = 0; l <= 4; l++)
-            BN_CUDA((launch_conv_umma<EPI_RELU_BF16, 32>(l == 0 ? n->map_in : n->map_act[l - 1], n->map_wf[l],
+            BN_CUDA((launch_conv_umma<EPI_RELU_BF16, 32>(n->map_fwd[l], n->map_wf[l],
                                                           n->d_master + n->poff[l] + layer_w_count(l), nullptr,
-                                                          n->d_act[l], Bi, hi, wi, DIL[l], 32, 32, n->d_err, st)));
-        BN_CUDA((launch_conv_umma<EPI_LINEAR_F32, 16>(n->map_act[4], n->map_wf[5],
+                                                          n->d_act[l], Bi, hi, wi, DIL[l], 32, 32, n->num_sms, l > 0,
+                                                          n->d_err, st)));
+        BN_CUDA((launch_conv_umma<EPI_LINEAR_F32, 16>(n->map_fwd[5], n->map_wf[5],
                                                        n->d_master + n->poff[5] + layer_w_count(5), nullptr, n->d_out,
-                                                       Bi, hi, wi, DIL[5], 3, 3, n->d_err, st)));
+                                                       Bi, hi, wi, DIL[5], 3, 3, n->num_sms, true, n->d_err, st)));
         return BM_OK;
     }
     for (int l = 0; l <= 4; l++)
@@ -1674,8 +1763,9 @@ bm_status bm_net_train_step(bm_net* n, uint32_t B, uint32_t h, uint32_t w, const
         s = weight_grad(n, l, cur, Bi, hi, wi, st);
         if (s != BM_OK) return s;
         if (n->umma)
-            BN_CUDA((launch_conv_umma<EPI_MASK_BF16, 32>(n->map_dy[cur], n->map_wb[l], nullptr, n->d_act[l - 1],
-                                                          n->d_dy[cur ^ 1], Bi, hi, wi, DIL[l], 32, 32, n->d_err, st)));
+            BN_CUDA((launch_conv_umma<EPI_MASK_BF16, 32>(n->map_bwd[l], n->map_wb[l], nullptr, n->d_act[l - 1],
+                                                          n->d_dy[cur ^ 1], Bi, hi, wi, DIL[l], 32, 32, n->num_sms,
+                                                          false, n->d_err, st)));
         else
             BN_CUDA(conv_bwd_data(l, n->d_dy[cur], n->d_wb[l], n->d_act[l - 1], n->d_dy[cur ^ 1], Bi, hi, wi, st));
         cur ^= 1;
