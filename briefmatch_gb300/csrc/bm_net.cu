@@ -786,34 +786,32 @@ __global__ void __launch_bounds__(CV_THREADS) k_conv_umma(const __grid_constant_
 // tcgen05 weight gradient of a 3x3 layer:
 //   dW[co][tap][ci] += sum over cells p of dY[p][co] * X[p + shift(tap)][ci],
 //   db[co] += sum over p of dY[p][co].
-// The cells are the reduction: both operands are MN-major (channels contiguous), as TMA
-// lands them -- per 128 cells of an image row nine shifted X tiles of 128 x 32 channels
-// (zero outside the image: the map is 4-D, so a tap's row cannot run into the next
-// image) and one dY tile of 128 x NCH.  Four X tiles 8 KB apart make the M = 128 rows
-// (tap, ci) of one MMA, so three accumulators (taps 0-3, 4-7 and 8) of NCH columns each
-// stay in tensor memory over all of a CTA's tiles, 24 MMAs of K = 16 cells per tile.  A
-// tile of ones behind tap 8 gives the bias gradient as one more row; rows past it are
-// not read out.  Two stages: the copies of the next tile run under the MMAs of this one.
-// At the end each warp adds its accumulator lanes (one tap, 32 input channels) to the
-// FP32 gradient, 128 contiguous bytes per output channel.
+// The cells q = p + shift are the reduction: both operands are MN-major (channels
+// contiguous), as TMA lands them -- per 128 cells of an image row the three source rows
+// of X and one row of dY, 128 + 2 dil cells.  One MMA takes all nine taps of 16 cells:
+// its M = 128 rows are dY shifted by 0, dil and 2 dil cells (32-channel groups dil * 64
+// bytes apart that overlap; the groups past the third read on and are not read out), its
+// N = 96 columns the three rows of X.  A source row outside the image is neither loaded
+// nor multiplied: the columns then are the range of rows inside.  The accumulator stays
+// in tensor memory over all of a CTA's tiles, 8 MMAs per tile; the two warps without MMAs
+// or copies sum dY for the bias gradient.  Four stages: the next tiles' copies run under
+// the MMAs of this one.  At the end the accumulator is turned through shared memory, so
+// that a warp adds 32 input channels, 128 contiguous bytes, to the FP32 gradient at once.
 //
-// It replaces mma.sync tiles with transposed shared-memory staging and an atomic flush
-// per 128 cells, which kept the L1 60-80 % busy: per layer of 32 images of 128 x 96 cells
-// 133 us (dilation 1) to 233 us (dilation 8), now 35 us, 245 MB of copies from L2.
+// What bounds an MMA here is reading its M x 16 operand (about 90 cycles, whatever N is):
+// dY is that operand, and the taps go into N.  Per layer of 32 images of 128 x 96 cells:
+// mma.sync tiles with transposed shared-memory staging 133 us (dilation 1) to 233 us
+// (dilation 8); X as the M operand, three MMAs per 16 cells, 31 us; now 22 us (24 us with scalar adds at the end).
 // ---------------------------------------------------------------------------
-constexpr uint32_t WG_ONES = 9, WG_TILES = 10;   // tile 9 holds ones
-__host__ __device__ constexpr uint32_t wg_stage(int nch) { return WG_TILES * U_TAP_A + (uint32_t)(UM * nch * 2); }
-// two stages, and room for the last MMA's unused rows past them
-constexpr size_t wgrad_umma_smem(int nch) { return 1024 + 2 * (size_t)wg_stage(nch) + 2 * U_TAP_A; }
+constexpr int WG_STAGES = 4;
+constexpr uint32_t WG_DY = 10240, WG_STAGE = WG_DY + 3 * U_TAP_A;   // dY, then three rows of X
+constexpr int WG_PITCH = 97;                                        // floats of a turned row
+constexpr size_t WG_SMEM = 1024 + WG_STAGES * (size_t)WG_STAGE;
+// the groups past the third stay inside dY's room (32 channels: 4 groups, dilation up to
+// 8; 16 channels: 8 groups, the head's dilation is 1)
+static_assert((UM + 3 * 8) * 64 <= WG_DY && (UM + 7 * 1) * 32 <= WG_DY && DIL[NL - 1] == 1, "unused rows");
+static_assert(96 * WG_PITCH * 4 <= WG_STAGES * WG_STAGE, "the turned accumulator fits the stages");
 
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, int c3,
-                                            uint64_t* bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-        ::"r"(s_addr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(s_addr(bar))
-        : "memory");
-}
 // Shared-memory matrix descriptor, MN-major: rows (K) of `width` channels contiguous and
 // swizzled by their width, 8-row groups 8 rows apart, the next `width` of MN `lead` bytes on.
 template <int WIDTH>
@@ -837,27 +835,27 @@ __global__ void __launch_bounds__(128) k_wgrad_umma(const __grid_constant__ CUte
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t full[2], empty[2], done;
+    __shared__ __align__(8) uint64_t full[WG_STAGES], empty[WG_STAGES], done;
     __shared__ uint32_t s_tmem;
-    __shared__ volatile int s_fail;
+    __shared__ volatile int s_fail, s_used;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_x = (w + UM - 1) / UM;
     const int tiles = tiles_x * rows;
+    auto fail = [&](int code) {
+        atomicExch(err, code);
+        s_fail = 1;
+    };
 
     if (threadIdx.x == 0) {
-        for (int k = 0; k < 2; k++) {
+        for (int k = 0; k < WG_STAGES; k++) {
             mbar_init(&full[k], 1);
-            mbar_init(&empty[k], 1);
+            mbar_init(&empty[k], 3);   // the MMAs and two summing warps
         }
         mbar_init(&done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_fail = 0;
+        s_used = 0;
     }
-    for (int k = 0; k < 2; k++) {   // the tiles of ones (the same under any swizzle)
-        uint32_t* ones = reinterpret_cast<uint32_t*>(sm + k * wg_stage(NCH) + WG_ONES * U_TAP_A);
-        for (uint32_t i = threadIdx.x; i < U_TAP_A / 4; i += 128) ones[i] = 0x3F803F80u;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(s_addr(&s_tmem))
                      : "memory");
@@ -872,53 +870,100 @@ __global__ void __launch_bounds__(128) k_wgrad_umma(const __grid_constant__ CUte
         // producer
         int k = 0;
         for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, k++) {
-            const int st = k & 1;
-            if (k >= 2 && !mbar_wait(&empty[st], (uint32_t)((k >> 1) - 1) & 1u, U_POLLS)) {
-                atomicExch(err, 2);
-                s_fail = 1;
-            }
+            const int st = k % WG_STAGES, use = k / WG_STAGES;
+            if (use > 0 && !mbar_wait(&empty[st], (uint32_t)(use - 1) & 1u, U_POLLS)) fail(2);
             if (s_fail) break;
             const int row = tile / tiles_x, x0 = (tile - row * tiles_x) * UM;
-            const int b = row / h, y = row - b * h;
-            unsigned char* base = sm + st * wg_stage(NCH);
-            mbar_expect_tx(&full[st], 9 * U_TAP_A + UM * NCH * 2);
-            for (int t = 0; t < 9; t++)
-                tma_load_4d(base + t * U_TAP_A, &tmX, 0, x0 + (t % 3 - 1) * dil, y + (t / 3 - 1) * dil, b, &full[st]);
-            tma_load_3d(base + WG_TILES * U_TAP_A, &tmD, 0, x0, row, &full[st]);
+            const int y = row % h;
+            unsigned char* base = sm + st * WG_STAGE;
+            uint32_t bytes = (uint32_t)(UM + 2 * dil) * NCH * 2;
+            for (int v = -1; v <= 1; v++)
+                if (y + v * dil >= 0 && y + v * dil < h) bytes += U_TAP_A;
+            mbar_expect_tx(&full[st], bytes);
+            tma_load_3d(base, &tmD, 0, x0 - dil, row, &full[st]);
+            for (int v = -1; v <= 1; v++)
+                if (y + v * dil >= 0 && y + v * dil < h)
+                    tma_load_3d(base + WG_DY + (v + 1) * U_TAP_A, &tmX, 0, x0, row + v * dil, &full[st]);
         }
+        // this CTA's copies land before it leaves, whatever happened
+        for (int j = k > WG_STAGES ? k - WG_STAGES : 0; j < k; j++)
+            mbar_wait(&full[j % WG_STAGES], (uint32_t)(j / WG_STAGES) & 1u, U_POLLS);
     } else if (threadIdx.x == 32) {
         // MMA issuer
-        constexpr uint32_t idesc = umma_idesc(UM, NCH) | (1u << 15) | (1u << 16);   // both operands MN-major
+        constexpr uint32_t mn = (1u << 15) | (1u << 16);   // both operands MN-major
+        uint32_t used = 0;   // source rows whose columns hold a sum
         int k = 0;
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, k++) {
-            const int st = k & 1;
-            if (!mbar_wait(&full[st], (uint32_t)(k >> 1) & 1u, U_POLLS)) {
-                // give this CTA's copies one more bounded wait, then let everybody go
-                atomicExch(err, 1);
-                s_fail = 1;
-                mbar_wait(&full[st], (uint32_t)(k >> 1) & 1u, U_POLLS);
+        for (int tile = blockIdx.x; tile < tiles && !s_fail; tile += gridDim.x, k++) {
+            const int st = k % WG_STAGES;
+            if (!mbar_wait(&full[st], (uint32_t)(k / WG_STAGES) & 1u, U_POLLS)) {
+                fail(1);
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t base = s_addr(sm + st * wg_stage(NCH)), dbase = base + WG_TILES * U_TAP_A;
-            for (int kk = 0; kk < UM / 16; kk++) {   // 16 cells per MMA
-                const uint64_t bd = umma_desc_mn<NCH>(dbase + kk * 16 * NCH * 2, UM * NCH * 2);
-#pragma unroll
-                for (int g = 0; g < 3; g++) {
-                    const uint64_t ad = umma_desc_mn<32>(base + g * 4 * U_TAP_A + kk * 16 * 64, U_TAP_A);
-                    asm volatile(
-                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                        ::"r"(tmem + 32 * g), "l"(ad), "l"(bd), "r"(idesc), "r"((k | kk) ? 1u : 0u)
-                        : "memory");
-                }
+            const int y = (tile / tiles_x) % h;
+            const int v0 = y - dil < 0 ? 1 : 0, v1 = y + dil >= h ? 1 : 2;
+            const uint32_t base = s_addr(sm + st * WG_STAGE);
+            auto mma = [&](int kk, int va, int vb, uint32_t add) {   // 16 cells, source rows va..vb
+                const uint64_t ad = umma_desc_mn<NCH>(base + kk * 16 * NCH * 2, dil * NCH * 2);
+                const uint64_t bd = umma_desc_mn<32>(base + WG_DY + va * U_TAP_A + kk * 16 * 64, U_TAP_A);
+                const uint32_t idesc = umma_idesc(UM, 32 * (vb - va + 1)) | mn;
+                asm volatile(
+                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                    ::"r"(tmem + 32 * va), "l"(ad), "l"(bd), "r"(idesc), "r"(add)
+                    : "memory");
+            };
+            const uint32_t rng = (2u << v1) - (1u << v0);
+            if ((used & rng) == rng) {
+                mma(0, v0, v1, 1u);
+            } else {   // a row's first sum overwrites its columns
+                for (int v = v0; v <= v1; v++) mma(0, v, v, (used >> v) & 1u);
+                used |= rng;
             }
+#pragma unroll
+            for (int kk = 1; kk < UM / 16; kk++) mma(kk, v0, v1, 1u);
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                          ::"r"(s_addr(&empty[st])) : "memory");
         }
+        s_used = (int)used;
         // arrives once the MMAs issued so far are done, also after a wait that gave up
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                      ::"r"(s_addr(&done)) : "memory");
+    } else if (warp >= 2) {
+        // db: a lane owns 2 channels; a warp reads 64 of the tile's cells, 64 / NCH at a time
+        // (a cell's 16-byte chunks lie permuted by the swizzle)
+        constexpr int LPR = NCH / 2, RPW = 32 / LPR;
+        const int c = (lane % LPR) >> 2, cin = lane & 3;
+        float s0 = 0.0f, s1 = 0.0f;
+        int k = 0;
+        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, k++) {
+            const int st = k % WG_STAGES;
+            const bool got = mbar_wait(&full[st], (uint32_t)(k / WG_STAGES) & 1u, U_POLLS);
+            if (!__all_sync(0xffffffffu, got)) {
+                if (lane == 0) fail(1);
+                break;
+            }
+            const unsigned char* dt = sm + st * WG_STAGE;
+#pragma unroll 8
+            for (int i = 0; i < UM / 2; i += RPW) {
+                const int p = dil + (warp - 2) * (UM / 2) + i + lane / LPR;
+                const int chunk = NCH == 32 ? c ^ ((p >> 1) & 3) : c ^ ((p >> 2) & 1);
+                const uint32_t q = *reinterpret_cast<const uint32_t*>(dt + p * NCH * 2 + chunk * 16 + cin * 4);
+                s0 += __uint_as_float(q << 16);
+                s1 += __uint_as_float(q & 0xffff0000u);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[st]);
+        }
+#pragma unroll
+        for (int o = LPR; o < 32; o *= 2) {
+            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        }
+        if (!s_fail && lane < LPR) {
+            if (2 * lane < cout_real) atomicAdd(db + 2 * lane, s0);
+            if (2 * lane + 1 < cout_real) atomicAdd(db + 2 * lane + 1, s1);
+        }
     }
     __syncwarp();
     // tcgen05.ld is warp-collective: the block agrees on one outcome of the wait.  The
@@ -928,20 +973,30 @@ __global__ void __launch_bounds__(128) k_wgrad_umma(const __grid_constant__ CUte
     if (!ok && threadIdx.x == 0) atomicExch(err, 2);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok) {
+        // lane NCH g + co holds tap column u = 2 - g (dY moves against X), column 32 v + ci
+        float* turned = reinterpret_cast<float*>(sm);
+        if (warp * 32 < 3 * NCH) {
 #pragma unroll 1
-        for (int g = 0; g < 3; g++) {
-            const int tap = 4 * g + warp;   // tap 9: the row of ones
-            if (tap > 9) continue;
-            uint32_t r[NCH];
-            umma_load<NCH>(r, tmem + ((uint32_t)(warp * 32) << 16) + 32 * g);
+            for (int v = 0; v < 3; v++) {
+                uint32_t r[32];
+                umma_load<32>(r, tmem + ((uint32_t)(warp * 32) << 16) + 32 * v);
+                if (warp * 32 + lane < 3 * NCH)
 #pragma unroll
-            for (int co = 0; co < NCH; co++) {
-                if (co >= cout_real) continue;
-                if (tap < 9)
-                    atomicAdd(dW + ((size_t)co * 9 + tap) * 32 + lane, __uint_as_float(r[co]));
-                else if (lane == 0)
-                    atomicAdd(db + co, __uint_as_float(r[co]));
+                    for (int ci = 0; ci < 32; ci++)
+                        turned[(warp * 32 + lane) * WG_PITCH + 32 * v + ci] = __uint_as_float(r[ci]);
             }
+        }
+        __syncthreads();
+        // 4 rows of dW, 8 lanes each, per pass; dW is 16-byte aligned (a layer's parameters
+        // are a multiple of 4)
+        const int n = 9 * cout_real, c4 = (lane & 7) * 4;
+#pragma unroll 2
+        for (int i = warp * 4 + (lane >> 3); i < n; i += 16) {
+            const int co = i / 9, tap = i - co * 9, v = tap / 3, u = tap - v * 3;
+            const float* t = turned + ((2 - u) * NCH + co) * WG_PITCH + 32 * v + c4;
+            if ((s_used >> v) & 1)
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dW + i * 32 + c4), "f"(t[0]),
+                             "f"(t[1]), "f"(t[2]), "f"(t[3]) : "memory");
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -970,18 +1025,18 @@ EncodeTiled encoder()
 }
 
 // A 3-D BF16 tensor map with 64-byte rows: dims {32 channels, d1, d2}, box {32, b1, b2},
-// 64-byte swizzle, zero fill out of bounds.
-bool encode_map(CUtensorMap* map, const void* base, uint64_t d1, uint64_t d2, uint32_t b1, uint32_t b2)
+// 64-byte swizzle, zero fill out of bounds (nch = 16: 32-byte rows and swizzle).
+bool encode_map(CUtensorMap* map, const void* base, uint64_t d1, uint64_t d2, uint32_t b1, uint32_t b2, uint32_t nch = 32)
 {
     EncodeTiled enc = encoder();
     if (!enc) return false;
-    const cuuint64_t dims[3] = {32, d1, d2};
-    const cuuint64_t strides[2] = {64, 64 * d1};
-    const cuuint32_t box[3] = {32, b1, b2};
+    const cuuint64_t dims[3] = {nch, d1, d2};
+    const cuuint64_t strides[2] = {2 * nch, 2 * nch * d1};
+    const cuuint32_t box[3] = {nch, b1, b2};
     const cuuint32_t estr[3] = {1, 1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+               CU_TENSOR_MAP_INTERLEAVE_NONE, nch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Activations [B*h][w][32] as the A operand of a conv layer.
@@ -989,29 +1044,14 @@ bool act_map(CUtensorMap* map, const __nv_bfloat16* X, int B, int h, int w)
 {
     return encode_map(map, X, (uint64_t)w, (uint64_t)B * h, UM, 1);
 }
-// A BF16 tensor map for the weight gradient: dims {nch, w, h, b} (b omitted when 0), box
-// {nch, UM, 1, 1}, rows swizzled by their width (64 or 32 bytes), zero fill.
-bool wgrad_map(CUtensorMap* map, const void* base, int nch, uint64_t w, uint64_t h, uint64_t b)
-{
-    EncodeTiled enc = encoder();
-    if (!enc) return false;
-    const uint64_t px = (uint64_t)nch * 2;
-    const cuuint64_t dims[4] = {(cuuint64_t)nch, w, h, b};
-    const cuuint64_t strides[3] = {px, px * w, px * w * h};
-    const cuuint32_t box[4] = {(cuuint32_t)nch, UM, 1, 1};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, b ? 4 : 3, const_cast<void*>(base), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, nch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 // Weights [9][n][32] as the B operand (all nine taps in one copy).
 bool weight_map(CUtensorMap* map, const __nv_bfloat16* W, int n) { return encode_map(map, W, (uint64_t)n, 9, n, 9); }
 
-// Activations [B*h][w][32] as a conv layer's source rows: UM cells and a dilation's more
-// on either side.
-bool row_map(CUtensorMap* map, const __nv_bfloat16* X, int B, int h, int w, int dil)
+// Activations [B*h][w][nch] as a layer's source rows: UM cells and a dilation's more on
+// either side.
+bool row_map(CUtensorMap* map, const __nv_bfloat16* X, int B, int h, int w, int dil, int nch = 32)
 {
-    return encode_map(map, X, (uint64_t)w, (uint64_t)B * h, (uint32_t)(UM + 2 * dil), 1);
+    return encode_map(map, X, (uint64_t)w, (uint64_t)B * h, (uint32_t)(UM + 2 * dil), 1, nch);
 }
 
 template <int EPI, int N>
@@ -1271,8 +1311,8 @@ cudaError_t conv_smem_optin()
         set((const void*)k_conv_umma<EPI_MASK_BF16, 32>, conv_umma_smem(32)),
         set((const void*)k_conv_umma<EPI_LINEAR_F32, 16>, conv_umma_smem(16)),
         set((const void*)k_net_fused, umma_smem(32)),
-        set((const void*)k_wgrad_umma<32>, wgrad_umma_smem(32)),
-        set((const void*)k_wgrad_umma<16>, wgrad_umma_smem(16)),
+        set((const void*)k_wgrad_umma<32>, WG_SMEM),
+        set((const void*)k_wgrad_umma<16>, WG_SMEM),
     };
     for (cudaError_t x : es)
         if (x != cudaSuccess) return x;
@@ -1330,10 +1370,7 @@ struct bm_net {
     uint32_t map_B = 0, map_h = 0, map_w = 0;
     CUtensorMap map_in;
     CUtensorMap map_act[NL - 1];
-    CUtensorMap map_dy[2];
-    CUtensorMap map_fwd[NL], map_bwd[NL];    // source rows of each layer's forward and backward-data pass
-    CUtensorMap map_in4, map_act4[NL - 1];   // the layers' inputs, images apart (weight gradient)
-    CUtensorMap map_dy16;                    // the head's gradient, 16 channels
+    CUtensorMap map_fwd[NL], map_dy[NL];   // source rows of each layer's input and of its output gradient
     int num_sms = 1;
 };
 
@@ -1386,11 +1423,9 @@ bool ensure_act_maps(bm_net* n, uint32_t B, uint32_t h, uint32_t w)
     const int Bi = (int)B, hi = (int)h, wi = (int)w;
     bool ok = act_map(&n->map_in, n->d_in, Bi, hi, wi);
     for (int l = 0; ok && l < NL - 1; l++) ok = act_map(&n->map_act[l], n->d_act[l], Bi, hi, wi);
-    for (int k = 0; ok && k < 2; k++) ok = act_map(&n->map_dy[k], n->d_dy[k], Bi, hi, wi);
     for (int l = 0; ok && l < NL; l++) ok = row_map(&n->map_fwd[l], l ? n->d_act[l - 1] : n->d_in, Bi, hi, wi, DIL[l]);
-    for (int l = 1; ok && l < NL - 1; l++) ok = row_map(&n->map_bwd[l], n->d_dy[dy_slot(l)], Bi, hi, wi, DIL[l]);
-    ok = ok && wgrad_map(&n->map_in4, n->d_in, 32, w, h, B) && wgrad_map(&n->map_dy16, n->d_dy[0], 16, w, (uint64_t)B * h, 0);
-    for (int l = 0; ok && l < NL - 1; l++) ok = wgrad_map(&n->map_act4[l], n->d_act[l], 32, w, h, B);
+    for (int l = 0; ok && l < NL; l++)
+        ok = row_map(&n->map_dy[l], n->d_dy[dy_slot(l)], Bi, hi, wi, DIL[l], l == NL - 1 ? 16 : 32);
     if (!ok) return false;
     n->map_B = B;
     n->map_h = h;
@@ -1465,13 +1500,13 @@ bm_status weight_grad(bm_net* n, int l, int cur, int B, int h, int w, cudaStream
     float* dW = n->d_grad + n->poff[l];
     float* db = dW + layer_w_count(l);
     if (n->umma) {
-        const CUtensorMap& mx = l == 0 ? n->map_in4 : n->map_act4[l - 1];
+        const CUtensorMap& mx = l == 0 ? n->map_in : n->map_act[l - 1];
         const int rows = B * h, tiles = ((w + UM - 1) / UM) * rows, grid = std::min(tiles, n->num_sms);
         if (l == NL - 1)
-            k_wgrad_umma<16><<<grid, 128, wgrad_umma_smem(16), st>>>(mx, n->map_dy16, dW, db, h, w, rows, DIL[l], COUT_R[l],
+            k_wgrad_umma<16><<<grid, 128, WG_SMEM, st>>>(mx, n->map_dy[l], dW, db, h, w, rows, DIL[l], COUT_R[l],
                                                                      n->d_err);
         else
-            k_wgrad_umma<32><<<grid, 128, wgrad_umma_smem(32), st>>>(mx, n->map_dy[cur], dW, db, h, w, rows, DIL[l],
+            k_wgrad_umma<32><<<grid, 128, WG_SMEM, st>>>(mx, n->map_dy[l], dW, db, h, w, rows, DIL[l],
                                                                      COUT_R[l], n->d_err);
         BN_CUDA(cudaGetLastError());
     } else if (l == NL - 1) {
@@ -1763,7 +1798,7 @@ bm_status bm_net_train_step(bm_net* n, uint32_t B, uint32_t h, uint32_t w, const
         s = weight_grad(n, l, cur, Bi, hi, wi, st);
         if (s != BM_OK) return s;
         if (n->umma)
-            BN_CUDA((launch_conv_umma<EPI_MASK_BF16, 32>(n->map_bwd[l], n->map_wb[l], nullptr, n->d_act[l - 1],
+            BN_CUDA((launch_conv_umma<EPI_MASK_BF16, 32>(n->map_dy[l], n->map_wb[l], nullptr, n->d_act[l - 1],
                                                           n->d_dy[cur ^ 1], Bi, hi, wi, DIL[l], 32, 32, n->num_sms,
                                                           false, n->d_err, st)));
         else
