@@ -413,24 +413,31 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
     p[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
 }
 
-// FP32 master parameters of one layer -> the BF16 forward layout W[tap][COUTP][CINP]
-// and the backward-data layout Wb[tap][CINP_as_out][COUTP16_as_in] (taps flipped).
-__global__ void k_pack_layer(const float* __restrict__ master, int cin, int cout, int cinp, int coutp, int coutp16,
-                             __nv_bfloat16* __restrict__ Wf, __nv_bfloat16* __restrict__ Wb)
+// FP32 master parameters -> each layer's BF16 forward layout Wf[tap][COUTP][CINP] and,
+// from layer 1 on, its backward-data layout Wb[tap][CINP][coutp16] (taps flipped).  One
+// launch for all layers, blockIdx.y the layer: one launch a layer took 3.1 us each, mostly
+// its own start, twice six a training step.
+struct PackArgs {
+    const float* master[NL];
+    __nv_bfloat16 *Wf[NL], *Wb[NL];
+    int cin[NL], cout[NL], cinp[NL], coutp[NL], coutp16[NL];
+};
+__global__ void k_pack_weights(const __grid_constant__ PackArgs a)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int l = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int cin = a.cin[l], cout = a.cout[l], cinp = a.cinp[l], coutp = a.coutp[l], coutp16 = a.coutp16[l];
     const int nf = 9 * coutp * cinp;
     if (i < nf) {
         const int tap = i / (coutp * cinp), r = i - tap * coutp * cinp, co = r / cinp, ci = r - co * cinp;
-        const float v = (co < cout && ci < cin) ? master[((size_t)co * 9 + tap) * cin + ci] : 0.0f;
-        Wf[i] = __float2bfloat16(v);
+        const float v = (co < cout && ci < cin) ? a.master[l][((size_t)co * 9 + tap) * cin + ci] : 0.0f;
+        a.Wf[l][i] = __float2bfloat16(v);
     }
     const int nb = 9 * cinp * coutp16;
-    if (Wb && i < nb) {
+    if (a.Wb[l] && i < nb) {
         const int tap = i / (cinp * coutp16), r = i - tap * cinp * coutp16, ci = r / coutp16, co = r - ci * coutp16;
         const int ftap = 8 - tap;
-        const float v = (co < cout && ci < cin) ? master[((size_t)co * 9 + ftap) * cin + ci] : 0.0f;
-        Wb[i] = __float2bfloat16(v);
+        const float v = (co < cout && ci < cin) ? a.master[l][((size_t)co * 9 + ftap) * cin + ci] : 0.0f;
+        a.Wb[l][i] = __float2bfloat16(v);
     }
 }
 
@@ -1394,13 +1401,21 @@ bm_status nfail(bm_status st, const char* msg)
 
 bm_status pack_weights(bm_net* n, cudaStream_t st)
 {
+    PackArgs a;
+    int cnt = 0;
     for (int l = 0; l < NL; l++) {
-        const int coutp16 = COUT_P[l] < 16 ? 16 : COUT_P[l];
-        const int cnt = 9 * CIN_P[l] * coutp16 > 9 * COUT_P[l] * CIN_P[l] ? 9 * CIN_P[l] * coutp16 : 9 * COUT_P[l] * CIN_P[l];
-        k_pack_layer<<<(cnt + 255) / 256, 256, 0, st>>>(n->d_master + n->poff[l], CIN_R[l], COUT_R[l], CIN_P[l], COUT_P[l],
-                                                          coutp16, n->d_wf[l], l > 0 ? n->d_wb[l] : nullptr);
-        BN_CUDA(cudaGetLastError());
+        a.master[l] = n->d_master + n->poff[l];
+        a.Wf[l] = n->d_wf[l];
+        a.Wb[l] = l > 0 ? n->d_wb[l] : nullptr;
+        a.cin[l] = CIN_R[l];
+        a.cout[l] = COUT_R[l];
+        a.cinp[l] = CIN_P[l];
+        a.coutp[l] = COUT_P[l];
+        a.coutp16[l] = COUT_P[l] < 16 ? 16 : COUT_P[l];
+        cnt = std::max(cnt, 9 * CIN_P[l] * a.coutp16[l]);
     }
+    k_pack_weights<<<dim3((cnt + 255) / 256, NL), 256, 0, st>>>(a);
+    BN_CUDA(cudaGetLastError());
     n->packed = true;
     return BM_OK;
 }
