@@ -290,8 +290,9 @@ bm_status features_into(bm_ctx* c, const float* d_up, uint32_t* F, bool padded =
 }
 
 // One jump-flood pass; the random search of this iteration is fused into the last
-// level when fuse_rs is set (it reads only the pixel's own state).
-bm_status propagate_pass(bm_ctx* c, int pd, bool fuse_rs, uint32_t jfMax)
+// level when fuse_rs is set (it reads only the pixel's own state).  `chained`: the
+// initialisation or another pass is the launch before it.
+bm_status propagate_pass(bm_ctx* c, int pd, bool fuse_rs, uint32_t jfMax, bool chained)
 {
     const bm_params& p = c->prm;
     int levels = 0;
@@ -302,7 +303,7 @@ bm_status propagate_pass(bm_ctx* c, int pd, bool fuse_rs, uint32_t jfMax)
         bmk::RsArgs rs = rs_args(c, fuse_rs && last);
         BM_LAUNCH(c, rs.enabled ? "jump_level_rs" : "jump_level", bmk::jump_level(c->feat1_ptr(), c->feat2_ptr(), c->d_flow[c->flow_cur], c->d_flow[c->flow_cur ^ 1],
                                      c->d_cost, (int)p.sx, (int)p.sy, (int)c->nsp, step, pd, p.doubleProp ? 1 : 0, rs,
-                                     next_order(c), c->stream));
+                                     next_order(c), chained || lvl > 0, c->stream));
         c->flow_cur ^= 1;
     }
     if (fuse_rs) {
@@ -325,7 +326,7 @@ bm_status local_steps_impl(bm_ctx* c)
     for (uint32_t k = 0; k < c->local_steps; k++) {
         BM_LAUNCH(c, "local_step", bmk::local_step(c->feat1_ptr(), c->feat2_ptr(), c->d_flow[c->flow_cur],
                                                    c->d_flow[c->flow_cur ^ 1], c->d_cost, (int)p.sx, (int)p.sy,
-                                                   (int)c->nsp, r, next_order(c), c->stream));
+                                                   (int)c->nsp, r, next_order(c), true, c->stream));
         c->flow_cur ^= 1;
         r = r > 1 ? r / 2 : 1;
     }
@@ -366,7 +367,7 @@ bm_status match_impl(bm_ctx* c, const float* d_im2, bool seeded, bool padded = f
     }
     int pd = -1;
     for (uint32_t it = 0; it < iterations; it++) {
-        st = propagate_pass(c, pd, true, jfMax);
+        st = propagate_pass(c, pd, true, jfMax, true);
         if (st != BM_OK) return st;
         pd = -pd;
     }
@@ -767,7 +768,7 @@ bm_status bm_initialize(bm_ctx* c, int first)
 bm_status bm_propagate(bm_ctx* c, int pd)
 {
     if (check_ctx(c)) return BM_ERR_INVALID;
-    return propagate_pass(c, pd, false, c->prm.jfMax);
+    return propagate_pass(c, pd, false, c->prm.jfMax, false);
 }
 
 bm_status bm_random_search(bm_ctx* c)
@@ -965,7 +966,7 @@ bm_status bm_local_step(bm_ctx* c, uint32_t radius)
     const bm_params& p = c->prm;
     BM_LAUNCH(c, "local_step", bmk::local_step(c->feat1_ptr(), c->feat2_ptr(), c->d_flow[c->flow_cur],
                                                c->d_flow[c->flow_cur ^ 1], c->d_cost, (int)p.sx, (int)p.sy, (int)c->nsp,
-                                               (int)radius, next_order(c), c->stream));
+                                               (int)radius, next_order(c), false, c->stream));
     c->flow_cur ^= 1;
     return BM_OK;
 }

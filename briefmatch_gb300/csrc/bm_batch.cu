@@ -459,7 +459,7 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
         cur ^= 1;
         int r = (int)b->local_radius;
         for (uint32_t k = 0; k < b->local_steps; k++) {
-            BB_CUDA(local_step(d.F[0], d.F[1], d.flow[cur], d.flow[cur ^ 1], d.cost, d.sx, d.sy, (int)b->nsp, r, rev, st));
+            BB_CUDA(local_step(d.F[0], d.F[1], d.flow[cur], d.flow[cur ^ 1], d.cost, d.sx, d.sy, (int)b->nsp, r, rev, false, st));
             rev ^= s.snake ? 1 : 0;
             cur ^= 1;
             r = r > 1 ? r / 2 : 1;
@@ -483,7 +483,7 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
             rs.call = it;
             rs.dist = d.dist;
             BB_CUDA(jump_level(d.F[0], d.F[1], d.flow[cur], d.flow[cur ^ 1], d.cost, d.sx, d.sy, (int)b->nsp, q, pd,
-                               b->doubleProp, rs, rev, st));
+                               b->doubleProp, rs, rev, false, st));
             rev ^= s.snake ? 1 : 0;
             cur ^= 1;
         }

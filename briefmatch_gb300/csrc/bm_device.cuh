@@ -303,6 +303,16 @@ __device__ __forceinline__ bool tile_interior(int bx, int by, int sx, int sy, in
     return (bx - rmax >= 0) && (bx + TX - 1 + rmax < sx) && (by - rmax >= 0) && (by + TY - 1 + rmax < sy);
 }
 
+// Chained launches (programmatic dependent launch): a kernel may start while the one
+// before it runs its last blocks, and waits here for that one to be complete.  The
+// trigger for the next kernel comes after the wait, so everything older than a kernel's
+// immediate predecessor is complete when it starts; only what that predecessor wrote
+// (or read) has to be touched after the wait, and never by the read-only path.  A pair's
+// levels are 17 or more launches in a row, 2.5 us apart on small frames: chained, a pair of
+// 96x64 frames took 166 us (207), 320x240 263 (299), 1024x436 u2.9 1209 (1254).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // PatchMatch (briefmatch_cuda.cu:126-246).
 // ---------------------------------------------------------------------------
@@ -387,9 +397,10 @@ __device__ __forceinline__ void seed_px(const uint32_t* __restrict__ F1, const u
 // With RS the iteration's random-search candidate (:237-243) is evaluated last; it
 // reads only this pixel's own state, so fusing it into the last level gives the
 // reference's result.
-// INLAUNCH: the field and cost were written by an earlier phase of the same launch
-// (the persistent batched kernel); they are then read through L2 (ld.global.cg),
-// never through the non-coherent read-only path.
+// INLAUNCH: the field and cost were written after this kernel started -- by an earlier
+// phase of the same launch (the persistent batched kernel), or by the level before it
+// (chained launches); they are then read through L2 (ld.global.cg), never through the
+// non-coherent read-only path.
 template <bool INLAUNCH>
 __device__ __forceinline__ uint32_t field_load(const uint32_t* p)
 {
@@ -660,12 +671,12 @@ __device__ __forceinline__ void jump_level_px(const uint32_t* __restrict__ F1, c
 // best so far.  Reads flow_in (a snapshot) and writes flow_out, like a jump level.
 template <int NSP>
 __device__ __forceinline__ void local_px(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
-                                         const uint32_t* __restrict__ flow_in, uint32_t* __restrict__ flow_out,
-                                         uint16_t* __restrict__ cost, int sx, int sy, int r, int x, int y)
+                                         const uint32_t* flow_in, uint32_t* flow_out,
+                                         uint16_t* cost, int sx, int sy, int r, int x, int y)
 {
     const long pix = x + (long)y * sx;
-    const uint32_t own = __ldg(flow_in + pix);
-    const int h0 = (int)cost[pix];
+    const uint32_t own = __ldcg(flow_in + pix);
+    const int h0 = (int)__ldcg(cost + pix);
     const int ox = lo16(own), oy = hi16(own);
     uint32_t cand[4];
     bool live[4];

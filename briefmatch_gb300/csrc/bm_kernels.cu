@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(256) k_initialize(const uint32_t* __restrict__
 {
     const int2 t0 = block_tile(rev);
     const int x = t0.x + threadIdx.x, y = t0.y + threadIdx.y;
+    chain_trigger();   // launched unchained: what is older is complete
     if (x >= sx || y >= sy) return;
     init_px<NSP>(F1, F2, flow_prev, flow_out, cost, sx, sy, first, x, y);
 }
@@ -314,6 +315,7 @@ __global__ void __launch_bounds__(256) k_seed(const uint32_t* __restrict__ F1, c
                                               float scale_y, float inv_x, float inv_y, float logit_min)
 {
     const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
+    chain_trigger();   // launched unchained: what is older is complete
     if (x >= sx || y >= sy) return;
     seed_px<NSP>(F1, F2, flow_prev, flow_out, cost, sx, sy, first, x, y, pred, w4, h4, scale_x, scale_y, inv_x, inv_y,
                  logit_min);
@@ -327,22 +329,25 @@ template <int NSP, bool RS>
 __host__ __device__ constexpr int jump_blocks() { return NSP <= 4 ? (RS ? 6 : 8) : (NSP == 16 && RS ? 6 : 5); }
 template <int NSP, bool RS>
 __global__ void __launch_bounds__(256, (jump_blocks<NSP, RS>())) k_jump_level(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
-                                                    const uint32_t* __restrict__ flow_in, uint32_t* __restrict__ flow_out,
-                                                    uint16_t* __restrict__ cost, int sx, int sy,
-                                                    int p, int pd, int doubleProp, RsArgs rs, int rev)
+                                                    const uint32_t* flow_in, uint32_t* flow_out, uint16_t* cost,
+                                                    int sx, int sy, int p, int pd, int doubleProp, RsArgs rs, int rev)
 {
     const int2 t0 = block_tile(rev);
     const int x = t0.x + threadIdx.x, y = t0.y + threadIdx.y;
-    jump_level_px<NSP, RS>(F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, x, y);
+    chain_wait();
+    chain_trigger();
+    jump_level_px<NSP, RS, true>(F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, x, y);
 }
 
 template <int NSP>
 __global__ void __launch_bounds__(256) k_local_step(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
-                                                    const uint32_t* __restrict__ flow_in, uint32_t* __restrict__ flow_out,
-                                                    uint16_t* __restrict__ cost, int sx, int sy, int r, int rev)
+                                                    const uint32_t* flow_in, uint32_t* flow_out, uint16_t* cost,
+                                                    int sx, int sy, int r, int rev)
 {
     const int2 t0 = block_tile(rev);
     const int x = t0.x + threadIdx.x, y = t0.y + threadIdx.y;
+    chain_wait();
+    chain_trigger();
     if (x >= sx || y >= sy) return;
     local_px<NSP>(F1, F2, flow_in, flow_out, cost, sx, sy, r, x, y);
 }
@@ -590,6 +595,25 @@ cudaError_t features_keys(const uint32_t* keys, const float* up, int pitch, uint
     return cudaGetLastError();
 }
 
+// Launch of a TX x TY kernel that waits for its predecessor itself (chain_wait), on a
+// grid; `chained`: that predecessor is a kernel, and what it wrote is read after the wait.
+cudaLaunchConfig_t chain_config(dim3 grid, bool chained, cudaStream_t st)
+{
+    static cudaLaunchAttribute attr = [] {
+        cudaLaunchAttribute a = {};
+        a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        a.val.programmaticStreamSerializationAllowed = 1;
+        return a;
+    }();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(TX, TY);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cfg;
+}
+
 cudaError_t initialize(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_prev,
                        uint32_t* flow_out, uint16_t* cost, int sx, int sy, int nsp, int first, int rev,
                        cudaStream_t st)
@@ -610,21 +634,25 @@ cudaError_t seed_field(const uint32_t* F1, const uint32_t* F2, const uint32_t* f
 
 cudaError_t jump_level(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_in,
                        uint32_t* flow_out, uint16_t* cost, int sx, int sy, int nsp,
-                       int p, int pd, int doubleProp, const RsArgs& rs, int rev, cudaStream_t st)
+                       int p, int pd, int doubleProp, const RsArgs& rs, int rev, bool chained, cudaStream_t st)
 {
+    const cudaLaunchConfig_t cfg = chain_config(grid2d(sx, sy), chained, st);
+    cudaError_t e = cudaSuccess;
     if (rs.enabled) {
-        BM_DISPATCH_NSP(nsp, k_jump_level<NSP, true><<<grid2d(sx, sy), dim3(TX, TY), 0, st>>>(F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, rev));
+        BM_DISPATCH_NSP(nsp, (e = cudaLaunchKernelEx(&cfg, k_jump_level<NSP, true>, F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, rev)));
     } else {
-        BM_DISPATCH_NSP(nsp, k_jump_level<NSP, false><<<grid2d(sx, sy), dim3(TX, TY), 0, st>>>(F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, rev));
+        BM_DISPATCH_NSP(nsp, (e = cudaLaunchKernelEx(&cfg, k_jump_level<NSP, false>, F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, rev)));
     }
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t local_step(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_in, uint32_t* flow_out,
-                       uint16_t* cost, int sx, int sy, int nsp, int r, int rev, cudaStream_t st)
+                       uint16_t* cost, int sx, int sy, int nsp, int r, int rev, bool chained, cudaStream_t st)
 {
-    BM_DISPATCH_NSP(nsp, k_local_step<NSP><<<grid2d(sx, sy), dim3(TX, TY), 0, st>>>(F1, F2, flow_in, flow_out, cost, sx, sy, r, rev));
-    return cudaGetLastError();
+    const cudaLaunchConfig_t cfg = chain_config(grid2d(sx, sy), chained, st);
+    cudaError_t e = cudaSuccess;
+    BM_DISPATCH_NSP(nsp, (e = cudaLaunchKernelEx(&cfg, k_local_step<NSP>, F1, F2, flow_in, flow_out, cost, sx, sy, r, rev)));
+    return e;
 }
 
 cudaError_t random_search(const uint32_t* F1, const uint32_t* F2, uint32_t* flow, uint16_t* cost,
