@@ -397,11 +397,22 @@ __global__ void k_nn_table(unsigned int* __restrict__ idx, int n_up, int n_in)
 }
 
 
-__global__ void __launch_bounds__(256) k_downsample(const uint32_t* __restrict__ flow, float* __restrict__ U,
+__global__ void __launch_bounds__(256) k_downsample(const uint32_t* flow, float* __restrict__ U,
                                                     float* __restrict__ V, int sx, int sy, int sx_in, int sy_in,
                                                     const float* __restrict__ taps, int P, float mx, float my,
                                                     const unsigned int* __restrict__ nnx,
-                                                    const unsigned int* __restrict__ nny)
+                                                    const unsigned int* __restrict__ nny, int rows)
+{
+    extern __shared__ float2 down_h[];
+    downsample_block(flow, U, V, sx, sy, sx_in, sy_in, taps, P, mx, my, nnx, nny, blockIdx.x * TX, blockIdx.y * rows,
+                     rows, down_h);
+}
+// Small frames, and scales whose window does not fit shared memory.
+__global__ void __launch_bounds__(256) k_downsample_px(const uint32_t* __restrict__ flow, float* __restrict__ U,
+                                                       float* __restrict__ V, int sx, int sy, int sx_in, int sy_in,
+                                                       const float* __restrict__ taps, int P, float mx, float my,
+                                                       const unsigned int* __restrict__ nnx,
+                                                       const unsigned int* __restrict__ nny)
 {
     const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
     if (x >= sx_in || y >= sy_in) return;
@@ -674,12 +685,36 @@ cudaError_t nn_table(unsigned int* idx, int n_up, int n_in, cudaStream_t st)
     return cudaGetLastError();
 }
 
+// SMs of the current device.
+static cudaError_t sm_count(int* sms)
+{
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    return e == cudaSuccess ? cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) : e;
+}
+
 cudaError_t downsample(const uint32_t* flow, float* U, float* V, int sx, int sy, int sx_in, int sy_in,
                        const float* taps, int P, float mx, float my, const unsigned int* nnx,
                        const unsigned int* nny, cudaStream_t st)
 {
-    k_downsample<<<grid2d(sx_in, sy_in), dim3(TX, TY), 0, st>>>(flow, U, V, sx, sy, sx_in, sy_in, taps, P, mx, my,
-                                                                nnx, nny);
+    // By blocks of 32 rows, or as many as fit the 48 KB that need no opt-in, for windows
+    // of 11 taps and more (1920x1080 from u2.9 on) where those give every SM two blocks:
+    // 1920x1080 u4.9, 19 taps, 426 us per pixel, 184 by blocks.  With fewer taps a pass per
+    // pixel is as fast (1024x436 u2.9, 7 taps: 22.5 and 21.5; 584x388 u1.5, 3 taps: 8.2 and
+    // 8.8) and does not change the SMs' split between L1 and
+    // shared memory, which cost a batch of 12 pairs on several streams 1 %.
+    int sms = 0;
+    const cudaError_t e = sm_count(&sms);
+    if (e != cudaSuccess) return e;
+    int rows = 4 * TY;
+    while (rows > TY && down_smem_bytes(rows, sy, sy_in, P) > DOWN_SMEM_MAX) rows /= 2;
+    const size_t smem = down_smem_bytes(rows, sy, sy_in, P);
+    if (P < 11 || smem > DOWN_SMEM_MAX || (long)((sx_in + TX - 1) / TX) * ((sy_in + 4 * TY - 1) / (4 * TY)) < 2L * sms)
+        k_downsample_px<<<grid2d(sx_in, sy_in), dim3(TX, TY), 0, st>>>(flow, U, V, sx, sy, sx_in, sy_in, taps, P, mx, my,
+                                                                       nnx, nny);
+    else
+        k_downsample<<<dim3((sx_in + TX - 1) / TX, (sy_in + rows - 1) / rows), dim3(TX, TY), smem, st>>>(
+            flow, U, V, sx, sy, sx_in, sy_in, taps, P, mx, my, nnx, nny, rows);
     return cudaGetLastError();
 }
 
@@ -756,9 +791,8 @@ cudaError_t trilateral(const float* U, const float* V, const float* Um, const fl
             kernel<<<g, dim3(TX, ty, TRI_G), tri_smem_bytes(s, ty), st>>>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, tc.kE, tc.kI,
                                                                          cS);
         };
-        int dev = 0, sms = 0;
-        e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        int sms = 0;
+        e = sm_count(&sms);
         if (e != cudaSuccess) return e;
         switch (trilateral_rows(sx, sy, s, sms)) {
         case 2: launch(k_trilateral<2>, 2); break;
