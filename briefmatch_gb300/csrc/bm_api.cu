@@ -276,12 +276,13 @@ bmk::RsArgs rs_args(const bm_ctx* c, bool enabled)
     return rs;
 }
 
-bm_status features_into(bm_ctx* c, const float* d_up, uint32_t* F, bool padded = false)
+// `chained`: the up-sampling is the launch before (padded only).
+bm_status features_into(bm_ctx* c, const float* d_up, uint32_t* F, bool padded = false, bool chained = false)
 {
     const bm_params& p = c->prm;
     if (padded) {
         BM_LAUNCH(c, "features", bmk::features_keys(c->upad_keys(), c->d_upad, c->up_pitch(), F, (int)p.sx, (int)p.sy,
-                                                    (int)c->nsp, c->pattern_off_pad, next_order(c), c->stream));
+                                                    (int)c->nsp, c->pattern_off_pad, next_order(c), chained, c->stream));
         return BM_OK;
     }
     BM_LAUNCH(c, "features", bmk::features(d_up, F, (int)p.sx, (int)p.sy, (int)p.N, (int)c->nsp, c->d_pattern, c->pattern_rmax,
@@ -336,10 +337,10 @@ bm_status local_steps_impl(bm_ctx* c)
 // BriefMatch::match.  With a proposal network attached (and its prediction in
 // d_pred), the initialisation is the seeded one and the iteration count and jump
 // maximum are the proposal's.
-bm_status match_impl(bm_ctx* c, const float* d_im2, bool seeded, bool padded = false)
+bm_status match_impl(bm_ctx* c, const float* d_im2, bool seeded, bool padded = false, bool chained = false)
 {
     const bm_params& p = c->prm;
-    bm_status st = features_into(c, d_im2, c->feat2_ptr(), padded);
+    bm_status st = features_into(c, d_im2, c->feat2_ptr(), padded, chained);
     if (st != BM_OK) return st;
     const int first = (c->first_match || !p.tInit) ? 1 : 0;
     uint32_t iterations = p.iterations, jfMax = p.jfMax;
@@ -348,13 +349,14 @@ bm_status match_impl(bm_ctx* c, const float* d_im2, bool seeded, bool padded = f
         const int w4 = (int)c->net_w4(), h4 = (int)c->net_h4();
         const float cell = 4.0f * (float)c->net_reduce;
         const float scx = cell * (float)p.sx / (float)p.sx_in, scy = cell * (float)p.sy / (float)p.sy_in;
+        const bool waited = c->net_pending;
         if (c->net_pending) {  // the proposal computed on the side stream
             BM_CUDA(cudaStreamWaitEvent(c->stream, c->ev_net, 0));
             c->net_pending = false;
         }
         BM_LAUNCH(c, "seed", bmk::seed_field(c->feat1_ptr(), c->feat2_ptr(), c->d_flow[c->flow_cur], c->d_flow[c->flow_cur ^ 1],
                                              c->d_cost, (int)p.sx, (int)p.sy, (int)c->nsp, first, c->d_pred, w4, h4, scx,
-                                             scy, c->net_logit_min, c->stream));
+                                             scy, c->net_logit_min, !waited, c->stream));
         iterations = c->net_iterations;
         if (c->net_jfMax) jfMax = c->net_jfMax;
         c->flow_cur ^= 1;
@@ -362,7 +364,7 @@ bm_status match_impl(bm_ctx* c, const float* d_im2, bool seeded, bool padded = f
         if (st != BM_OK) return st;
     } else {
         BM_LAUNCH(c, "initialize", bmk::initialize(c->feat1_ptr(), c->feat2_ptr(), c->d_flow[c->flow_cur], c->d_flow[c->flow_cur ^ 1],
-                                     c->d_cost, (int)p.sx, (int)p.sy, (int)c->nsp, first, next_order(c), c->stream));
+                                     c->d_cost, (int)p.sx, (int)p.sy, (int)c->nsp, first, next_order(c), true, c->stream));
         c->flow_cur ^= 1;
     }
     int pd = -1;
@@ -375,7 +377,8 @@ bm_status match_impl(bm_ctx* c, const float* d_im2, bool seeded, bool padded = f
     return BM_OK;
 }
 
-bm_status downsample_impl(bm_ctx* c)
+// `chained`: a level is the launch before.
+bm_status downsample_impl(bm_ctx* c, bool chained)
 {
     const bm_params& p = c->prm;
     float* U = c->d_flow_in;
@@ -384,15 +387,16 @@ bm_status downsample_impl(bm_ctx* c)
         const float mx = (float)p.sx_in / (float)p.sx;  // briefmatch.cpp:316-317
         const float my = (float)p.sy_in / (float)p.sy;
         BM_LAUNCH(c, "downsample", bmk::downsample(c->d_flow[c->flow_cur], U, V, (int)p.sx, (int)p.sy, (int)p.sx_in, (int)p.sy_in,
-                                     c->d_taps, (int)p.P, mx, my, c->d_nnx, c->d_nny, c->stream));
+                                     c->d_taps, (int)p.P, mx, my, c->d_nnx, c->d_nny, chained, c->stream));
     } else {
         // briefmatch.cpp:319-323: the converted field is the output
-        BM_LAUNCH(c, "flow_to_planes", bmk::flow_to_planes(c->d_flow[c->flow_cur], U, V, c->npix, c->stream));
+        BM_LAUNCH(c, "flow_to_planes", bmk::flow_to_planes(c->d_flow[c->flow_cur], U, V, c->npix, chained, c->stream));
     }
     return BM_OK;
 }
 
-bm_status process_impl(bm_ctx* c, const float* d_prev_in)
+// `chained`: the down-sampling is the launch before.
+bm_status process_impl(bm_ctx* c, const float* d_prev_in, bool chained)
 {
     const bm_params& p = c->prm;
     const size_t n = c->npix_in;
@@ -401,12 +405,12 @@ bm_status process_impl(bm_ctx* c, const float* d_prev_in)
     if (p.filter) {
         if (!d_prev_in) return fail(BM_ERR_INVALID, "process: the guide frame is required when filtering");
         const int fs = p.fsize == 0 ? 1 : (int)p.fsize;
-        BM_LAUNCH(c, "median_pass", bmk::median_pass(U, V, c->d_tmp, c->d_tmp + n, 1, fs, (int)p.sx_in, (int)p.sy_in, c->stream));
+        BM_LAUNCH(c, "median_pass", bmk::median_pass(U, V, c->d_tmp, c->d_tmp + n, 1, fs, (int)p.sx_in, (int)p.sy_in, chained, c->stream));
         BM_LAUNCH(c, "median_pass", bmk::median_pass(c->d_tmp, c->d_tmp + n, c->d_flow_med, c->d_flow_med + n, 0, fs, (int)p.sx_in,
-                                      (int)p.sy_in, c->stream));
+                                      (int)p.sy_in, true, c->stream));
         BM_LAUNCH(c, "trilateral", bmk::trilateral(U, V, c->d_flow_med, c->d_flow_med + n, d_prev_in, c->d_flow_out,
                                      c->d_flow_out + n, (int)p.sx_in, (int)p.sy_in, c->tri_s, p.sEPE * p.sEPE,
-                                     p.sI * p.sI, p.sS * p.sS, c->stream));
+                                     p.sI * p.sI, p.sS * p.sS, true, c->stream));
     } else {
         BM_CUDA(cudaMemcpyAsync(c->d_flow_out, c->d_flow_in, 2 * n * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
     }
@@ -760,7 +764,7 @@ bm_status bm_initialize(bm_ctx* c, int first)
     if (check_ctx(c)) return BM_ERR_INVALID;
     const bm_params& p = c->prm;
     BM_LAUNCH(c, "initialize", bmk::initialize(c->feat1_ptr(), c->feat2_ptr(), c->d_flow[c->flow_cur], c->d_flow[c->flow_cur ^ 1],
-                                 c->d_cost, (int)p.sx, (int)p.sy, (int)c->nsp, first ? 1 : 0, next_order(c), c->stream));
+                                 c->d_cost, (int)p.sx, (int)p.sy, (int)c->nsp, first ? 1 : 0, next_order(c), false, c->stream));
     c->flow_cur ^= 1;
     return BM_OK;
 }
@@ -794,14 +798,14 @@ bm_status bm_downsample(bm_ctx* c)
 {
     if (check_ctx(c)) return BM_ERR_INVALID;
     BM_CUDA(join_refine(c));
-    return downsample_impl(c);
+    return downsample_impl(c, false);
 }
 
 bm_status bm_process(bm_ctx* c, const float* d_prev_in)
 {
     if (check_ctx(c)) return BM_ERR_INVALID;
     BM_CUDA(join_refine(c));
-    return process_impl(c, d_prev_in);
+    return process_impl(c, d_prev_in, false);
 }
 
 bm_status bm_swap(bm_ctx* c)
@@ -982,7 +986,7 @@ bm_status bm_seed(bm_ctx* c, int first, const float* d_pred, uint32_t w4, uint32
     BM_LAUNCH(c, "seed", bmk::seed_field(c->feat1_ptr(), c->feat2_ptr(), c->d_flow[c->flow_cur], c->d_flow[c->flow_cur ^ 1],
                                          c->d_cost, (int)p.sx, (int)p.sy, (int)c->nsp, first ? 1 : 0, d_pred, (int)w4,
                                          (int)h4, scx, scy, std::log(conf_threshold / (1.0f - conf_threshold)),
-                                         c->stream));
+                                         false, c->stream));
     c->flow_cur ^= 1;
     return BM_OK;
 }
@@ -1057,17 +1061,19 @@ bm_status bm_frame(bm_ctx* c, const uint8_t* frame, int frame_on_device, float* 
         c->launches += 7;
     }
     float* cur = c->d_frame[slot];
-    BM_LAUNCH(c, "u8_to_f32", bmk::u8_to_f32(d_u8, cur, ni, c->stream));
     // of_pipeline.cpp:301-310
     const float* up = cur;
     const bool padded = c->upad_use;
     if (padded) {
-        BM_LAUNCH(c, "upsample_u8", bmk::upsample_u8_pad(d_u8, c->d_upad, c->upad_keys(), c->up_pitch(), c->up_margin,
+        BM_LAUNCH(c, "upsample_u8", bmk::upsample_u8_pad(d_u8, cur, c->d_upad, c->upad_keys(), c->up_pitch(), c->up_margin,
                                                          (int)p.sx_in, (int)p.sy_in, (int)p.sx, (int)p.sy, c->d_lx,
                                                          c->d_ix, c->d_ly, c->d_iy, c->stream));
         up = c->upad_origin();
         c->upad_valid = true;
-    } else if (p.sx != p.sx_in || p.sy != p.sy_in) {
+    } else {
+        BM_LAUNCH(c, "u8_to_f32", bmk::u8_to_f32(d_u8, cur, ni, c->stream));
+    }
+    if (!padded && (p.sx != p.sx_in || p.sy != p.sy_in)) {
         BM_LAUNCH(c, "upsample_u8", bmk::upsample_u8(d_u8, c->d_up, (int)p.sx_in, (int)p.sy_in, (int)p.sx, (int)p.sy,
                                                      c->d_lx, c->d_ix, c->d_ly, c->d_iy, c->stream));
         up = c->d_up;
@@ -1076,7 +1082,7 @@ bm_status bm_frame(bm_ctx* c, const uint8_t* frame, int frame_on_device, float* 
     bm_status st;
     bool refine_async = false;
     if (!c->primed) {
-        st = features_into(c, up, c->feat2_ptr(), padded);
+        st = features_into(c, up, c->feat2_ptr(), padded, padded);
         if (st != BM_OK) return st;
         BM_CUDA(join_refine(c));
         BM_CUDA(cudaMemsetAsync(c->d_flow_out, 0, 2 * ni * sizeof(float), c->stream));
@@ -1089,7 +1095,7 @@ bm_status bm_frame(bm_ctx* c, const uint8_t* frame, int frame_on_device, float* 
             if (st != BM_OK) return st;
             c->launches += 7;
         }
-        st = match_impl(c, up, seeded, padded);                   // of_pipeline.cpp:314
+        st = match_impl(c, up, seeded, padded, padded && !(seeded && !c->net_side));                   // of_pipeline.cpp:314
         if (st != BM_OK) return st;
         if (c->pipelined) {
             // the down-sampled flow alternates between two buffers; the refinement of
@@ -1098,7 +1104,7 @@ bm_status bm_frame(bm_ctx* c, const uint8_t* frame, int frame_on_device, float* 
             c->d_flow_in = c->d_flow_in_buf[c->flow_in_slot];
             BM_CUDA(cudaStreamWaitEvent(c->stream, c->ev_flowin_free[c->flow_in_slot], 0));
         }
-        st = downsample_impl(c);                                  // :319
+        st = downsample_impl(c, !c->pipelined);                                  // :319
         if (st != BM_OK) return st;
         if (c->pipelined) {
             // refinement (:324) and the output copies on the refinement stream, while
@@ -1107,7 +1113,7 @@ bm_status bm_frame(bm_ctx* c, const uint8_t* frame, int frame_on_device, float* 
             BM_CUDA(cudaStreamWaitEvent(c->refine_stream, c->ev_ready, 0));
             const cudaStream_t main = c->stream;
             c->stream = c->refine_stream;
-            st = process_impl(c, c->d_frame[prev]);
+            st = process_impl(c, c->d_frame[prev], false);
             cudaError_t e = cudaSuccess;
             if (st == BM_OK) {
                 e = cudaEventRecord(c->ev_flowin_free[c->flow_in_slot], c->refine_stream);
@@ -1118,7 +1124,7 @@ bm_status bm_frame(bm_ctx* c, const uint8_t* frame, int frame_on_device, float* 
             BM_CUDA(e);
             refine_async = true;
         } else {
-            st = process_impl(c, c->d_frame[prev]);               // :324
+            st = process_impl(c, c->d_frame[prev], true);               // :324
             if (st != BM_OK) return st;
         }
     }

@@ -415,7 +415,6 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
     const PairDev& d = b->pairs[j];
     const size_t ni = (size_t)d.sx_in * d.sy_in;
     const bool resample = d.sx != d.sx_in || d.sy != d.sy_in;
-    BB_CUDA(u8_to_f32(d.frame[0], d.guide, ni, st));
     int rev = 0;
     // descriptors from the edge-replicated up-sampled image while the pair's pattern
     // fits the margin its buffer was laid out with; from the dense image otherwise
@@ -424,11 +423,12 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
     for (int which = 0; which < 2; which++) {
         if (padded) {
             uint32_t* keys = reinterpret_cast<uint32_t*>(d.up + (size_t)pitch * (d.sy + 2 * d.up_margin));
-            BB_CUDA(upsample_u8_pad(d.frame[which], d.up, keys, pitch, d.up_margin, d.sx_in, d.sy_in, d.sx, d.sy, d.lx,
-                                    d.ix, d.ly, d.iy, st));
+            BB_CUDA(upsample_u8_pad(d.frame[which], which == 0 ? d.guide : nullptr, d.up, keys, pitch, d.up_margin,
+                                    d.sx_in, d.sy_in, d.sx, d.sy, d.lx, d.ix, d.ly, d.iy, st));
             BB_CUDA(features_keys(keys, d.up, pitch, d.F[which], d.sx, d.sy, (int)b->nsp, b->pattern_off_pad[j], rev,
-                                  st));
+                                  false, st));
         } else {
+            if (which == 0) BB_CUDA(u8_to_f32(d.frame[0], d.guide, ni, st));
             if (resample)
                 BB_CUDA(upsample_u8(d.frame[which], d.up, d.sx_in, d.sy_in, d.sx, d.sy, d.lx, d.ix, d.ly, d.iy, st));
             else
@@ -451,7 +451,7 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
         const float cell = 4.0f * (float)red;
         const float scx = cell * (float)d.sx / (float)d.sx_in, scy = cell * (float)d.sy / (float)d.sy_in;
         BB_CUDA(seed_field(d.F[0], d.F[1], d.flow[cur], d.flow[cur ^ 1], d.cost, d.sx, d.sy, (int)b->nsp, 1, d_pred,
-                           (int)w4, (int)h4, scx, scy, b->net_logit_min, st));
+                           (int)w4, (int)h4, scx, scy, b->net_logit_min, false, st));
         iterations = b->net_iterations;
         if (b->net_jfMax) jfMax = b->net_jfMax;
         b->launches += 8;
@@ -466,7 +466,7 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
         }
         b->launches += b->local_steps;
     } else {
-        BB_CUDA(initialize(d.F[0], d.F[1], d.flow[cur], d.flow[cur ^ 1], d.cost, d.sx, d.sy, (int)b->nsp, 1, rev, st));
+        BB_CUDA(initialize(d.F[0], d.F[1], d.flow[cur], d.flow[cur ^ 1], d.cost, d.sx, d.sy, (int)b->nsp, 1, rev, false, st));
         rev ^= s.snake ? 1 : 0;
         cur ^= 1;
     }
@@ -491,11 +491,11 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
     }
     if (resample) {
         BB_CUDA(downsample(d.flow[cur], d.flow_in, d.flow_in + ni, d.sx, d.sy, d.sx_in, d.sy_in, d.taps, d.P, d.mx,
-                           d.my, d.nnx, d.nny, st));
+                           d.my, d.nnx, d.nny, false, st));
     } else {
-        BB_CUDA(flow_to_planes(d.flow[cur], d.flow_in, d.flow_in + ni, ni, st));
+        BB_CUDA(flow_to_planes(d.flow[cur], d.flow_in, d.flow_in + ni, ni, false, st));
     }
-    b->launches += 6 + (uint64_t)iterations * levels - (net ? 1 : 0);
+    b->launches += (padded ? 5 : 6) + (uint64_t)iterations * levels - (net ? 1 : 0);
     return BM_OK;
 }
 
@@ -642,11 +642,11 @@ bm_status enqueue_refine_pair(bm_batch* b, int j, cudaStream_t st)
     const size_t ni = (size_t)d.sx_in * d.sy_in;
     if (b->filter) {
         const int fs = d.fsize == 0 ? 1 : d.fsize;
-        BB_CUDA(median_pass(d.flow_in, d.flow_in + ni, d.tmp, d.tmp + ni, 1, fs, d.sx_in, d.sy_in, st));
-        BB_CUDA(median_pass(d.tmp, d.tmp + ni, d.flow_med, d.flow_med + ni, 0, fs, d.sx_in, d.sy_in, st));
+        BB_CUDA(median_pass(d.flow_in, d.flow_in + ni, d.tmp, d.tmp + ni, 1, fs, d.sx_in, d.sy_in, false, st));
+        BB_CUDA(median_pass(d.tmp, d.tmp + ni, d.flow_med, d.flow_med + ni, 0, fs, d.sx_in, d.sy_in, false, st));
         BB_CUDA(trilateral(d.flow_in, d.flow_in + ni, d.flow_med, d.flow_med + ni, d.guide, d.flow_out,
                            d.flow_out + ni, d.sx_in, d.sy_in, d.tri_s, p.sEPE * p.sEPE, p.sI * p.sI, p.sS * p.sS,
-                           st));
+                           false, st));
         b->launches += 3;
     } else {
         BB_CUDA(cudaMemcpyAsync(d.flow_out, d.flow_in, 2 * ni * sizeof(float), cudaMemcpyDeviceToDevice, st));

@@ -35,32 +35,32 @@ __device__ __forceinline__ void store_desc(uint32_t* dst, const uint32_t (&w)[NS
     }
 }
 
-template <int NSP>
-__device__ __forceinline__ void load_desc(uint32_t (&w)[NSP], const uint32_t* __restrict__ src)
+template <int NSP, bool L2 = false>
+__device__ __forceinline__ void load_desc(uint32_t (&w)[NSP], const uint32_t* src)
 {
     if constexpr (NSP >= 4) {
 #pragma unroll
         for (int k = 0; k < NSP / 4; k++) {
-            uint4 v = __ldg(reinterpret_cast<const uint4*>(src) + k);
+            uint4 v = L2 ? __ldcg(reinterpret_cast<const uint4*>(src) + k) : __ldg(reinterpret_cast<const uint4*>(src) + k);
             w[4 * k] = v.x;
             w[4 * k + 1] = v.y;
             w[4 * k + 2] = v.z;
             w[4 * k + 3] = v.w;
         }
     } else if constexpr (NSP == 2) {
-        uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+        uint2 v = L2 ? __ldcg(reinterpret_cast<const uint2*>(src)) : __ldg(reinterpret_cast<const uint2*>(src));
         w[0] = v.x;
         w[1] = v.y;
     } else {
-        w[0] = __ldg(src);
+        w[0] = L2 ? __ldcg(src) : __ldg(src);
     }
 }
 
-template <int NSP>
-__device__ __forceinline__ int hamming(const uint32_t (&a)[NSP], const uint32_t* __restrict__ pb)
+template <int NSP, bool L2 = false>
+__device__ __forceinline__ int hamming(const uint32_t (&a)[NSP], const uint32_t* pb)
 {
     uint32_t b[NSP];
-    load_desc<NSP>(b, pb);
+    load_desc<NSP, L2>(b, pb);
     int h = 0;
 #pragma unroll
     for (int k = 0; k < NSP; k++) h += __popc(a[k] ^ b[k]);
@@ -317,9 +317,11 @@ __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.l
 // PatchMatch (briefmatch_cuda.cu:126-246).
 // ---------------------------------------------------------------------------
 // Zero or temporal initialisation (briefmatch_cuda.cu:149-184); temporal init reads
-// the previous field from flow_prev (a snapshot) and writes flow_out.
-template <int NSP>
-__device__ __forceinline__ void init_px(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
+// the previous field from flow_prev (a snapshot) and writes flow_out.  CHAINED: the
+// launch before may have written the descriptors after this one started; they are read
+// through L2.
+template <int NSP, bool CHAINED = false>
+__device__ __forceinline__ void init_px(const uint32_t* F1, const uint32_t* F2,
                                         const uint32_t* __restrict__ flow_prev, uint32_t* __restrict__ flow_out,
                                         uint16_t* __restrict__ cost, int sx, int sy, int first, int x, int y)
 {
@@ -334,8 +336,8 @@ __device__ __forceinline__ void init_px(const uint32_t* __restrict__ F1, const u
         ny = min(max(hi16(t), -y), sy - y - 1);
     }
     uint32_t f1[NSP];
-    load_desc<NSP>(f1, F1 + pix * NSP);
-    cost[pix] = (uint16_t)hamming<NSP>(f1, F2 + (pix + nx + (long)ny * sx) * NSP);
+    load_desc<NSP, CHAINED>(f1, F1 + pix * NSP);
+    cost[pix] = (uint16_t)hamming<NSP, CHAINED>(f1, F2 + (pix + nx + (long)ny * sx) * NSP);
     flow_out[pix] = pack_flow(nx, ny);
 }
 
@@ -343,9 +345,10 @@ __device__ __forceinline__ void init_px(const uint32_t* __restrict__ F1, const u
 // temporal candidate when !first, exactly as init_px), then the network's proposal
 // for this pixel -- pred is [h4][w4][3] (u, v in quarter-resolution input pixels,
 // confidence logit) -- where its confidence logit reaches logit_min; the proposal
-// replaces the plain vector only if its Hamming cost is strictly lower.
+// replaces the plain vector only if its Hamming cost is strictly lower.  Descriptors are
+// read through L2 (chained launch, as init_px).
 template <int NSP>
-__device__ __forceinline__ void seed_px(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
+__device__ __forceinline__ void seed_px(const uint32_t* F1, const uint32_t* F2,
                                         const uint32_t* __restrict__ flow_prev, uint32_t* __restrict__ flow_out,
                                         uint16_t* __restrict__ cost, int sx, int sy, int first, int x, int y,
                                         const float* __restrict__ pred, int w4, int h4, float scale_x, float scale_y,
@@ -362,8 +365,8 @@ __device__ __forceinline__ void seed_px(const uint32_t* __restrict__ F1, const u
         ny = min(max(hi16(t), -y), sy - y - 1);
     }
     uint32_t f1[NSP];
-    load_desc<NSP>(f1, F1 + pix * NSP);
-    int h = hamming<NSP>(f1, F2 + (pix + nx + (long)ny * sx) * NSP);
+    load_desc<NSP, true>(f1, F1 + pix * NSP);
+    int h = hamming<NSP, true>(f1, F2 + (pix + nx + (long)ny * sx) * NSP);
     // quarter-resolution cell of this up-sampled pixel (scale = up-sampled px per
     // quarter-resolution px, inv = its reciprocal from the host, so the cell index
     // is one IEEE add and multiply: no approximate division)
@@ -374,7 +377,7 @@ __device__ __forceinline__ void seed_px(const uint32_t* __restrict__ F1, const u
         const int sxv = min(max(__float2int_rn(pr[0] * scale_x), -x), sx - x - 1);
         const int syv = min(max(__float2int_rn(pr[1] * scale_y), -y), sy - y - 1);
         if (sxv != nx || syv != ny) {
-            const int hs = hamming<NSP>(f1, F2 + (pix + sxv + (long)syv * sx) * NSP);
+            const int hs = hamming<NSP, true>(f1, F2 + (pix + sxv + (long)syv * sx) * NSP);
             if (hs < h) {
                 h = hs;
                 nx = sxv;
@@ -722,7 +725,7 @@ __device__ __forceinline__ void local_px(const uint32_t* __restrict__ F1, const 
 // decimation samples (source index tables nnx/nny), scaled by (mx, my).  Each
 // pass keeps the reference's float rounding and fused multiply-adds.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void downsample_px(const uint32_t* __restrict__ flow, float* __restrict__ U,
+__device__ __forceinline__ void downsample_px(const uint32_t* flow, float* __restrict__ U,
                                               float* __restrict__ V, int sx, int sy, int sx_in,
                                               const float* __restrict__ taps, int P, float mx, float my,
                                               const unsigned int* __restrict__ nnx, const unsigned int* __restrict__ nny,
@@ -742,7 +745,7 @@ __device__ __forceinline__ void downsample_px(const uint32_t* __restrict__ flow,
         const uint32_t* row = flow + (size_t)yy * sx;
         float hu = 0, hv = 0;
         for (int k = 0; k < P; k++) {
-            const uint32_t f = __ldg(row + min(sx - 1, max(0, (int)x1 + k - ks2)));
+            const uint32_t f = row[min(sx - 1, max(0, (int)x1 + k - ks2))];
             const float tk = taps[k];
             hu += tk * float(lo16(f));
             hv += tk * float(hi16(f));
@@ -828,11 +831,11 @@ __device__ __forceinline__ void downsample_block(const uint32_t* flow, float* __
 // FS-1) serves both outputs.
 // ---------------------------------------------------------------------------
 template <int FS>
-__device__ __forceinline__ void median2_px(const float* __restrict__ in, float* __restrict__ out, long p, long step,
+__device__ __forceinline__ void median2_px(const float* in, float* __restrict__ out, long p, long step,
                                            long n, int fsize, bool second)
 {
     const int ks = fsize / 2;
-    auto sample = [&](long idx) { return (idx >= 0 && idx < n) ? __ldg(in + idx) : 0.0f; };
+    auto sample = [&](long idx) { return (idx >= 0 && idx < n) ? in[idx] : 0.0f; };
     const float a = sample(p - (long)ks * step);
     const float b = second ? sample(p + (long)(fsize - ks) * step) : 0.0f;
     if (fsize == 1) {
@@ -930,7 +933,7 @@ __device__ __forceinline__ f2x ex2n_2(f2x a) { return pk2(ex2n(lo2(a)), ex2n(hi2
 
 template <int TY>
 __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, const float* __restrict__ V,
-                                                 const float* __restrict__ Um, const float* __restrict__ Vm,
+                                                 const float* Um, const float* Vm,
                                                  const float* __restrict__ I, float* __restrict__ Uo,
                                                  float* __restrict__ Vo, int sx, int sy, int s, float kE, float kI,
                                                  float cS, int bx0, int by0, float4* smem4)
@@ -945,7 +948,7 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
     const int x0 = bx0 - s, y0 = by0 - s;
     // the block's reference flow and intensity
     const size_t mid = (size_t)min(sx - 1, bx0 + TX / 2) + (size_t)min(sy - 1, by0 + tri_rows(TY) / 2) * sx;
-    const float ru = tri_reference(__ldg(Um + mid)), rv = tri_reference(__ldg(Vm + mid)), ri = tri_reference(__ldg(I + mid));
+    const float ru = tri_reference(Um[mid]), rv = tri_reference(Vm[mid]), ri = tri_reference(__ldg(I + mid));
     for (int r = threadIdx.z * TY + threadIdx.y; r < TH; r += TY * TRI_G) {
         const size_t row = (size_t)min(sy - 1, max(0, y0 + r)) * sx;
         for (int c = threadIdx.x; c < TW; c += TX) {
@@ -970,7 +973,7 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
 #pragma unroll
     for (int r = 0; r < TRI_R; r++) {
         const size_t o = (size_t)min(sx - 1, x) + (size_t)min(sy - 1, yb + r) * sx;
-        const float a = __fmul_rn(-kE, __fsub_rn(__ldg(Um + o), ru)), b = __fmul_rn(-kE, __fsub_rn(__ldg(Vm + o), rv));
+        const float a = __fmul_rn(-kE, __fsub_rn(Um[o], ru)), b = __fmul_rn(-kE, __fsub_rn(Vm[o], rv));
         const float i0 = -sI[(threadIdx.x + s) * P + threadIdx.y * TRI_R + r + s];
         um[r] = pk2(a, a);
         vm[r] = pk2(b, b);

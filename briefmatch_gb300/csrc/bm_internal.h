@@ -50,7 +50,7 @@ cudaError_t upsample_u8(const uint8_t* in, float* out, int sxi, int syi, int sxo
 // side; `out` is the start of the (sxo + 2m) x (syo + 2m) buffer, row pitch `pitch`.
 // `keys`, of the same shape, receives the 16-bit keys the descriptors compare first: per
 // word the pixel's key and that of the pixel below it.
-cudaError_t upsample_u8_pad(const uint8_t* in, float* out, uint32_t* keys, int pitch, int m, int sxi, int syi, int sxo,
+cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_t* keys, int pitch, int m, int sxi, int syi, int sxo,
                             int syo, const float* lx, const int* ix, const float* ly, const int* iy, cudaStream_t st);
 cudaError_t u8_to_f32(const uint8_t* in, float* out, size_t n, cudaStream_t st);
 
@@ -76,22 +76,23 @@ void key_offsets(KeyOffsets& ko, const int4* pat, int N, int m, int pitch);
 // pixels does not); the dense image serves the others.
 bool key_image_fits(int m, int pitch);
 
+// `chained` in a launcher: the launch before it on the stream is a kernel that either was
+// launched unchained or itself waits for its predecessor before it lets the next start
+// (the stages of one frame in a row); this one may then start under its last blocks.
+
 // Descriptors from an edge-replicated image and its keys (upsample_u8_pad): both point
 // at the start of the margin, which is no narrower than the largest pattern offset.
 cudaError_t features_keys(const uint32_t* keys, const float* up, int pitch, uint32_t* F, int sx, int sy, int nsp,
-                          const KeyOffsets& ko, int rev, cudaStream_t st);
+                          const KeyOffsets& ko, int rev, bool chained, cudaStream_t st);
 
 cudaError_t initialize(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_prev,
                        uint32_t* flow_out, uint16_t* cost, int sx, int sy, int nsp, int first, int rev,
-                       cudaStream_t st);
+                       bool chained, cudaStream_t st);
 
 cudaError_t seed_field(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_prev, uint32_t* flow_out,
                        uint16_t* cost, int sx, int sy, int nsp, int first, const float* pred, int w4, int h4,
-                       float scale_x, float scale_y, float logit_min, cudaStream_t st);
+                       float scale_x, float scale_y, float logit_min, bool chained, cudaStream_t st);
 
-// `chained` (here and in jump_level): the launch before this one on the stream is the
-// initialisation, a local step or a level of the same field and descriptors, and this
-// one may start under its last blocks.
 cudaError_t local_step(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_in, uint32_t* flow_out,
                        uint16_t* cost, int sx, int sy, int nsp, int r, int rev, bool chained, cudaStream_t st);
 
@@ -107,12 +108,12 @@ cudaError_t normals(float2* out, int sx, int sy, const RsArgs& rs, cudaStream_t 
 cudaError_t nn_table(unsigned int* idx, int n_up, int n_in, cudaStream_t st);
 cudaError_t downsample(const uint32_t* flow, float* U, float* V, int sx, int sy, int sx_in, int sy_in,
                        const float* taps, int P, float mx, float my, const unsigned int* nnx,
-                       const unsigned int* nny, cudaStream_t st);
+                       const unsigned int* nny, bool chained, cudaStream_t st);
 
-cudaError_t flow_to_planes(const uint32_t* flow, float* U, float* V, size_t n, cudaStream_t st);
+cudaError_t flow_to_planes(const uint32_t* flow, float* U, float* V, size_t n, bool chained, cudaStream_t st);
 
 cudaError_t median_pass(const float* inU, const float* inV, float* outU, float* outV,
-                        int dir, int fsize, int sx, int sy, cudaStream_t st);
+                        int dir, int fsize, int sx, int sy, bool chained, cudaStream_t st);
 
 // Half window of the cross-trilateral filter, s = ceil(2.5*sqrt(sS^2))
 // (briefmatch_cuda.cu:266), for an input frame of w x h pixels.  Returns -1 when a
@@ -131,7 +132,7 @@ inline int trilateral_half_window(float sEPE, float sI, float sS, uint32_t w, ui
 cudaError_t ensure_trilateral_smem(int s);
 cudaError_t trilateral(const float* U, const float* V, const float* Um, const float* Vm,
                        const float* I, float* Uo, float* Vo, int sx, int sy, int s,
-                       float sigmaEPE2, float sigmaI2, float sigmaS2, cudaStream_t st);
+                       float sigmaEPE2, float sigmaI2, float sigmaS2, bool chained, cudaStream_t st);
 
 // Colour coding of a flow field (u, v planes of n floats) into n*3 bytes R G B
 // (briefmatch.cpp:373-421, colorcode.cpp:52-74).  max_motion > 0 normalises by it;

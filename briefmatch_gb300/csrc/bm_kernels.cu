@@ -86,16 +86,26 @@ __global__ void __launch_bounds__(256) k_upsample(const T* __restrict__ in, floa
 // Beside the float image the kernel writes the key image the descriptors read: a word
 // per pixel with the 16-bit key (sample_key) of the pixel in its low half and of the
 // pixel below it in its high half.  A thread pairs the keys of its own rows; the word
-// that spans two threads' rows is written as two halves.
+// that spans two threads' rows is written as two halves.  Beside that
+// the threads write the frame itself as float into `frame` (if any), for the refinement:
+// 2 us at 1024x436 where a launch of its own took 4 to 6.  (Extra blocks for it: as fast
+// on large frames, 4 us slower on small ones.)
 constexpr int UP_R = 8;
-__global__ void __launch_bounds__(TX * TY) k_upsample_pad_rows(const uint8_t* __restrict__ in, float* __restrict__ out,
+__global__ void __launch_bounds__(TX * TY) k_upsample_pad_rows(const uint8_t* __restrict__ in, float* __restrict__ frame,
+                                                               float* __restrict__ out,
                                                                uint32_t* __restrict__ keys, int pitch, int m, int sxi,
                                                                int syi, int sxo, int syo,
                                                                const float* __restrict__ lx, const int* __restrict__ ix,
                                                                const float* __restrict__ ly, const int* __restrict__ iy)
 {
+    chain_trigger();   // launched unchained: what is older is complete
     const int X = blockIdx.x * TX + threadIdx.x;
     const int Y0 = (blockIdx.y * TY + threadIdx.y) * UP_R;
+    if (frame) {
+        const size_t n = (size_t)sxi * syi, threads = (size_t)gridDim.x * gridDim.y * (TX * TY);
+        const size_t block = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+        for (size_t i = block * (TX * TY) + threadIdx.y * TX + threadIdx.x; i < n; i += threads) frame[i] = (float)in[i];
+    }
     if (X >= sxo + 2 * m || Y0 >= syo + 2 * m) return;
     const int x = min(sxo - 1, max(0, X - m));
     float Lx[6];
@@ -205,10 +215,12 @@ __global__ void __launch_bounds__(256) k_features(const float* __restrict__ I, u
 // 1-3 % better than five, seven or eight.
 constexpr int FLAT_TIES = 12, MANY_TIES = 12;
 template <int NSP>
-__global__ void __launch_bounds__(256, 6) k_features_keys(const uint32_t* __restrict__ W, const float* __restrict__ I,
+__global__ void __launch_bounds__(256, 6) k_features_keys(const uint32_t* W, const float* I,
                                                           int pitch, uint32_t* __restrict__ F, int sx, int sy,
                                                           const __grid_constant__ KeyOffsets po, int rev)
 {
+    chain_wait();
+    chain_trigger();
     int bx = blockIdx.x, by = blockIdx.y;
     if (rev) {
         bx = gridDim.x - 1 - bx;
@@ -228,7 +240,7 @@ __global__ void __launch_bounds__(256, 6) k_features_keys(const uint32_t* __rest
     // sample b of word w of pixel v on the float image
     auto larger = [&](uint2 o, int v) {
         const char* f = fbase + v * down;
-        return __ldg(reinterpret_cast<const float*>(f + o.x)) > __ldg(reinterpret_cast<const float*>(f + o.y));
+        return *reinterpret_cast<const float*>(f + o.x) > *reinterpret_cast<const float*>(f + o.y);
     };
     auto compare = [&](int w, int b, const uint32_t (&ask)[2], uint32_t (&bits)[2]) {
         const uint2 o = po.off[w * 32 + b];
@@ -259,8 +271,8 @@ __global__ void __launch_bounds__(256, 6) k_features_keys(const uint32_t* __rest
 #pragma unroll
                     for (int b = 7; b >= 0; b--) {   // the byte's low bit is its first sample
                         const uint2 o = po.off[w * 32 + g * 8 + b];
-                        const uint32_t k1 = __ldg(reinterpret_cast<const uint32_t*>(base + o.x));
-                        const uint32_t k2 = __ldg(reinterpret_cast<const uint32_t*>(base + o.y));
+                        const uint32_t k1 = *reinterpret_cast<const uint32_t*>(base + o.x);
+                        const uint32_t k2 = *reinterpret_cast<const uint32_t*>(base + o.y);
                         gt[g] = half2_shift_in(gt[g], half2_gt(k1, k2));
                         eq[g] = half2_shift_in(eq[g], half2_eq(k1, k2));
                     }
@@ -296,26 +308,28 @@ __global__ void __launch_bounds__(256, 6) k_features_keys(const uint32_t* __rest
 }
 
 template <int NSP>
-__global__ void __launch_bounds__(256) k_initialize(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
+__global__ void __launch_bounds__(256) k_initialize(const uint32_t* F1, const uint32_t* F2,
                                                     const uint32_t* __restrict__ flow_prev, uint32_t* __restrict__ flow_out,
                                                     uint16_t* __restrict__ cost, int sx, int sy, int first, int rev)
 {
     const int2 t0 = block_tile(rev);
     const int x = t0.x + threadIdx.x, y = t0.y + threadIdx.y;
-    chain_trigger();   // launched unchained: what is older is complete
+    chain_wait();
+    chain_trigger();
     if (x >= sx || y >= sy) return;
-    init_px<NSP>(F1, F2, flow_prev, flow_out, cost, sx, sy, first, x, y);
+    init_px<NSP, true>(F1, F2, flow_prev, flow_out, cost, sx, sy, first, x, y);
 }
 
 template <int NSP>
-__global__ void __launch_bounds__(256) k_seed(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
+__global__ void __launch_bounds__(256) k_seed(const uint32_t* F1, const uint32_t* F2,
                                               const uint32_t* __restrict__ flow_prev, uint32_t* __restrict__ flow_out,
                                               uint16_t* __restrict__ cost, int sx, int sy, int first,
                                               const float* __restrict__ pred, int w4, int h4, float scale_x,
                                               float scale_y, float inv_x, float inv_y, float logit_min)
 {
     const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
-    chain_trigger();   // launched unchained: what is older is complete
+    chain_wait();
+    chain_trigger();
     if (x >= sx || y >= sy) return;
     seed_px<NSP>(F1, F2, flow_prev, flow_out, cost, sx, sy, first, x, y, pred, w4, h4, scale_x, scale_y, inv_x, inv_y,
                  logit_min);
@@ -403,26 +417,31 @@ __global__ void __launch_bounds__(256) k_downsample(const uint32_t* flow, float*
                                                     const unsigned int* __restrict__ nnx,
                                                     const unsigned int* __restrict__ nny, int rows)
 {
+    chain_wait();
+    chain_trigger();
     extern __shared__ float2 down_h[];
     downsample_block(flow, U, V, sx, sy, sx_in, sy_in, taps, P, mx, my, nnx, nny, blockIdx.x * TX, blockIdx.y * rows,
                      rows, down_h);
 }
 // Small frames, and scales whose window does not fit shared memory.
-__global__ void __launch_bounds__(256) k_downsample_px(const uint32_t* __restrict__ flow, float* __restrict__ U,
+__global__ void __launch_bounds__(256) k_downsample_px(const uint32_t* flow, float* __restrict__ U,
                                                        float* __restrict__ V, int sx, int sy, int sx_in, int sy_in,
                                                        const float* __restrict__ taps, int P, float mx, float my,
                                                        const unsigned int* __restrict__ nnx,
                                                        const unsigned int* __restrict__ nny)
 {
+    chain_wait();
+    chain_trigger();
     const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
     if (x >= sx_in || y >= sy_in) return;
     downsample_px(flow, U, V, sx, sy, sx_in, taps, P, mx, my, nnx, nny, x, y);
 }
 
 // CUDA_convert, util_cuda.cu:174-183, for both components when no resampling is needed.
-__global__ void k_flow_to_planes(const uint32_t* __restrict__ flow, float* __restrict__ U, float* __restrict__ V,
-                                 size_t n)
+__global__ void k_flow_to_planes(const uint32_t* flow, float* __restrict__ U, float* __restrict__ V, size_t n)
 {
+    chain_wait();
+    chain_trigger();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint32_t f = flow[i];
@@ -437,11 +456,13 @@ __global__ void k_flow_to_planes(const uint32_t* __restrict__ flow, float* __res
 // 2t+1 (the reference's window runs over linear indices, so a pair may span a row
 // end).
 template <int FS>
-__global__ void __launch_bounds__(256) k_median_pass(const float* __restrict__ inU, const float* __restrict__ inV,
+__global__ void __launch_bounds__(256) k_median_pass(const float* inU, const float* inV,
                                                      float* __restrict__ outU, float* __restrict__ outV,
                                                      int dir, int fsize, int sx, int sy)
 {
     static_assert(FS % 2 == 1, "median register windows are odd");
+    chain_wait();
+    chain_trigger();
     const float* in = blockIdx.z ? inV : inU;
     float* out = blockIdx.z ? outV : outU;
     const long n = (long)sx * sy;
@@ -459,23 +480,27 @@ __global__ void __launch_bounds__(256) k_median_pass(const float* __restrict__ i
 template <int TY>
 __global__ void __launch_bounds__(TX * TY * TRI_G, 8 / TY) k_trilateral(const float* __restrict__ U,
                                                                        const float* __restrict__ V,
-                                                                       const float* __restrict__ Um,
-                                                                       const float* __restrict__ Vm,
+                                                                       const float* Um,
+                                                                       const float* Vm,
                                                                        const float* __restrict__ I,
                                                                        float* __restrict__ Uo, float* __restrict__ Vo,
                                                                        int sx, int sy, int s, float kE, float kI, float cS)
 {
+    chain_wait();
+    chain_trigger();
     extern __shared__ float4 smem4[];
     trilateral_block<TY>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, kE, kI, cS, blockIdx.x * TX, blockIdx.y * tri_rows(TY),
                          smem4);
 }
 
 __global__ void __launch_bounds__(256) k_trilateral_global(const float* __restrict__ U, const float* __restrict__ V,
-                                                           const float* __restrict__ Um, const float* __restrict__ Vm,
+                                                           const float* Um, const float* Vm,
                                                            const float* __restrict__ I, float* __restrict__ Uo,
                                                            float* __restrict__ Vo, int sx, int sy, int s,
                                                            float cE, float cI, float cS)
 {
+    chain_wait();
+    chain_trigger();
     const int x = blockIdx.x * TX + threadIdx.x, y = blockIdx.y * TY + threadIdx.y;
     if (x >= sx || y >= sy) return;
     const size_t o = (size_t)x + (size_t)y * sx;
@@ -533,6 +558,25 @@ __global__ void k_import_field(const int16_t* __restrict__ nx, const int16_t* __
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
+// Launch of a kernel that waits for its predecessor itself (chain_wait); `chained`: that
+// predecessor is the kernel launched last on the stream, and this one may start under its
+// last blocks.
+template <typename Kernel, typename... Args>
+static cudaError_t launch(Kernel kernel, dim3 grid, dim3 block, size_t smem, bool chained, cudaStream_t st, Args... args)
+{
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 cudaError_t lanczos_tables(float* w, int* idx, int n_in, int n_out, cudaStream_t st)
 {
     k_lanczos_tables<<<(n_out + 127) / 128, 128, 0, st>>>(w, idx, n_in, n_out);
@@ -553,12 +597,12 @@ cudaError_t upsample_u8(const uint8_t* in, float* out, int sxi, int syi, int sxo
     return cudaGetLastError();
 }
 
-cudaError_t upsample_u8_pad(const uint8_t* in, float* out, uint32_t* keys, int pitch, int m, int sxi, int syi, int sxo,
+cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_t* keys, int pitch, int m, int sxi, int syi, int sxo,
                             int syo, const float* lx, const int* ix, const float* ly, const int* iy, cudaStream_t st)
 {
     if (m < 0 || pitch < sxo + 2 * m) return cudaErrorInvalidValue;
     const dim3 g((sxo + 2 * m + TX - 1) / TX, (syo + 2 * m + TY * UP_R - 1) / (TY * UP_R));
-    k_upsample_pad_rows<<<g, dim3(TX, TY), 0, st>>>(in, out, keys, pitch, m, sxi, syi, sxo, syo, lx, ix, ly, iy);
+    k_upsample_pad_rows<<<g, dim3(TX, TY), 0, st>>>(in, frame, out, keys, pitch, m, sxi, syi, sxo, syo, lx, ix, ly, iy);
     return cudaGetLastError();
 }
 
@@ -599,71 +643,48 @@ void key_offsets(KeyOffsets& ko, const int4* pat, int N, int m, int pitch)
 }
 
 cudaError_t features_keys(const uint32_t* keys, const float* up, int pitch, uint32_t* F, int sx, int sy, int nsp,
-                          const KeyOffsets& ko, int rev, cudaStream_t st)
+                          const KeyOffsets& ko, int rev, bool chained, cudaStream_t st)
 {
     const dim3 g((sx + TX - 1) / TX, (sy + 2 * TY - 1) / (2 * TY));
-    BM_DISPATCH_NSP(nsp, (k_features_keys<NSP><<<g, dim3(TX, TY), 0, st>>>(keys, up, pitch, F, sx, sy, ko, rev)));
-    return cudaGetLastError();
-}
-
-// Launch of a TX x TY kernel that waits for its predecessor itself (chain_wait), on a
-// grid; `chained`: that predecessor is a kernel, and what it wrote is read after the wait.
-cudaLaunchConfig_t chain_config(dim3 grid, bool chained, cudaStream_t st)
-{
-    static cudaLaunchAttribute attr = [] {
-        cudaLaunchAttribute a = {};
-        a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        a.val.programmaticStreamSerializationAllowed = 1;
-        return a;
-    }();
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(TX, TY);
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = chained ? 1 : 0;
-    return cfg;
+    BM_DISPATCH_NSP(nsp, return launch(k_features_keys<NSP>, g, dim3(TX, TY), 0, chained, st, keys, up, pitch, F, sx, sy, ko, rev));
+    return cudaSuccess;
 }
 
 cudaError_t initialize(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_prev,
                        uint32_t* flow_out, uint16_t* cost, int sx, int sy, int nsp, int first, int rev,
-                       cudaStream_t st)
+                       bool chained, cudaStream_t st)
 {
-    BM_DISPATCH_NSP(nsp, k_initialize<NSP><<<grid2d(sx, sy), dim3(TX, TY), 0, st>>>(F1, F2, flow_prev, flow_out, cost, sx, sy, first, rev));
-    return cudaGetLastError();
+    BM_DISPATCH_NSP(nsp, return launch(k_initialize<NSP>, grid2d(sx, sy), dim3(TX, TY), 0, chained, st, F1, F2, flow_prev, flow_out, cost, sx, sy, first, rev));
+    return cudaSuccess;
 }
 
 cudaError_t seed_field(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_prev, uint32_t* flow_out,
                        uint16_t* cost, int sx, int sy, int nsp, int first, const float* pred, int w4, int h4,
-                       float scale_x, float scale_y, float logit_min, cudaStream_t st)
+                       float scale_x, float scale_y, float logit_min, bool chained, cudaStream_t st)
 {
     // host IEEE reciprocals: the device cell lookup multiplies by them
     const float inv_x = 1.0f / scale_x, inv_y = 1.0f / scale_y;
-    BM_DISPATCH_NSP(nsp, k_seed<NSP><<<grid2d(sx, sy), dim3(TX, TY), 0, st>>>(F1, F2, flow_prev, flow_out, cost, sx, sy, first, pred, w4, h4, scale_x, scale_y, inv_x, inv_y, logit_min));
-    return cudaGetLastError();
+    BM_DISPATCH_NSP(nsp, return launch(k_seed<NSP>, grid2d(sx, sy), dim3(TX, TY), 0, chained, st, F1, F2, flow_prev, flow_out, cost, sx, sy, first, pred, w4, h4, scale_x, scale_y, inv_x, inv_y, logit_min));
+    return cudaSuccess;
 }
 
 cudaError_t jump_level(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_in,
                        uint32_t* flow_out, uint16_t* cost, int sx, int sy, int nsp,
                        int p, int pd, int doubleProp, const RsArgs& rs, int rev, bool chained, cudaStream_t st)
 {
-    const cudaLaunchConfig_t cfg = chain_config(grid2d(sx, sy), chained, st);
-    cudaError_t e = cudaSuccess;
     if (rs.enabled) {
-        BM_DISPATCH_NSP(nsp, (e = cudaLaunchKernelEx(&cfg, k_jump_level<NSP, true>, F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, rev)));
+        BM_DISPATCH_NSP(nsp, return launch(k_jump_level<NSP, true>, grid2d(sx, sy), dim3(TX, TY), 0, chained, st, F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, rev));
     } else {
-        BM_DISPATCH_NSP(nsp, (e = cudaLaunchKernelEx(&cfg, k_jump_level<NSP, false>, F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, rev)));
+        BM_DISPATCH_NSP(nsp, return launch(k_jump_level<NSP, false>, grid2d(sx, sy), dim3(TX, TY), 0, chained, st, F1, F2, flow_in, flow_out, cost, sx, sy, p, pd, doubleProp, rs, rev));
     }
-    return e;
+    return cudaSuccess;
 }
 
 cudaError_t local_step(const uint32_t* F1, const uint32_t* F2, const uint32_t* flow_in, uint32_t* flow_out,
                        uint16_t* cost, int sx, int sy, int nsp, int r, int rev, bool chained, cudaStream_t st)
 {
-    const cudaLaunchConfig_t cfg = chain_config(grid2d(sx, sy), chained, st);
-    cudaError_t e = cudaSuccess;
-    BM_DISPATCH_NSP(nsp, (e = cudaLaunchKernelEx(&cfg, k_local_step<NSP>, F1, F2, flow_in, flow_out, cost, sx, sy, r, rev)));
-    return e;
+    BM_DISPATCH_NSP(nsp, return launch(k_local_step<NSP>, grid2d(sx, sy), dim3(TX, TY), 0, chained, st, F1, F2, flow_in, flow_out, cost, sx, sy, r, rev));
+    return cudaSuccess;
 }
 
 cudaError_t random_search(const uint32_t* F1, const uint32_t* F2, uint32_t* flow, uint16_t* cost,
@@ -695,51 +716,47 @@ static cudaError_t sm_count(int* sms)
 
 cudaError_t downsample(const uint32_t* flow, float* U, float* V, int sx, int sy, int sx_in, int sy_in,
                        const float* taps, int P, float mx, float my, const unsigned int* nnx,
-                       const unsigned int* nny, cudaStream_t st)
+                       const unsigned int* nny, bool chained, cudaStream_t st)
 {
     // By blocks of 32 rows, or as many as fit the 48 KB that need no opt-in, for windows
-    // of 11 taps and more (1920x1080 from u2.9 on) where those give every SM two blocks:
-    // 1920x1080 u4.9, 19 taps, 426 us per pixel, 184 by blocks.  With fewer taps a pass per
-    // pixel is as fast (1024x436 u2.9, 7 taps: 22.5 and 21.5; 584x388 u1.5, 3 taps: 8.2 and
-    // 8.8) and does not change the SMs' split between L1 and
-    // shared memory, which cost a batch of 12 pairs on several streams 1 %.
+    // of 16 taps and more where those give every SM two blocks: 1920x1080 u4.9, 19 taps,
+    // 426 us per pixel, 184 by blocks.  With few taps a pass per pixel is as fast
+    // (1024x436 u2.9, 7 taps: 22.5 and 21.5; 584x388 u1.5, 3 taps: 8.2 and 8.8), and it does
+    // not change the SMs' split between L1 and shared memory: blocks from 11 taps on made
+    // a batch of 12 pairs on several streams 0.8 % slower.
     int sms = 0;
     const cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) return e;
     int rows = 4 * TY;
     while (rows > TY && down_smem_bytes(rows, sy, sy_in, P) > DOWN_SMEM_MAX) rows /= 2;
     const size_t smem = down_smem_bytes(rows, sy, sy_in, P);
-    if (P < 11 || smem > DOWN_SMEM_MAX || (long)((sx_in + TX - 1) / TX) * ((sy_in + 4 * TY - 1) / (4 * TY)) < 2L * sms)
-        k_downsample_px<<<grid2d(sx_in, sy_in), dim3(TX, TY), 0, st>>>(flow, U, V, sx, sy, sx_in, sy_in, taps, P, mx, my,
-                                                                       nnx, nny);
-    else
-        k_downsample<<<dim3((sx_in + TX - 1) / TX, (sy_in + rows - 1) / rows), dim3(TX, TY), smem, st>>>(
-            flow, U, V, sx, sy, sx_in, sy_in, taps, P, mx, my, nnx, nny, rows);
-    return cudaGetLastError();
+    if (P < 16 || smem > DOWN_SMEM_MAX || (long)((sx_in + TX - 1) / TX) * ((sy_in + 4 * TY - 1) / (4 * TY)) < 2L * sms)
+        return launch(k_downsample_px, grid2d(sx_in, sy_in), dim3(TX, TY), 0, chained, st, flow, U, V, sx, sy, sx_in, sy_in,
+                      taps, P, mx, my, nnx, nny);
+    return launch(k_downsample, dim3((sx_in + TX - 1) / TX, (sy_in + rows - 1) / rows), dim3(TX, TY), smem, chained, st,
+                  flow, U, V, sx, sy, sx_in, sy_in, taps, P, mx, my, nnx, nny, rows);
 }
 
-cudaError_t flow_to_planes(const uint32_t* flow, float* U, float* V, size_t n, cudaStream_t st)
+cudaError_t flow_to_planes(const uint32_t* flow, float* U, float* V, size_t n, bool chained, cudaStream_t st)
 {
-    k_flow_to_planes<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(flow, U, V, n);
-    return cudaGetLastError();
+    return launch(k_flow_to_planes, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, chained, st, flow, U, V, n);
 }
 
 cudaError_t median_pass(const float* inU, const float* inV, float* outU, float* outV,
-                        int dir, int fsize, int sx, int sy, cudaStream_t st)
+                        int dir, int fsize, int sx, int sy, bool chained, cudaStream_t st)
 {
     const long n = (long)sx * sy;
     const dim3 g = dir ? dim3((unsigned)((n + 2 * TX * TY - 1) / (2 * TX * TY)), 1, 2)
                        : dim3((sx + TX - 1) / TX, (sy + 2 * TY - 1) / (2 * TY), 2);
-#define BM_MED(FSV) k_median_pass<FSV><<<g, dim3(TX, TY), 0, st>>>(inU, inV, outU, outV, dir, fsize, sx, sy)
+#define BM_MED(FSV) return launch(k_median_pass<FSV>, g, dim3(TX, TY), 0, chained, st, inU, inV, outU, outV, dir, fsize, sx, sy)
     if (fsize <= 9) BM_MED(9);
     else if (fsize <= 13) BM_MED(13);
     else if (fsize <= 15) BM_MED(15);
     else if (fsize <= 23) BM_MED(23);
     else if (fsize <= 31) BM_MED(31);
     else if (fsize <= BM_MAX_MEDIAN) BM_MED(BM_MAX_MEDIAN);
-    else return cudaErrorInvalidValue;
 #undef BM_MED
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 // The trilateral kernel's dynamic shared-memory opt-in, raised only when a larger
@@ -779,30 +796,29 @@ static int trilateral_rows(int sx, int sy, int s, int sms)
 
 cudaError_t trilateral(const float* U, const float* V, const float* Um, const float* Vm,
                        const float* I, float* Uo, float* Vo, int sx, int sy, int s,
-                       float sigmaEPE2, float sigmaI2, float sigmaS2, cudaStream_t st)
+                       float sigmaEPE2, float sigmaI2, float sigmaS2, bool chained, cudaStream_t st)
 {
     const TriCoef tc = tri_coef(sigmaEPE2, sigmaI2, sigmaS2);
     const float cE = tc.cE, cI = tc.cI, cS = tc.cS;
     if (s <= TRI_MAX_S) {
         cudaError_t e = ensure_trilateral_smem(s);
         if (e != cudaSuccess) return e;
-        auto launch = [&](auto kernel, int ty) {
+        auto by_rows = [&](auto kernel, int ty) {
             dim3 g((sx + TX - 1) / TX, (sy + tri_rows(ty) - 1) / tri_rows(ty));
-            kernel<<<g, dim3(TX, ty, TRI_G), tri_smem_bytes(s, ty), st>>>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, tc.kE, tc.kI,
-                                                                         cS);
+            return launch(kernel, g, dim3(TX, ty, TRI_G), tri_smem_bytes(s, ty), chained, st, U, V, Um, Vm, I, Uo, Vo, sx, sy,
+                          s, tc.kE, tc.kI, cS);
         };
         int sms = 0;
         e = sm_count(&sms);
         if (e != cudaSuccess) return e;
         switch (trilateral_rows(sx, sy, s, sms)) {
-        case 2: launch(k_trilateral<2>, 2); break;
-        case 4: launch(k_trilateral<4>, 4); break;
-        default: launch(k_trilateral<8>, 8); break;
+        case 2: return by_rows(k_trilateral<2>, 2);
+        case 4: return by_rows(k_trilateral<4>, 4);
+        default: return by_rows(k_trilateral<8>, 8);
         }
-    } else {
-        k_trilateral_global<<<grid2d(sx, sy), dim3(TX, TY), 0, st>>>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, cE, cI, cS);
     }
-    return cudaGetLastError();
+    return launch(k_trilateral_global, grid2d(sx, sy), dim3(TX, TY), 0, chained, st, U, V, Um, Vm, I, Uo, Vo, sx, sy, s, cE,
+                  cI, cS);
 }
 
 cudaError_t export_field(const uint32_t* flow, const uint16_t* cost, int16_t* nx, int16_t* ny,

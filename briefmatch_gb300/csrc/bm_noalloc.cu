@@ -151,10 +151,10 @@ bm_status bm_refine_noalloc(const float* d_u, const float* d_v, const float* d_g
     const int fs = fsize == 0 ? 1 : (int)fsize;
     const int w = (int)width, h = (int)height;
     // Every scratch element is written before it is read, so nothing is cleared.
-    cudaError_t e = bmk::median_pass(d_u, d_v, hU, hV, 1, fs, w, h, s);
-    if (e == cudaSuccess) e = bmk::median_pass(hU, hV, mU, mV, 0, fs, w, h, s);
+    cudaError_t e = bmk::median_pass(d_u, d_v, hU, hV, 1, fs, w, h, false, s);
+    if (e == cudaSuccess) e = bmk::median_pass(hU, hV, mU, mV, 0, fs, w, h, false, s);
     if (e == cudaSuccess)
-        e = bmk::trilateral(d_u, d_v, mU, mV, d_guide, d_uo, d_vo, w, h, tri_s, sEPE * sEPE, sI * sI, sS * sS, s);
+        e = bmk::trilateral(d_u, d_v, mU, mV, d_guide, d_uo, d_vo, w, h, tri_s, sEPE * sEPE, sI * sI, sS * sS, false, s);
     if (e != cudaSuccess) {
         char buf[256];
         std::snprintf(buf, sizeof(buf), "bm_refine_noalloc: launch failed: %s", cudaGetErrorString(e));

@@ -17,7 +17,7 @@ if not torch.cuda.is_available():
     pytest.skip("no GPU", allow_module_level=True)
 
 
-@pytest.mark.parametrize("W,H,u", [(1025, 310, 5.6), (1024, 311, 11.0), (1030, 321, 4.1), (97, 61, 4.9), (33, 20, 24.0),
+@pytest.mark.parametrize("W,H,u", [(1700, 620, 5.6), (1024, 311, 11.0), (1030, 321, 4.1), (97, 61, 4.9), (33, 20, 24.0),
                                    (5, 3, 2.0)])
 def test_downsample_blocks(W, H, u):
     prm = small_params(W, H, u, u, N=32)
