@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256) k_upsample(const T* __restrict__ in, floa
 // the threads write the frame itself as float into `frame` (if any), for the refinement:
 // 2 us at 1024x436 where a launch of its own took 4 to 6.  (Extra blocks for it: as fast
 // on large frames, 4 us slower on small ones.)
-constexpr int UP_R = 8;
+template <int UP_R>
 __global__ void __launch_bounds__(TX * TY) k_upsample_pad_rows(const uint8_t* __restrict__ in, float* __restrict__ frame,
                                                                float* __restrict__ out,
                                                                uint32_t* __restrict__ keys, int pitch, int m, int sxi,
@@ -558,6 +558,14 @@ __global__ void k_import_field(const int16_t* __restrict__ nx, const int16_t* __
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
+// SMs of the current device.
+static cudaError_t sm_count(int* sms)
+{
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    return e == cudaSuccess ? cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) : e;
+}
+
 // Launch of a kernel that waits for its predecessor itself (chain_wait); `chained`: that
 // predecessor is the kernel launched last on the stream, and this one may start under its
 // last blocks.
@@ -601,8 +609,22 @@ cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_
                             int syo, const float* lx, const int* ix, const float* ly, const int* iy, cudaStream_t st)
 {
     if (m < 0 || pitch < sxo + 2 * m) return cudaErrorInvalidValue;
-    const dim3 g((sxo + 2 * m + TX - 1) / TX, (syo + 2 * m + TY * UP_R - 1) / (TY * UP_R));
-    k_upsample_pad_rows<<<g, dim3(TX, TY), 0, st>>>(in, frame, out, keys, pitch, m, sxi, syi, sxo, syo, lx, ix, ly, iy);
+    // Eight rows a thread share the most products; a grid of fewer blocks than SMs takes
+    // fewer rows a thread and with them less time for its chain of rows (96x64 u1.5: 11.4
+    // us with eight, 8.8, 8.0 and 6.9 with four, two and one; 1024x436 u2.9 47.6, 46.0,
+    // 56.7 and 76.3, 1920x1080 u4.9 434, 490, 622 and 913).
+    int sms = 0;
+    const cudaError_t e = sm_count(&sms);
+    if (e != cudaSuccess) return e;
+    auto rows = [&](auto kernel, int r) {
+        const dim3 g((sxo + 2 * m + TX - 1) / TX, (syo + 2 * m + TY * r - 1) / (TY * r));
+        kernel<<<g, dim3(TX, TY), 0, st>>>(in, frame, out, keys, pitch, m, sxi, syi, sxo, syo, lx, ix, ly, iy);
+    };
+    const long columns = (sxo + 2 * m + TX - 1) / TX, eights = (syo + 2 * m + TY - 1) / TY;
+    if (columns * eights >= 8L * sms) rows(k_upsample_pad_rows<8>, 8);
+    else if (columns * eights >= 4L * sms) rows(k_upsample_pad_rows<4>, 4);
+    else if (columns * eights >= 2L * sms) rows(k_upsample_pad_rows<2>, 2);
+    else rows(k_upsample_pad_rows<1>, 1);
     return cudaGetLastError();
 }
 
@@ -704,14 +726,6 @@ cudaError_t nn_table(unsigned int* idx, int n_up, int n_in, cudaStream_t st)
 {
     k_nn_table<<<(n_in + 127) / 128, 128, 0, st>>>(idx, n_up, n_in);
     return cudaGetLastError();
-}
-
-// SMs of the current device.
-static cudaError_t sm_count(int* sms)
-{
-    int dev = 0;
-    const cudaError_t e = cudaGetDevice(&dev);
-    return e == cudaSuccess ? cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) : e;
 }
 
 cudaError_t downsample(const uint32_t* flow, float* U, float* V, int sx, int sy, int sx_in, int sy_in,
