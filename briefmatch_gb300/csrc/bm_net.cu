@@ -545,15 +545,17 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
         ::"r"(s_addr(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(s_addr(bar))
         : "memory");
 }
-// Shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups 512 B apart.
+// Shared-memory matrix descriptor: K-major, rows of KC channels swizzled by their width
+// (64 or 32 bytes), 8-row groups 8 rows apart.
+template <int KC = 32>
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr)
 {
     uint64_t d = 0;
     d |= (uint64_t)((saddr >> 4) & 0x3FFF);       // start address
     d |= (uint64_t)1 << 16;                       // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(512 >> 4) << 32;              // stride byte offset: next 8-row group
+    d |= (uint64_t)(KC * 2 * 8 >> 4) << 32;       // stride byte offset: next 8-row group
     d |= (uint64_t)1 << 46;                       // descriptor version (sm_100 family)
-    d |= (uint64_t)4 << 61;                       // swizzle mode: 64-byte
+    d |= (uint64_t)(KC == 32 ? 4 : 6) << 61;      // swizzle mode: 64- or 32-byte
     return d;
 }
 // Instruction descriptor of kind::f16: BF16 A and B (K-major), FP32 D, M x N.
@@ -607,7 +609,7 @@ constexpr uint32_t CV_ROW = (UM + 16) * 64;      // a source row's cells, dilati
 constexpr uint32_t CV_STAGE = 3 * CV_ROW;
 constexpr size_t conv_umma_smem(int n) { return 1024 + CV_STAGES * (size_t)CV_STAGE + 9 * (size_t)n * 64; }
 
-template <int EPI, int N>
+template <int EPI, int N, int KC = 32>
 __global__ void __launch_bounds__(CV_THREADS) k_conv_umma(const __grid_constant__ CUtensorMap tmX,
                                                           const __grid_constant__ CUtensorMap tmW,
                                                           const float* __restrict__ bias,
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(CV_THREADS) k_conv_umma(const __grid_constant_
                                                           int h, int w, int rows, int dil, int cout_real, int out_stride,
                                                           int chained, int* __restrict__ err)
 {
-    static_assert(N == 16 || N == 32, "N is 16 or 32 output channels");
+    static_assert((N == 16 || N == 32) && (KC == 16 || KC == 32), "16 or 32 channels out and in");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* sB = sm + CV_STAGES * CV_STAGE;   // 9 taps x N rows x 64 B
@@ -658,7 +660,7 @@ __global__ void __launch_bounds__(CV_THREADS) k_conv_umma(const __grid_constant_
     if (warp == 4) {
         if (lane == 0) {   // copies
             auto weights = [&]() {
-                mbar_expect_tx(&bar_w, 9u * N * 64);
+                mbar_expect_tx(&bar_w, 9u * N * KC * 2);
                 tma_load_3d(sB, &tmW, 0, 0, 0, &bar_w);
             };
             if (chained) weights();
@@ -674,7 +676,7 @@ __global__ void __launch_bounds__(CV_THREADS) k_conv_umma(const __grid_constant_
                 const int y = row % h;
                 uint32_t bytes = 0;
                 for (int v = -1; v <= 1; v++)
-                    if (y + v * dil >= 0 && y + v * dil < h) bytes += (uint32_t)(UM + 2 * dil) * 64;
+                    if (y + v * dil >= 0 && y + v * dil < h) bytes += (uint32_t)(UM + 2 * dil) * KC * 2;
                 mbar_expect_tx(&full[st], bytes);
                 for (int v = -1; v <= 1; v++)
                     if (y + v * dil >= 0 && y + v * dil < h)
@@ -707,9 +709,9 @@ __global__ void __launch_bounds__(CV_THREADS) k_conv_umma(const __grid_constant_
 #pragma unroll
                     for (int u = 0; u < 3; u++) {
 #pragma unroll
-                        for (int kh = 0; kh < 2; kh++) {  // K = 16 channels (32 bytes) per MMA
-                            const uint64_t ad = umma_desc(a0 + v * CV_ROW + u * dil * 64 + kh * 32);
-                            const uint64_t bd = umma_desc(b0 + (v * 3 + u) * N * 64 + kh * 32);
+                        for (int kh = 0; kh < KC / 16; kh++) {  // K = 16 channels (32 bytes) per MMA
+                            const uint64_t ad = umma_desc<KC>(a0 + v * CV_ROW + u * dil * KC * 2 + kh * 32);
+                            const uint64_t bd = umma_desc<KC>(b0 + (v * 3 + u) * N * KC * 2 + kh * 32);
                             asm volatile(
                                 "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
                                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
@@ -1051,8 +1053,11 @@ bool act_map(CUtensorMap* map, const __nv_bfloat16* X, int B, int h, int w)
 {
     return encode_map(map, X, (uint64_t)w, (uint64_t)B * h, UM, 1);
 }
-// Weights [9][n][32] as the B operand (all nine taps in one copy).
-bool weight_map(CUtensorMap* map, const __nv_bfloat16* W, int n) { return encode_map(map, W, (uint64_t)n, 9, n, 9); }
+// Weights [9][n][nch] as the B operand (all nine taps in one copy).
+bool weight_map(CUtensorMap* map, const __nv_bfloat16* W, int n, int nch = 32)
+{
+    return encode_map(map, W, (uint64_t)n, 9, n, 9, nch);
+}
 
 // Activations [B*h][w][nch] as a layer's source rows: UM cells and a dilation's more on
 // either side.
@@ -1061,7 +1066,7 @@ bool row_map(CUtensorMap* map, const __nv_bfloat16* X, int B, int h, int w, int 
     return encode_map(map, X, (uint64_t)w, (uint64_t)B * h, (uint32_t)(UM + 2 * dil), 1, nch);
 }
 
-template <int EPI, int N>
+template <int EPI, int N, int KC = 32>
 cudaError_t launch_conv_umma(const CUtensorMap& mx, const CUtensorMap& mw, const float* bias, const __nv_bfloat16* act,
                              void* out, int B, int h, int w, int dil, int cout_real, int out_stride, int sms,
                              bool chained, int* err, cudaStream_t st)
@@ -1077,7 +1082,7 @@ cudaError_t launch_conv_umma(const CUtensorMap& mx, const CUtensorMap& mw, const
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = chained ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_conv_umma<EPI, N>, mx, mw, bias, act, out, h, w, B * h, dil, cout_real, out_stride,
+    return cudaLaunchKernelEx(&cfg, k_conv_umma<EPI, N, KC>, mx, mw, bias, act, out, h, w, B * h, dil, cout_real, out_stride,
                               chained ? 1 : 0, err);
 }
 
@@ -1231,7 +1236,7 @@ __global__ void __launch_bounds__(128) k_net_fused(const __grid_constant__ NetFu
                         const uint32_t a0 = s_addr(sA + t * U_TAP_A), b0 = s_addr(sB + t * n * 64);
 #pragma unroll
                         for (int kh = 0; kh < 2; kh++) {
-                            const uint64_t ad = umma_desc(a0 + kh * 32), bd = umma_desc(b0 + kh * 32);
+                            const uint64_t ad = umma_desc<>(a0 + kh * 32), bd = umma_desc<>(b0 + kh * 32);
                             asm volatile(
                                 "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
                                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
@@ -1316,6 +1321,7 @@ cudaError_t conv_smem_optin()
         set((const void*)k_conv_wgrad<32, 32, 8>, wgrad_smem(32, 32, 8)),
         set((const void*)k_conv_umma<EPI_RELU_BF16, 32>, conv_umma_smem(32)),
         set((const void*)k_conv_umma<EPI_MASK_BF16, 32>, conv_umma_smem(32)),
+        set((const void*)k_conv_umma<EPI_MASK_BF16, 32, 16>, conv_umma_smem(32)),
         set((const void*)k_conv_umma<EPI_LINEAR_F32, 16>, conv_umma_smem(16)),
         set((const void*)k_net_fused, umma_smem(32)),
         set((const void*)k_wgrad_umma<32>, WG_SMEM),
@@ -1582,7 +1588,7 @@ bm_status bm_net_create(uint32_t max_batch, uint32_t max_h4, uint32_t max_w4, bm
     // the tcgen05 path, when the driver encodes the weights' tensor maps
     n->umma = true;
     for (int l = 0; n->umma && l < NL; l++) n->umma = weight_map(&n->map_wf[l], n->d_wf[l], COUT_P[l]);
-    for (int l = 1; n->umma && l < NL - 1; l++) n->umma = weight_map(&n->map_wb[l], n->d_wb[l], CIN_P[l]);
+    for (int l = 1; n->umma && l < NL; l++) n->umma = weight_map(&n->map_wb[l], n->d_wb[l], CIN_P[l], COUT_P[l]);
     {
         // co-resident CTAs of the fused launch (mode 2); the per-layer launches (mode 1)
         // measured faster and are the default
@@ -1742,7 +1748,7 @@ bm_status bm_net_set_umma(bm_net* n, int mode)
         return nfail(BM_ERR_CUDA, "bm_net_set_umma: no cooperative launch of the fused network on this device");
     bool ok = true;
     for (int l = 0; ok && l < NL; l++) ok = weight_map(&n->map_wf[l], n->d_wf[l], COUT_P[l]);
-    for (int l = 1; ok && l < NL - 1; l++) ok = weight_map(&n->map_wb[l], n->d_wb[l], CIN_P[l]);
+    for (int l = 1; ok && l < NL; l++) ok = weight_map(&n->map_wb[l], n->d_wb[l], CIN_P[l], COUT_P[l]);
     if (!ok) return nfail(BM_ERR_CUDA, "bm_net_set_umma: tensor map encoding unavailable");
     n->umma = true;
     n->fused = mode == 2;
@@ -1806,8 +1812,12 @@ bm_status bm_net_train_step(bm_net* n, uint32_t B, uint32_t h, uint32_t w, const
     float* g = n->d_grad;
     s = weight_grad(n, 5, 0, Bi, hi, wi, st);
     if (s != BM_OK) return s;
-    BN_CUDA((launch_conv<16, 32, EPI_MASK_BF16, 1>(n->d_dy[0], n->d_wb[5], nullptr, n->d_act[4], n->d_dy[1], Bi, hi, wi,
-                                                   32, 32, st)));
+    if (n->umma)
+        BN_CUDA((launch_conv_umma<EPI_MASK_BF16, 32, 16>(n->map_dy[5], n->map_wb[5], nullptr, n->d_act[4], n->d_dy[1], Bi, hi,
+                                                         wi, DIL[5], 32, 32, n->num_sms, false, n->d_err, st)));
+    else
+        BN_CUDA((launch_conv<16, 32, EPI_MASK_BF16, 1>(n->d_dy[0], n->d_wb[5], nullptr, n->d_act[4], n->d_dy[1], Bi, hi, wi,
+                                                       32, 32, st)));
     int cur = 1;
     for (int l = 4; l >= 1; l--) {
         s = weight_grad(n, l, cur, Bi, hi, wi, st);
