@@ -9,19 +9,17 @@
 // Every layer is a 3x3 convolution; the dilated middle layers widen the receptive
 // field to 63 cells (252 pixels) at the same cost per layer.
 //
-// Weights and activations are BF16, accumulation FP32, on the tensor cores.  The
-// forward pass of every layer and the backward-data pass of the 32-channel layers run
-// on the fifth-generation tensor cores (k_conv_umma): per CTA 128 cells of one image
-// row are the GEMM's M, the nine taps' 32 input channels its K (two K=16 steps per
-// tap), the output channels its N; TMA brings each tap's 128x32 activation tile and
-// the weights into shared memory in the 64-byte-swizzled K-major layout the MMA
-// reads, tcgen05.mma accumulates in tensor memory and tcgen05.ld hands each thread
-// its cell's channels for the epilogue.  The mma.sync m16n8k16 kernels (k_conv) stay
-// for the backward-data pass of the head (16 gradient channels), as the alternative
-// forward path (bm_net_set_umma), and the weight gradients (k_conv_wgrad: pixels as
-// the reduction dimension).  Activations are NHWC with the channel count padded to a
-// multiple of 16 (32-byte rows).  Training keeps FP32 master weights and Adam
-// moments; every step repacks the BF16 copies the kernels read.
+// Weights and activations are BF16, accumulation FP32, on the tensor cores.  Forward,
+// backward-data and weight gradients of every layer run on the fifth-generation tensor
+// cores: TMA brings image rows and weights into shared memory in the swizzled layouts the
+// MMAs read, tcgen05.mma accumulates in tensor memory and tcgen05.ld hands the sums to
+// the epilogue.  In k_conv_umma 128 cells of one image row are the GEMM's M, the nine
+// taps' input channels its K, the output channels its N; in k_wgrad_umma the cells are
+// the reduction, the output gradient's three shifts M and three input rows N.  The
+// mma.sync m16n8k16 kernels (k_conv, k_conv_wgrad) stay as the alternative path
+// (bm_net_set_umma).  Activations are NHWC with the channel count padded to a multiple of
+// 16 (32-byte rows).  Training keeps FP32 master weights and Adam moments; every step
+// repacks the BF16 copies the kernels read.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -602,8 +600,10 @@ __device__ __forceinline__ void umma_load(uint32_t (&r)[N], uint32_t taddr)
 // the wait, so whatever ran before that layer -- the packing of the weights -- is
 // complete when this one starts.
 //
-// 32 images of 128 x 96 cells, 32 -> 32 channels: 45.5 us with one CTA per tile and nine
-// copies, one layer of one 256 x 109 image 7.6 us.
+// What bounds a layer of many cells is the MMAs' reading of the 128 x 16 operand (about
+// 64 cycles each, 18 a tile); a layer of one image is latency.  32 images of 128 x 96
+// cells, 32 -> 32 channels: 45.5 us with one CTA per tile and nine copies, now 19 (21 with
+// the ReLU mask); the six layers and the input of one 256 x 109 image 59 -> 46 us.
 constexpr int CV_STAGES = 3, CV_THREADS = 192;
 constexpr uint32_t CV_ROW = (UM + 16) * 64;      // a source row's cells, dilation up to 8
 constexpr uint32_t CV_STAGE = 3 * CV_ROW;
@@ -810,7 +810,8 @@ __global__ void __launch_bounds__(CV_THREADS) k_conv_umma(const __grid_constant_
 // What bounds an MMA here is reading its M x 16 operand (about 90 cycles, whatever N is):
 // dY is that operand, and the taps go into N.  Per layer of 32 images of 128 x 96 cells:
 // mma.sync tiles with transposed shared-memory staging 133 us (dilation 1) to 233 us
-// (dilation 8); X as the M operand, three MMAs per 16 cells, 31 us; now 22 us (24 us with scalar adds at the end).
+// (dilation 8); X as the M operand, three MMAs per 16 cells, 31 us; now 22 us (25 us
+// with scalar adds at the end).
 // ---------------------------------------------------------------------------
 constexpr int WG_STAGES = 4;
 constexpr uint32_t WG_DY = 10240, WG_STAGE = WG_DY + 3 * U_TAP_A;   // dY, then three rows of X

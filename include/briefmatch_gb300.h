@@ -347,8 +347,8 @@ bm_status bm_net_train_step(bm_net* n, uint32_t B, uint32_t h, uint32_t w, const
 bm_status bm_net_snapshot(bm_net* n, uint32_t slot, void* stream);
 bm_status bm_net_restore(bm_net* n, uint32_t slot, void* stream);
 /* Which tensor-core path the convolutions take.  mode 1 (the default where the driver
- * encodes tensor maps): every layer of the forward pass, and the backward-data pass of
- * the 32-channel layers, is a launch of tcgen05 MMAs into tensor memory fed by TMA;
+ * encodes tensor maps): every layer of the forward pass, of the backward-data pass and
+ * of the weight gradients is a launch of tcgen05 MMAs into tensor memory fed by TMA;
  * mode 2: the six forward layers in one cooperative launch of the same MMAs with a
  * grid barrier between layers (measured slower than mode 1 at 1024x436: the barrier
  * costs more than the launches it saves); mode 0: mma.sync m16n8k16 kernels.  All
