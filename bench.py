@@ -247,7 +247,8 @@ def algorithmic_bytes(kernel, prm):
         # up-sampled image read once, descriptors written once
         "features": n * (4 + ns * 4),
         "initialize": n * (2 * ns * 4 + 4 + 2),
-        "upsample_u8": ni + n * 4,
+        # frame read; image, key image and the frame as float written
+        "upsample_u8": ni + n * (4 + 4) + ni * 4,
         # five float planes read, two written
         "trilateral": ni * 7 * 4,
         "median_pass": ni * 2 * 2 * 4,
