@@ -53,6 +53,11 @@ bm_status fail(bm_status st, const char* fmt, ...)
 
 void bmk::set_error_text(const char* msg) { g_last_error = msg ? msg : ""; }
 
+// Largest output of both planes that goes to the host through a pinned buffer: a pair of
+// 96x64 frames (48 KB) took 135 us with two copies to pageable memory, 120 with one to the
+// pinned buffer; 160x120 (150 KB) 146 and 145, 320x240 (600 KB) 209 and 260.
+constexpr size_t STAGE_MAX = 96 * 1024;
+
 struct bm_ctx {
     bm_params prm;
     uint32_t nsp = 1;
@@ -96,6 +101,7 @@ struct bm_ctx {
     cudaEvent_t ev_refined = nullptr;             // refine stream: last refinement and copies done
     float* d_flow_med = nullptr;
     float* d_flow_out = nullptr;
+    float* h_stage = nullptr;   // pinned copy of d_flow_out for host outputs of small frames (copy_out)
     float* d_tmp = nullptr;
     int4* d_pattern = nullptr;
     int pattern_rmax = 0;
@@ -224,6 +230,8 @@ bm_status dev_alloc(T** p, size_t count)
 
 void release(bm_ctx* c)
 {
+    if (c->h_stage) cudaFreeHost(c->h_stage);
+    c->h_stage = nullptr;
     void* ptrs[] = {c->d_u8[0], c->d_u8[1], c->d_u8[2], c->d_pred, c->d_frame[0], c->d_frame[1], c->d_frame[2], c->d_up, c->d_upad,
                     c->d_feat[0], c->d_feat[1], c->d_flow[0], c->d_flow[1], c->d_cost, c->d_flow_in_buf[0],
                     c->d_flow_in_buf[1], c->d_flow_med, c->d_flow_out,
@@ -547,6 +555,11 @@ bm_status bm_create(const bm_params* prm, bm_ctx** out)
     c->d_flow_in = c->d_flow_in_buf[0];
     BM_TRY(dev_alloc(&c->d_flow_med, 2 * ni));
     BM_TRY(dev_alloc(&c->d_flow_out, 2 * ni));
+    if (2 * ni * sizeof(float) <= STAGE_MAX &&
+        cudaMallocHost((void**)&c->h_stage, 2 * ni * sizeof(float)) != cudaSuccess) {
+        c->h_stage = nullptr;   // the planes are then copied directly
+        cudaGetLastError();
+    }
     BM_TRY(dev_alloc(&c->d_tmp, 2 * ni));
     BM_TRY(dev_alloc(&c->d_pattern, BM_PATCH_MAX / 4));
     BM_TRY(dev_alloc(&c->d_taps, BM_CONST_KERNEL_SIZE));
@@ -815,16 +828,39 @@ bm_status bm_swap(bm_ctx* c)
     return BM_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// The refined flow into host memory, and a wait for it.  Small frames go through a pinned
+// buffer: one copy of both planes, then host copies, instead of two copies to pageable
+// memory that each wait for the device (STAGE_MAX).
+bm_status copy_out(bm_ctx* c, float* h_u, float* h_v)
+{
+    const size_t b = c->npix_in * sizeof(float);
+    if (c->h_stage && h_u && h_v) {
+        BM_CUDA(cudaMemcpyAsync(c->h_stage, c->d_flow_out, 2 * b, cudaMemcpyDeviceToHost, c->stream));
+        BM_CUDA(cudaStreamSynchronize(c->stream));
+        std::memcpy(h_u, c->h_stage, b);
+        std::memcpy(h_v, c->h_stage + c->npix_in, b);
+        return BM_OK;
+    }
+    if (h_u) BM_CUDA(cudaMemcpyAsync(h_u, c->d_flow_out, b, cudaMemcpyDeviceToHost, c->stream));
+    if (h_v) BM_CUDA(cudaMemcpyAsync(h_v, c->d_flow_out + c->npix_in, b, cudaMemcpyDeviceToHost, c->stream));
+    BM_CUDA(cudaStreamSynchronize(c->stream));
+    return BM_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 bm_status bm_convert(bm_ctx* c, float* h_u, float* h_v)
 {
     if (check_ctx(c)) return BM_ERR_INVALID;
     if (!h_u || !h_v) return fail(BM_ERR_INVALID, "bm_convert: null output");
     BM_CUDA(join_refine(c));
-    const size_t b = c->npix_in * sizeof(float);
-    BM_CUDA(cudaMemcpyAsync(h_u, c->d_flow_out, b, cudaMemcpyDeviceToHost, c->stream));
-    BM_CUDA(cudaMemcpyAsync(h_v, c->d_flow_out + c->npix_in, b, cudaMemcpyDeviceToHost, c->stream));
-    BM_CUDA(cudaStreamSynchronize(c->stream));
-    return BM_OK;
+    return copy_out(c, h_u, h_v);
 }
 
 bm_status bm_colors(bm_ctx* c, uint8_t* rgb, int rgb_on_device)
@@ -1132,11 +1168,13 @@ bm_status bm_frame(bm_ctx* c, const uint8_t* frame, int frame_on_device, float* 
     c->cur_frame = (c->cur_frame + 1) % 3;
     c->feat1 ^= 1;
     const cudaStream_t out_stream = refine_async ? c->refine_stream : c->stream;
-    if (u || v) {
+    if ((u || v) && !out_on_device && !c->pipelined) {
+        st = copy_out(c, u, v);
+        if (st != BM_OK) return st;
+    } else if (u || v) {
         const cudaMemcpyKind kind = out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
         if (u) BM_CUDA(cudaMemcpyAsync(u, c->d_flow_out, ni * sizeof(float), kind, out_stream));
         if (v) BM_CUDA(cudaMemcpyAsync(v, c->d_flow_out + ni, ni * sizeof(float), kind, out_stream));
-        if (!out_on_device && !c->pipelined) BM_CUDA(cudaStreamSynchronize(c->stream));
     }
     if (refine_async) BM_CUDA(cudaEventRecord(c->ev_refined, c->refine_stream));
     return BM_OK;
