@@ -75,13 +75,18 @@ __global__ void __launch_bounds__(256) k_upsample(const T* __restrict__ in, floa
 // the nearest image pixel (each coordinate clamped), computed by the same Lanczos
 // expression, so every read of the margin equals a clamped read of the image.
 // Each thread computes UP_R output rows of one column (a block covers
-// TX x (TY * UP_R) outputs).  The rows share the column's six
-// weights and source columns, and rows whose Lanczos windows start on the same
-// source row share the products input * Lx: they are formed once per window (36
-// multiplies) and each output then takes its 36 multiply-adds onto them in the
-// reference's order (util_cuda.cu:140-152: over source columns, then rows;
-// v += (in * Lx) * Ly as one rounded product and an FMA, w += Lx * Ly as an FMA), so
-// every value equals upsample_val's bit for bit.
+// TX x (TY * UP_R) outputs).  The rows share the column's six weights and source
+// columns and the products input * Lx: those of the first row's Lanczos window are formed
+// once (36 multiplies), and a window one source row further on moves them by a row and
+// forms six more.  Each output takes its 36 multiply-adds onto them in the reference's
+// order (util_cuda.cu:140-152: over source columns, then rows; v += (in * Lx) * Ly as one
+// rounded product and an FMA, w += Lx * Ly as an FMA), so every value equals
+// upsample_val's bit for bit.
+//
+// The rows' sums are kept and divided, keyed and stored together after the last row: with
+// that the loads of later rows run ahead, and two blocks per SM at 121 registers take
+// 39.5 us at 1024x436 u2.9 where three at 79 with a division per row took 47.6 (1920x1080
+// u4.9 434 -> 393, 320x240 u2.9 14.8 -> 12.7; three blocks spill: 41.7 and 387).
 //
 // Beside the float image the kernel writes the key image the descriptors read: a word
 // per pixel with the 16-bit key (sample_key) of the pixel in its low half and of the
@@ -91,7 +96,7 @@ __global__ void __launch_bounds__(256) k_upsample(const T* __restrict__ in, floa
 // 2 us at 1024x436 where a launch of its own took 4 to 6.  (Extra blocks for it: as fast
 // on large frames, 4 us slower on small ones.)
 template <int UP_R>
-__global__ void __launch_bounds__(TX * TY) k_upsample_pad_rows(const uint8_t* __restrict__ in, float* __restrict__ frame,
+__global__ void __launch_bounds__(TX * TY, 2) k_upsample_pad_rows(const uint8_t* __restrict__ in, float* __restrict__ frame,
                                                                float* __restrict__ out,
                                                                uint32_t* __restrict__ keys, int pitch, int m, int sxi,
                                                                int syi, int sxo, int syo,
@@ -108,44 +113,53 @@ __global__ void __launch_bounds__(TX * TY) k_upsample_pad_rows(const uint8_t* __
     }
     if (X >= sxo + 2 * m || Y0 >= syo + 2 * m) return;
     const int x = min(sxo - 1, max(0, X - m));
+    const int x1 = __ldg(ix + x);
     float Lx[6];
     int col[6];
-    const int x1 = __ldg(ix + x);
 #pragma unroll
     for (int a = 0; a < 6; a++) {
         Lx[a] = __ldg(lx + x * 6 + a);
         col[a] = min(sxi - 1, max(0, x1 - 2 + a));
     }
     float P[6][6];  // P[a][b] = in[row b of the window][col a] * Lx[a]
-    int win = INT_MIN;
+    auto products = [&](int win, int b) {
+        const uint8_t* src = in + (size_t)min(syi - 1, max(0, win - 2 + b)) * sxi;
+#pragma unroll
+        for (int a = 0; a < 6; a++) P[a][b] = __fmul_rn((float)__ldg(src + col[a]), Lx[a]);
+    };
+    int win = __ldg(iy + min(syo - 1, max(0, Y0 - m)));   // uniform across the warp
+#pragma unroll
+    for (int b = 0; b < 6; b++) products(win, b);
+    float v[UP_R], w[UP_R];
+#pragma unroll
+    for (int r = 0; r < UP_R; r++) {
+        const int y = min(syo - 1, max(0, Y0 + r - m));
+        for (const int y1 = __ldg(iy + y); win < y1;) {   // windows only move down
+            win++;
+#pragma unroll
+            for (int a = 0; a < 6; a++)
+#pragma unroll
+                for (int b = 0; b < 5; b++) P[a][b] = P[a][b + 1];
+            products(win, 5);
+        }
+        float Ly[6];
+#pragma unroll
+        for (int b = 0; b < 6; b++) Ly[b] = __ldg(ly + y * 6 + b);
+        v[r] = w[r] = 0.0f;
+#pragma unroll
+        for (int a = 0; a < 6; a++)
+#pragma unroll
+            for (int b = 0; b < 6; b++) {
+                w[r] = __fmaf_rn(Lx[a], Ly[b], w[r]);
+                v[r] = __fmaf_rn(P[a][b], Ly[b], v[r]);
+            }
+    }
     uint32_t key_above = 0;
 #pragma unroll
     for (int r = 0; r < UP_R; r++) {
         const int Y = Y0 + r;
         if (Y >= syo + 2 * m) break;
-        const int y = min(syo - 1, max(0, Y - m));
-        const int y1 = __ldg(iy + y);
-        if (y1 != win) {  // uniform across the warp (one output row per warp)
-            win = y1;
-#pragma unroll
-            for (int b = 0; b < 6; b++) {
-                const uint8_t* src = in + (size_t)min(syi - 1, max(0, y1 - 2 + b)) * sxi;
-#pragma unroll
-                for (int a = 0; a < 6; a++) P[a][b] = __fmul_rn((float)__ldg(src + col[a]), Lx[a]);
-            }
-        }
-        float Ly[6];
-#pragma unroll
-        for (int b = 0; b < 6; b++) Ly[b] = __ldg(ly + y * 6 + b);
-        float v = 0.0f, w = 0.0f;
-#pragma unroll
-        for (int a = 0; a < 6; a++)
-#pragma unroll
-            for (int b = 0; b < 6; b++) {
-                w = __fmaf_rn(Lx[a], Ly[b], w);
-                v = __fmaf_rn(P[a][b], Ly[b], v);
-            }
-        const float val = v / w;
+        const float val = v[r] / w[r];
         const size_t o = X + (size_t)Y * pitch;
         out[o] = val;
         const uint32_t key = sample_key(val);
@@ -612,7 +626,7 @@ cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_
     // Eight rows a thread share the most products; a grid of fewer blocks than SMs takes
     // fewer rows a thread and with them less time for its chain of rows (96x64 u1.5: 11.4
     // us with eight, 8.8, 8.0 and 6.9 with four, two and one; 1024x436 u2.9 47.6, 46.0,
-    // 56.7 and 76.3, 1920x1080 u4.9 434, 490, 622 and 913).
+    // 56.7 and 76.3, 1920x1080 u4.9 434, 490, 622 and 913; with a division per row, above).
     int sms = 0;
     const cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) return e;
