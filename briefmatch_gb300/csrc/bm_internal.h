@@ -49,9 +49,11 @@ cudaError_t upsample_u8(const uint8_t* in, float* out, int sxi, int syi, int sxo
 // Up-sampling into an image with an edge-replicated margin of m pixels on every
 // side; `out` is the start of the (sxo + 2m) x (syo + 2m) buffer, row pitch `pitch`.
 // `keys`, of the same shape, receives the 16-bit keys the descriptors compare first: per
-// word the pixel's key and that of the pixel below it.
-cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_t* keys, int pitch, int m, int sxi, int syi, int sxo,
-                            int syo, const float* lx, const int* ix, const float* ly, const int* iy, cudaStream_t st);
+// word the pixel's key and that of the pixel below it.  `frame`, unless null, receives the
+// input frame as float.
+cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_t* keys, int pitch, int m, int sxi,
+                            int syi, int sxo, int syo, const float* lx, const int* ix, const float* ly, const int* iy,
+                            cudaStream_t st);
 cudaError_t u8_to_f32(const uint8_t* in, float* out, size_t n, cudaStream_t st);
 
 // Linear image offsets (o1, o2) of every BRIEF sample for one image width, padded
