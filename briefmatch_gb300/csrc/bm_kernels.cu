@@ -624,9 +624,9 @@ cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_
 {
     if (m < 0 || pitch < sxo + 2 * m) return cudaErrorInvalidValue;
     // Eight rows a thread share the most products; a grid of fewer blocks than SMs takes
-    // fewer rows a thread and with them less time for its chain of rows (96x64 u1.5: 11.4
-    // us with eight, 8.8, 8.0 and 6.9 with four, two and one; 1024x436 u2.9 47.6, 46.0,
-    // 56.7 and 76.3, 1920x1080 u4.9 434, 490, 622 and 913; with a division per row, above).
+    // four or two rows a thread and with them less time for its chain of rows (96x64 u1.5:
+    // 10.6 us with eight, 8.8 and 7.2 with four and two, 7.3 with one; 1024x436 u2.9 39.4,
+    // 43.6, 56.2, 1920x1080 u4.9 394, 492, 662).
     int sms = 0;
     const cudaError_t e = sm_count(&sms);
     if (e != cudaSuccess) return e;
@@ -637,8 +637,7 @@ cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_
     const long columns = (sxo + 2 * m + TX - 1) / TX, eights = (syo + 2 * m + TY - 1) / TY;
     if (columns * eights >= 8L * sms) rows(k_upsample_pad_rows<8>, 8);
     else if (columns * eights >= 4L * sms) rows(k_upsample_pad_rows<4>, 4);
-    else if (columns * eights >= 2L * sms) rows(k_upsample_pad_rows<2>, 2);
-    else rows(k_upsample_pad_rows<1>, 1);
+    else rows(k_upsample_pad_rows<2>, 2);
     return cudaGetLastError();
 }
 
