@@ -881,18 +881,25 @@ __device__ __forceinline__ void median2_px(const float* in, float* __restrict__ 
 //
 // The three Gaussians are one exp2 of the summed exponents:
 // q = du^2 + dv^2 + dI^2 + j^2 cS over scaled differences (kE = sqrt(cE), kI = sqrt(cI)).
-// Samples are staged as kE (u - ru) with one reference flow per block (a nearby median
-// value): scaling and subtraction round relative to the small difference, the sums are
-// of small numbers, and the reference is added back to the quotient, which leaves a
-// fifth of the error of sums over the flow itself (1920x1080: 3.9e-8 of the field's norm
-// against 64 bits, 2.1e-7 before).  The column factor exp2(-cS i^2) is applied once per
+// What is summed are the weighted differences du and dv to the output's own median value,
+// which is added back to the quotient: the sums are of small numbers whatever the flow is,
+// and a value depends on nothing outside its window.  The scaled centre's rounding is known
+// (one FMA) and taken off the quotient.  Against 64 bits that leaves an error of about half
+// a unit in the last place of the pixel's own flow: 3.5e-8 of the norm of a 1920x1080 field
+// (sums of the flow itself 2.1e-7).  Sums relative to one reference flow per block reach
+// 3.4e-8 there, but are up to 3e-4 px off at small flows beside a fast object (float32
+// restatement; these: 6e-10 px).  The column factor exp2(-cS i^2) is applied once per
 // column.  Nine FP32 lane operations per tap and output.
 //
 // What bounds it is the FP32 pipe's operand reads: a packed FMA with three different
 // 64-bit operands takes three cycles, with two it takes two (measured).  So differences
 // are additions, squares read one register twice, and only the two weighted sums need
 // three operands: 20 cycles per pair of taps, 18 by operation count.  1920x1080 with a
-// 94 x 94 window: 7.16 -> 5.66 ms; 1024x436 (48 x 48): 400 -> 344 us.
+// 94 x 94 window: 7.16 -> 5.72 ms (5.66 relative to one reference flow per block);
+// 1024x436 (48 x 48): 400 -> 345 us.
+//
+// Flows beyond TRI_FAR of a standard deviation (and infinite ones) as a centre: the sums
+// over differences would meet 0 * inf, so such an output takes its sums over the flow.
 //
 // Row pairs: source row m lies in output r's window when 0 <= m - r < 2s.  Outputs 0
 // and 2 take whole pairs; outputs 1 and 3 have a single row in their first and last
@@ -916,9 +923,13 @@ __host__ __device__ inline size_t tri_smem_bytes(int s, int ty)
     return (size_t)(s + 1) * sizeof(float4) + (tile > sums ? tile : sums) * sizeof(float);
 }
 
-// A common flow (or intensity) that the samples of a block are taken relative to: a
-// nearby value where that is an ordinary one, else 0.
-__device__ __forceinline__ float tri_reference(float v) { return fabsf(v) <= 1024.0f ? v : 0.0f; }
+constexpr float TRI_FAR = 1e30f;
+// A sample times its scale; a finite one stays finite.
+__device__ __forceinline__ float tri_scaled(float k, float v)
+{
+    const float big = 3.402823466e38f, t = __fmul_rn(k, v);
+    return fabsf(v) <= big ? fminf(fmaxf(t, -big), big) : t;
+}
 
 // 2^-x per half.  The negation is spelled without .ftz, which makes it a modifier of the
 // exponential's operand: under -use_fast_math a C++ minus is neg.ftz, an addition of its
@@ -946,16 +957,13 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
     float* sV = sU + TW * P;
     float* sI = sV + TW * P;
     const int x0 = bx0 - s, y0 = by0 - s;
-    // the block's reference flow and intensity
-    const size_t mid = (size_t)min(sx - 1, bx0 + TX / 2) + (size_t)min(sy - 1, by0 + tri_rows(TY) / 2) * sx;
-    const float ru = tri_reference(Um[mid]), rv = tri_reference(Vm[mid]), ri = tri_reference(__ldg(I + mid));
     for (int r = threadIdx.z * TY + threadIdx.y; r < TH; r += TY * TRI_G) {
         const size_t row = (size_t)min(sy - 1, max(0, y0 + r)) * sx;
         for (int c = threadIdx.x; c < TW; c += TX) {
             const size_t g = row + min(sx - 1, max(0, x0 + c));
-            sU[c * P + r] = __fmul_rn(kE, __fsub_rn(__ldg(U + g), ru));
-            sV[c * P + r] = __fmul_rn(kE, __fsub_rn(__ldg(V + g), rv));
-            sI[c * P + r] = __fmul_rn(kI, __fsub_rn(__ldg(I + g), ri));
+            sU[c * P + r] = tri_scaled(kE, __ldg(U + g));
+            sV[c * P + r] = tri_scaled(kE, __ldg(V + g));
+            sI[c * P + r] = __fmul_rn(kI, __ldg(I + g));
         }
     }
     for (int p = threadIdx.y * TX + threadIdx.x; p <= s; p += TX * TY) {
@@ -973,7 +981,7 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
 #pragma unroll
     for (int r = 0; r < TRI_R; r++) {
         const size_t o = (size_t)min(sx - 1, x) + (size_t)min(sy - 1, yb + r) * sx;
-        const float a = __fmul_rn(-kE, __fsub_rn(Um[o], ru)), b = __fmul_rn(-kE, __fsub_rn(Vm[o], rv));
+        const float a = __fmul_rn(-kE, Um[o]), b = __fmul_rn(-kE, Vm[o]);
         const float i0 = -sI[(threadIdx.x + s) * P + threadIdx.y * TRI_R + r + s];
         um[r] = pk2(a, a);
         vm[r] = pk2(b, b);
@@ -1000,13 +1008,11 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
             t.i = *reinterpret_cast<const f2x*>(cu + 2 * plane + 2 * p);
             return t;
         };
-        auto weight = [&](int r, const Pair& t, f2x row) {
+        auto sums = [&](int r, const Pair& t, f2x row) {
             const f2x du = add2(t.u, um[r]), dv = add2(t.v, vm[r]), dI = add2(t.i, ic[r]);
-            return ex2n_2(fma2(dI, dI, fma2(dv, dv, fma2(du, du, row))));
-        };
-        auto sums = [&](int r, const Pair& t, f2x w) {
-            au[r] = fma2(w, t.u, au[r]);
-            av[r] = fma2(w, t.v, av[r]);
+            const f2x w = ex2n_2(fma2(dI, dI, fma2(dv, dv, fma2(du, du, row))));
+            au[r] = fma2(w, du, au[r]);
+            av[r] = fma2(w, dv, av[r]);
             aw[r] = add2(aw[r], w);
         };
         auto upper = [&](const Pair& t) { return Pair{pk2(0.0f, hi2(t.u)), pk2(0.0f, hi2(t.v)), pk2(0.0f, hi2(t.i))}; };
@@ -1014,18 +1020,18 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
         ulonglong2 f = terms[0];
         f2x e0 = f.x, e1 = f.y;                       // the previous pair's terms
         Pair t = load(0);                             // rows 0, 1
-        sums(0, t, weight(0, t, e0));
+        sums(0, t, e0);
         Pair h = upper(t);
-        sums(1, h, weight(1, h, e1));
+        sums(1, h, e1);
         if (s > 1) {
             f = terms[1];
             t = load(1);                              // rows 2, 3
             f2x t0 = f.x, t1 = f.y;
-            sums(0, t, weight(0, t, t0));
-            sums(1, t, weight(1, t, t1));
-            sums(2, t, weight(2, t, e0));
+            sums(0, t, t0);
+            sums(1, t, t1);
+            sums(2, t, e0);
             h = upper(t);
-            sums(3, h, weight(3, h, e1));
+            sums(3, h, e1);
 #pragma unroll TRI_UNROLL
             for (int p = 2; p < s; p++) {
                 f = terms[p];
@@ -1035,10 +1041,10 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
                 e0 = f.x;
                 e1 = f.y;
                 t = load(p);
-                sums(0, t, weight(0, t, t0));
-                sums(1, t, weight(1, t, t1));
-                sums(2, t, weight(2, t, e0));
-                sums(3, t, weight(3, t, e1));
+                sums(0, t, t0);
+                sums(1, t, t1);
+                sums(2, t, e0);
+                sums(3, t, e1);
             }
             f = terms[s - 1];
             e0 = f.x;
@@ -1048,17 +1054,17 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
         t = load(s);                                  // rows 2s, 2s + 1
         const f2x last = f.y;
         h = lower(t);
-        sums(1, h, weight(1, h, last));
-        sums(2, t, weight(2, t, e0));
+        sums(1, h, last);
+        sums(2, t, e0);
         if (s > 1) {
-            sums(3, t, weight(3, t, e1));
+            sums(3, t, e1);
         } else {
             h = upper(t);
-            sums(3, h, weight(3, h, e1));
+            sums(3, h, e1);
         }
         t = load(s + 1);                              // row 2s + 2
         h = lower(t);
-        sums(3, h, weight(3, h, last));
+        sums(3, h, last);
         const float wi = exp2f(-(float)(i * i) * cS);
 #pragma unroll
         for (int r = 0; r < TRI_R; r++) {
@@ -1087,13 +1093,38 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
 #pragma unroll
     for (int r = 0; r < TRI_R; r++) {
         const float w = sw[r] + part[(3 * r + 2) * TX * TY + tid];
-        const float mu = (su[r] + part[(3 * r + 0) * TX * TY + tid]) * inv_k;
-        const float mv = (sv[r] + part[(3 * r + 1) * TX * TY + tid]) * inv_k;
+        const float mu = su[r] + part[(3 * r + 0) * TX * TY + tid];
+        const float mv = sv[r] + part[(3 * r + 1) * TX * TY + tid];
         if (yb + r < sy) {
             const size_t o = (size_t)x + (size_t)(yb + r) * sx;
-            // sum of w u over max(1e-5, sum of w), with u = ru + the centred scaled sample / kE
-            Uo[o] = w < 1e-5f ? __fdiv_rn(__fmaf_rn(ru, w, mu), 1e-5f) : ru + __fdiv_rn(mu, w);
-            Vo[o] = w < 1e-5f ? __fdiv_rn(__fmaf_rn(rv, w, mv), 1e-5f) : rv + __fdiv_rn(mv, w);
+            // sum of w u over max(1e-5, sum of w): with u = a + (d - e) / kE, a the centre, d
+            // the summed difference and e what the scaled centre was rounded by
+            auto quotient = [&](float a, float neg, float m) {
+                const float e = __fmaf_rn(kE, a, neg);
+                return w < 1e-5f ? __fdiv_rn(__fmaf_rn(a, w, __fmaf_rn(-e, w, m) * inv_k), 1e-5f)
+                                 : __fmaf_rn(__fdiv_rn(m, w) - e, inv_k, a);
+            };
+            const float a = Um[o], b = Vm[o];
+            float u = quotient(a, lo2(um[r]), mu), v = quotient(b, lo2(vm[r]), mv);
+            const bool far_u = fabsf(lo2(um[r])) > TRI_FAR, far_v = fabsf(lo2(vm[r])) > TRI_FAR;
+            if (far_u || far_v) {
+                float fu = 0.0f, fv = 0.0f, fw = 0.0f;
+#pragma unroll 1
+                for (int k = 0; k < 4 * s * s; k++) {
+                    const int i = k / (2 * s) - s, j = k % (2 * s) - s;
+                    const size_t g = (size_t)min(sx - 1, max(0, x + i)) + (size_t)min(sy - 1, max(0, yb + r + j)) * sx;
+                    const float du = tri_scaled(kE, U[g]) + lo2(um[r]), dv = tri_scaled(kE, V[g]) + lo2(vm[r]);
+                    const float dI = __fmul_rn(kI, I[g]) + lo2(ic[r]);
+                    const float f = exp2f(-(du * du + dv * dv + dI * dI + (float)(i * i + j * j) * cS));
+                    fu = __fmaf_rn(f, U[g], fu);
+                    fv = __fmaf_rn(f, V[g], fv);
+                    fw += f;
+                }
+                if (far_u) u = __fdiv_rn(fu, fmaxf(1e-5f, fw));
+                if (far_v) v = __fdiv_rn(fv, fmaxf(1e-5f, fw));
+            }
+            Uo[o] = u;
+            Vo[o] = v;
         }
     }
 }
