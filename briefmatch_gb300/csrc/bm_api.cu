@@ -832,13 +832,23 @@ bm_status bm_swap(bm_ctx* c)
 
 namespace {
 
+// Memory that only the device can write: the runtime's copies take it for a host pointer
+// all the same, a host copy cannot.
+bool device_memory(const void* p)
+{
+    cudaPointerAttributes a = {};
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeDevice;
+    cudaGetLastError();
+    return false;
+}
+
 // The refined flow into host memory, and a wait for it.  Small frames go through a pinned
 // buffer: one copy of both planes, then host copies, instead of two copies to pageable
 // memory that each wait for the device (STAGE_MAX).
 bm_status copy_out(bm_ctx* c, float* h_u, float* h_v)
 {
     const size_t b = c->npix_in * sizeof(float);
-    if (c->h_stage && h_u && h_v) {
+    if (c->h_stage && h_u && h_v && !device_memory(h_u) && !device_memory(h_v)) {
         BM_CUDA(cudaMemcpyAsync(c->h_stage, c->d_flow_out, 2 * b, cudaMemcpyDeviceToHost, c->stream));
         BM_CUDA(cudaStreamSynchronize(c->stream));
         std::memcpy(h_u, c->h_stage, b);
