@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -53,9 +54,12 @@ bm_status fail(bm_status st, const char* fmt, ...)
 
 void bmk::set_error_text(const char* msg) { g_last_error = msg ? msg : ""; }
 
-// Largest output of both planes that goes to the host through a pinned buffer: a pair of
-// 96x64 frames (48 KB) took 135 us with two copies to pageable memory, 120 with one to the
-// pinned buffer; 160x120 (150 KB) 146 and 145, 320x240 (600 KB) 209 and 260.
+// Largest output of both planes that goes to the host in one copy to a buffer of the
+// context's and two host copies, instead of two copies to the caller's memory that each wait
+// for the device: a host pair of 96x64 frames (48 KB) took 191 us with two copies, 183 with
+// one; 128x96 202 and 195, 160x120 217 and 213, but 240x180 274 and 282, 320x240 355 and 380.
+// The buffer is ordinary memory: a page-locked one saves 2 us a frame, but takes 310 us to
+// make and free, more than the rest of a 96x64 context does.
 constexpr size_t STAGE_MAX = 96 * 1024;
 
 struct bm_ctx {
@@ -101,7 +105,7 @@ struct bm_ctx {
     cudaEvent_t ev_refined = nullptr;             // refine stream: last refinement and copies done
     float* d_flow_med = nullptr;
     float* d_flow_out = nullptr;
-    float* h_stage = nullptr;   // pinned copy of d_flow_out for host outputs of small frames (copy_out)
+    float* h_stage = nullptr;   // host copy of d_flow_out for host outputs of small frames (copy_out)
     float* d_tmp = nullptr;
     int4* d_pattern = nullptr;
     int pattern_rmax = 0;
@@ -230,7 +234,7 @@ bm_status dev_alloc(T** p, size_t count)
 
 void release(bm_ctx* c)
 {
-    if (c->h_stage) cudaFreeHost(c->h_stage);
+    delete[] c->h_stage;
     c->h_stage = nullptr;
     void* ptrs[] = {c->d_u8[0], c->d_u8[1], c->d_u8[2], c->d_pred, c->d_frame[0], c->d_frame[1], c->d_frame[2], c->d_up, c->d_upad,
                     c->d_feat[0], c->d_feat[1], c->d_flow[0], c->d_flow[1], c->d_cost, c->d_flow_in_buf[0],
@@ -555,11 +559,8 @@ bm_status bm_create(const bm_params* prm, bm_ctx** out)
     c->d_flow_in = c->d_flow_in_buf[0];
     BM_TRY(dev_alloc(&c->d_flow_med, 2 * ni));
     BM_TRY(dev_alloc(&c->d_flow_out, 2 * ni));
-    if (2 * ni * sizeof(float) <= STAGE_MAX &&
-        cudaMallocHost((void**)&c->h_stage, 2 * ni * sizeof(float)) != cudaSuccess) {
-        c->h_stage = nullptr;   // the planes are then copied directly
-        cudaGetLastError();
-    }
+    // (without it the planes are copied directly)
+    if (2 * ni * sizeof(float) <= STAGE_MAX) c->h_stage = new (std::nothrow) float[2 * ni];
     BM_TRY(dev_alloc(&c->d_tmp, 2 * ni));
     BM_TRY(dev_alloc(&c->d_pattern, BM_PATCH_MAX / 4));
     BM_TRY(dev_alloc(&c->d_taps, BM_CONST_KERNEL_SIZE));
@@ -842,9 +843,9 @@ bool device_memory(const void* p)
     return false;
 }
 
-// The refined flow into host memory, and a wait for it.  Small frames go through a pinned
-// buffer: one copy of both planes, then host copies, instead of two copies to pageable
-// memory that each wait for the device (STAGE_MAX).
+// The refined flow into host memory, and a wait for it.  Small frames go through a buffer
+// of the context's: one copy of both planes, then host copies, instead of two copies that
+// each wait for the device (STAGE_MAX).
 bm_status copy_out(bm_ctx* c, float* h_u, float* h_v)
 {
     const size_t b = c->npix_in * sizeof(float);

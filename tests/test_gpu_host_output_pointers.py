@@ -3,6 +3,7 @@ pointer whatever the frame's size, through the host buffer of small frames and w
 from __future__ import annotations
 
 import ctypes
+import time
 
 import numpy as np
 import pytest
@@ -38,3 +39,19 @@ def test_device_memory_as_host_output(W, H):
     assert np.array_equal(got[0, 0], want[0]) and np.array_equal(got[0, 1], want[1])
     assert np.array_equal(host, want[0]) and np.array_equal(got[1, 1], want[1])
     eng.clean()
+
+
+def test_a_small_context_is_made_as_fast_as_a_larger_one():
+    """Contexts with the host buffer (96x64) and without it (160x120), in turn: the smaller
+    one's buffers are made and freed in less time, page-locked memory would double it."""
+    params = [bm.BMParams.derive(W, H, 1.5, 1.5, N=64) for W, H in ((96, 64), (160, 120))]
+    times = ([], [])
+    for _ in range(25):
+        for prm, t in zip(params, times):
+            t0 = time.perf_counter()
+            eng = bm.BriefMatch(prm)
+            eng.setup()
+            eng.clean()
+            t.append(time.perf_counter() - t0)
+    small, large = (float(np.median(t)) for t in times)
+    assert small <= 1.2 * large
