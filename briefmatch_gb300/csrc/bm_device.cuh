@@ -876,7 +876,7 @@ __device__ __forceinline__ void median2_px(const float* in, float* __restrict__ 
 // packed f32x2 registers hold the two rows, so a sample pair is used as it is read from
 // shared memory (the tile is stored column by column) and serves all four outputs.
 // TRI_G = 2 groups of TX x TY threads share a tile, each taking half of the window's
-// columns; their sums meet in shared memory.  The neighbourhood is staged with
+// columns; their sums meet in shared memory (small windows: one group, G = 1).  The neighbourhood is staged with
 // clamp-to-edge addressing, `smem` must hold tri_smem_bytes(s, TY).
 //
 // The three Gaussians are one exp2 of the summed exponents:
@@ -885,7 +885,7 @@ __device__ __forceinline__ void median2_px(const float* in, float* __restrict__ 
 // which is added back to the quotient: the sums are of small numbers whatever the flow is,
 // and a value depends on nothing outside its window.  The scaled centre's rounding is known
 // (one FMA) and taken off the quotient.  Against 64 bits that leaves an error of about half
-// a unit in the last place of the pixel's own flow: 3.5e-8 of the norm of a 1920x1080 field
+// a unit in the last place of the pixel's own flow: 3.0e-8 of the norm of a 1920x1080 field
 // (sums of the flow itself 2.1e-7).  Sums relative to one reference flow per block reach
 // 3.4e-8 there, but are up to 3e-4 px off at small flows beside a fast object (float32
 // restatement; these: 6e-10 px).  The column factor exp2(-cS i^2) is applied once per
@@ -895,8 +895,9 @@ __device__ __forceinline__ void median2_px(const float* in, float* __restrict__ 
 // 64-bit operands takes three cycles, with two it takes two (measured).  So differences
 // are additions, squares read one register twice, and only the two weighted sums need
 // three operands: 20 cycles per pair of taps, 18 by operation count.  1920x1080 with a
-// 94 x 94 window: 7.16 -> 5.72 ms (5.66 relative to one reference flow per block);
-// 1024x436 (48 x 48): 400 -> 345 us.
+// 94 x 94 window: 7.16 -> 5.61 ms; 1024x436 (48 x 48): 400 -> 344 us.  The tile's loads are
+// eight in flight per thread, the medians' before them; one after the other they took 0.1 ms
+// of the former, and half the time of small windows.
 //
 // Flows beyond TRI_FAR of a standard deviation (and infinite ones) as a centre: the sums
 // over differences would meet 0 * inf, so such an output takes its sums over the flow.
@@ -909,7 +910,7 @@ __device__ __forceinline__ void median2_px(const float* in, float* __restrict__ 
 constexpr int TRI_R = 4;       // outputs per thread
 constexpr int TRI_UNROLL = 8;  // row pairs per turn of the column walk (measured: 1, 2, 4, 8, 16)
 constexpr int TRI_MAX_S = 52;  // largest half window whose tile fits an SM's shared memory (226 KB)
-constexpr int TRI_G = 2;       // thread groups per block, each taking half of the window's columns
+constexpr int TRI_G = 2;       // thread groups per block, each taking half of the window's columns (small windows: 1)
 
 // Rows of a tile of TY thread rows, and floats per tile column: the rows, padded to 2
 // modulo 4 so that the 16 lanes of a 64-bit read phase fall on 32 different banks.
@@ -928,7 +929,7 @@ constexpr float TRI_FAR = 1e30f;
 __device__ __forceinline__ float tri_scaled(float k, float v)
 {
     const float big = 3.402823466e38f, t = __fmul_rn(k, v);
-    return fabsf(v) <= big ? fminf(fmaxf(t, -big), big) : t;
+    return fabsf(t) > big && fabsf(v) <= big ? copysignf(big, t) : t;
 }
 
 // 2^-x per half.  The negation is spelled without .ftz, which makes it a modifier of the
@@ -942,7 +943,7 @@ __device__ __forceinline__ float ex2n(float x)
 }
 __device__ __forceinline__ f2x ex2n_2(f2x a) { return pk2(ex2n(lo2(a)), ex2n(hi2(a))); }
 
-template <int TY>
+template <int TY, int G>
 __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, const float* __restrict__ V,
                                                  const float* Um, const float* Vm,
                                                  const float* __restrict__ I, float* __restrict__ Uo,
@@ -957,13 +958,45 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
     float* sV = sU + TW * P;
     float* sI = sV + TW * P;
     const int x0 = bx0 - s, y0 = by0 - s;
-    for (int r = threadIdx.z * TY + threadIdx.y; r < TH; r += TY * TRI_G) {
-        const size_t row = (size_t)min(sy - 1, max(0, y0 + r)) * sx;
-        for (int c = threadIdx.x; c < TW; c += TX) {
-            const size_t g = row + min(sx - 1, max(0, x0 + c));
-            sU[c * P + r] = tri_scaled(kE, __ldg(U + g));
-            sV[c * P + r] = tri_scaled(kE, __ldg(V + g));
-            sI[c * P + r] = __fmul_rn(kI, __ldg(I + g));
+    const int x = bx0 + threadIdx.x;
+    const int yb = by0 + threadIdx.y * TRI_R;
+    // (pixels outside the image compute on clamped centres and store nothing)
+    f2x um[TRI_R], vm[TRI_R], ic[TRI_R];   // negated scaled centres, twice
+#pragma unroll
+    for (int r = 0; r < TRI_R; r++) {
+        const size_t o = (size_t)min(sx - 1, x) + (size_t)min(sy - 1, yb + r) * sx;
+        const float a = __fmul_rn(-kE, Um[o]), b = __fmul_rn(-kE, Vm[o]);
+        um[r] = pk2(a, a);
+        vm[r] = pk2(b, b);
+    }
+    // four rows of two columns at a time: their loads are in flight together
+    constexpr int STEP = TY * G, ROWS = 4;
+    for (int c0 = threadIdx.x; c0 < TW; c0 += 2 * TX) {
+        const int gx[2] = {min(sx - 1, max(0, x0 + c0)), min(sx - 1, max(0, x0 + c0 + TX))};
+        const int cols = c0 + TX < TW ? 2 : 1;
+        for (int r0 = threadIdx.z * TY + threadIdx.y; r0 < TH; r0 += STEP * ROWS) {
+            float a[ROWS][2], b[ROWS][2], i[ROWS][2];
+#pragma unroll
+            for (int k = 0; k < ROWS; k++) {
+                const size_t row = (size_t)min(sy - 1, max(0, y0 + r0 + k * STEP)) * sx;
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    if (r0 + k * STEP < TH && h < cols) {
+                        a[k][h] = __ldg(U + row + gx[h]);
+                        b[k][h] = __ldg(V + row + gx[h]);
+                        i[k][h] = __ldg(I + row + gx[h]);
+                    }
+            }
+#pragma unroll
+            for (int k = 0; k < ROWS; k++)
+#pragma unroll
+                for (int h = 0; h < 2; h++)
+                    if (r0 + k * STEP < TH && h < cols) {
+                        const int at = (c0 + h * TX) * P + r0 + k * STEP;
+                        sU[at] = tri_scaled(kE, a[k][h]);
+                        sV[at] = tri_scaled(kE, b[k][h]);
+                        sI[at] = __fmul_rn(kI, i[k][h]);
+                    }
         }
     }
     for (int p = threadIdx.y * TX + threadIdx.x; p <= s; p += TX * TY) {
@@ -974,17 +1007,9 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
     }
     __syncthreads();
 
-    const int x = bx0 + threadIdx.x;
-    const int yb = by0 + threadIdx.y * TRI_R;
-    // (pixels outside the image compute on clamped centres and store nothing)
-    f2x um[TRI_R], vm[TRI_R], ic[TRI_R];   // negated scaled centres, twice
 #pragma unroll
     for (int r = 0; r < TRI_R; r++) {
-        const size_t o = (size_t)min(sx - 1, x) + (size_t)min(sy - 1, yb + r) * sx;
-        const float a = __fmul_rn(-kE, Um[o]), b = __fmul_rn(-kE, Vm[o]);
         const float i0 = -sI[(threadIdx.x + s) * P + threadIdx.y * TRI_R + r + s];
-        um[r] = pk2(a, a);
-        vm[r] = pk2(b, b);
         ic[r] = pk2(i0, i0);
     }
     float su[TRI_R], sv[TRI_R], sw[TRI_R];
@@ -1073,39 +1098,70 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
             sw[r] = __fmaf_rn(wi, lo2(aw[r]) + hi2(aw[r]), sw[r]);
         }
     };
-    // group z: columns [-s, 0) or [0, s)
-    for (int k = 0; k < s; k++) column(threadIdx.z ? k : k - s);
-
-    __syncthreads();   // every group is done with the tile
-    float* part = sU;  // [3 * TRI_R][TY * TX]
+    // the columns [-s, 0) and [0, s) are summed apart, by two groups or one after the other,
+    // and added at the end: a value is the same either way
     const int tid = threadIdx.y * TX + threadIdx.x;
-    if (threadIdx.z) {
+    float other_u[TRI_R], other_v[TRI_R], other_w[TRI_R];
+    if constexpr (G == 2) {
+        for (int k = 0; k < s; k++) column(threadIdx.z ? k : k - s);
+        __syncthreads();   // every group is done with the tile
+        if (threadIdx.z) {
 #pragma unroll
-        for (int r = 0; r < TRI_R; r++) {
-            part[(3 * r + 0) * TX * TY + tid] = su[r];
-            part[(3 * r + 1) * TX * TY + tid] = sv[r];
-            part[(3 * r + 2) * TX * TY + tid] = sw[r];
+            for (int r = 0; r < TRI_R; r++) {
+                sU[(3 * r + 0) * TX * TY + tid] = su[r];
+                sU[(3 * r + 1) * TX * TY + tid] = sv[r];
+                sU[(3 * r + 2) * TX * TY + tid] = sw[r];
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int half = 0; half < 2; half++) {
+            for (int k = 0; k < s; k++) column(half ? k : k - s);
+            if (half == 0) {
+#pragma unroll
+                for (int r = 0; r < TRI_R; r++) {
+                    other_u[r] = su[r];
+                    other_v[r] = sv[r];
+                    other_w[r] = sw[r];
+                    su[r] = sv[r] = sw[r] = 0.0f;
+                }
+            }
         }
     }
-    __syncthreads();
+    float a[TRI_R], b[TRI_R];
+#pragma unroll
+    for (int r = 0; r < TRI_R; r++) {
+        const size_t o = (size_t)min(sx - 1, x) + (size_t)min(sy - 1, yb + r) * sx;
+        a[r] = threadIdx.z ? 0.0f : Um[o];
+        b[r] = threadIdx.z ? 0.0f : Vm[o];
+    }
+    if constexpr (G == 2) {
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < TRI_R; r++) {
+            other_u[r] = sU[(3 * r + 0) * TX * TY + tid];
+            other_v[r] = sU[(3 * r + 1) * TX * TY + tid];
+            other_w[r] = sU[(3 * r + 2) * TX * TY + tid];
+        }
+    }
     if (threadIdx.z || x >= sx || yb >= sy) return;
     const float inv_k = __frcp_rn(kE);
 #pragma unroll
     for (int r = 0; r < TRI_R; r++) {
-        const float w = sw[r] + part[(3 * r + 2) * TX * TY + tid];
-        const float mu = su[r] + part[(3 * r + 0) * TX * TY + tid];
-        const float mv = sv[r] + part[(3 * r + 1) * TX * TY + tid];
+        const float w = sw[r] + other_w[r];
+        const float mu = su[r] + other_u[r];
+        const float mv = sv[r] + other_v[r];
         if (yb + r < sy) {
             const size_t o = (size_t)x + (size_t)(yb + r) * sx;
             // sum of w u over max(1e-5, sum of w): with u = a + (d - e) / kE, a the centre, d
             // the summed difference and e what the scaled centre was rounded by
-            auto quotient = [&](float a, float neg, float m) {
-                const float e = __fmaf_rn(kE, a, neg);
-                return w < 1e-5f ? __fdiv_rn(__fmaf_rn(a, w, __fmaf_rn(-e, w, m) * inv_k), 1e-5f)
-                                 : __fmaf_rn(__fdiv_rn(m, w) - e, inv_k, a);
+            auto quotient = [&](float centre, float neg, float m) {
+                const float e = __fmaf_rn(kE, centre, neg);
+                const bool none = w < 1e-5f;
+                const float q = __fdiv_rn(none ? __fmaf_rn(centre, w, __fmaf_rn(-e, w, m) * inv_k) : m, none ? 1e-5f : w);
+                return none ? q : __fmaf_rn(q - e, inv_k, centre);
             };
-            const float a = Um[o], b = Vm[o];
-            float u = quotient(a, lo2(um[r]), mu), v = quotient(b, lo2(vm[r]), mv);
+            float u = quotient(a[r], lo2(um[r]), mu), v = quotient(b[r], lo2(vm[r]), mv);
             const bool far_u = fabsf(lo2(um[r])) > TRI_FAR, far_v = fabsf(lo2(vm[r])) > TRI_FAR;
             if (far_u || far_v) {
                 float fu = 0.0f, fv = 0.0f, fw = 0.0f;

@@ -491,8 +491,8 @@ __global__ void __launch_bounds__(256) k_median_pass(const float* inU, const flo
     }
 }
 
-template <int TY>
-__global__ void __launch_bounds__(TX * TY * TRI_G, 8 / TY) k_trilateral(const float* __restrict__ U,
+template <int TY, int G>
+__global__ void __launch_bounds__(TX * TY * G, 16 / (TY * G)) k_trilateral(const float* __restrict__ U,
                                                                        const float* __restrict__ V,
                                                                        const float* Um,
                                                                        const float* Vm,
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(TX * TY * TRI_G, 8 / TY) k_trilateral(const fl
     chain_wait();
     chain_trigger();
     extern __shared__ float4 smem4[];
-    trilateral_block<TY>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, kE, kI, cS, blockIdx.x * TX, blockIdx.y * tri_rows(TY),
+    trilateral_block<TY, G>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, kE, kI, cS, blockIdx.x * TX, blockIdx.y * tri_rows(TY),
                          smem4);
 }
 
@@ -519,6 +519,8 @@ __global__ void __launch_bounds__(256) k_trilateral_global(const float* __restri
     if (x >= sx || y >= sy) return;
     const size_t o = (size_t)x + (size_t)y * sx;
     const float um0 = Um[o], vm0 = Vm[o], I0 = I[o];
+    // sums relative to the centre, as trilateral_block's
+    const float bu = fabsf(um0) <= TRI_FAR ? um0 : 0.0f, bv = fabsf(vm0) <= TRI_FAR ? vm0 : 0.0f;
     float uf = 0.0f, vf = 0.0f, W = 0.0f;
     for (int i = -s; i < s; i++) {
         const int gx = min(sx - 1, max(0, x + i));
@@ -531,14 +533,13 @@ __global__ void __launch_bounds__(256) k_trilateral_global(const float* __restri
             const float e = du * du + dv * dv;
             const float sp = si + (float)(j * j) * cS;
             const float w = exp2f(fmaf(e, -cE, fmaf(dI * dI, -cI, -sp)));
-            uf = fmaf(w, u1, uf);
-            vf = fmaf(w, v1, vf);
+            uf = fmaf(w, u1 - bu, uf);
+            vf = fmaf(w, v1 - bv, vf);
             W += w;
         }
     }
-    const float Wc = fmaxf(1e-5f, W);
-    Uo[o] = uf / Wc;
-    Vo[o] = vf / Wc;
+    Uo[o] = W < 1e-5f ? fmaf(bu, W, uf) / 1e-5f : bu + uf / W;
+    Vo[o] = W < 1e-5f ? fmaf(bv, W, vf) / 1e-5f : bv + vf / W;
 }
 
 // ---------------------------------------------------------------------------
@@ -802,9 +803,9 @@ cudaError_t ensure_trilateral_smem(int s)
     const int need = (int)tri_smem_bytes(s, 8);
     std::lock_guard<std::mutex> lock(mu);
     if (need <= granted[dev]) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_trilateral<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trilateral<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trilateral<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    e = cudaFuncSetAttribute(k_trilateral<8, TRI_G>, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trilateral<4, TRI_G>, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_trilateral<2, TRI_G>, cudaFuncAttributeMaxDynamicSharedMemorySize, need);
     if (e == cudaSuccess) granted[dev] = need;
     return e;
 }
@@ -821,27 +822,35 @@ static int trilateral_rows(int sx, int sy, int s, int sms)
     return 4 * tri_smem_bytes(s, 2) <= per_sm ? 2 : 2 * tri_smem_bytes(s, 4) <= per_sm ? 4 : 8;
 }
 
+// Half windows up to TRI_SMALL_S on a grid several waves deep take blocks of four warps
+// without the groups' exchange: a window this small is over before the next block's loads
+// arrive, so four blocks share an SM (with the medians, 1920x1080, s = 2, 4 and 8: 84, 122 and
+// 256 us by blocks of 8 rows, 66, 99 and 228 by these; s = 12: 467 and 439, where the larger
+// block is ahead from s = 16 on smaller frames).  A half window of 1 needs no tile: four taps
+// a pixel from memory, 42 us instead of 56.
+constexpr int TRI_SMALL_S = 8;
+
 cudaError_t trilateral(const float* U, const float* V, const float* Um, const float* Vm,
                        const float* I, float* Uo, float* Vo, int sx, int sy, int s,
                        float sigmaEPE2, float sigmaI2, float sigmaS2, bool chained, cudaStream_t st)
 {
     const TriCoef tc = tri_coef(sigmaEPE2, sigmaI2, sigmaS2);
     const float cE = tc.cE, cI = tc.cI, cS = tc.cS;
-    if (s <= TRI_MAX_S) {
+    if (s > 1 && s <= TRI_MAX_S) {
         cudaError_t e = ensure_trilateral_smem(s);
         if (e != cudaSuccess) return e;
-        auto by_rows = [&](auto kernel, int ty) {
+        auto by_rows = [&](auto kernel, int ty, int groups) {
             dim3 g((sx + TX - 1) / TX, (sy + tri_rows(ty) - 1) / tri_rows(ty));
-            return launch(kernel, g, dim3(TX, ty, TRI_G), tri_smem_bytes(s, ty), chained, st, U, V, Um, Vm, I, Uo, Vo, sx, sy,
-                          s, tc.kE, tc.kI, cS);
+            return launch(kernel, g, dim3(TX, ty, groups), tri_smem_bytes(s, ty), chained, st, U, V, Um, Vm, I, Uo, Vo, sx,
+                          sy, s, tc.kE, tc.kI, cS);
         };
         int sms = 0;
         e = sm_count(&sms);
         if (e != cudaSuccess) return e;
         switch (trilateral_rows(sx, sy, s, sms)) {
-        case 2: return by_rows(k_trilateral<2>, 2);
-        case 4: return by_rows(k_trilateral<4>, 4);
-        default: return by_rows(k_trilateral<8>, 8);
+        case 2: return by_rows(k_trilateral<2, TRI_G>, 2, TRI_G);
+        case 4: return by_rows(k_trilateral<4, TRI_G>, 4, TRI_G);
+        default: return s <= TRI_SMALL_S ? by_rows(k_trilateral<4, 1>, 4, 1) : by_rows(k_trilateral<8, TRI_G>, 8, TRI_G);
         }
     }
     return launch(k_trilateral_global, grid2d(sx, sy), dim3(TX, TY), 0, chained, st, U, V, Um, Vm, I, Uo, Vo, sx, sy, s, cE,

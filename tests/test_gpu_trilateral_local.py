@@ -101,3 +101,24 @@ def test_far_centres(bad):
         assert np.abs(out - clean)[:, near & ~own].max() <= 1.0 and np.isfinite(out).all()
     else:
         assert np.isnan(out[0][near]).all() and np.isnan(out[1, y, x])
+
+
+@pytest.mark.parametrize("sS", [0.3, 0.7, 1.1, 1.9, 3.1, 3.5, 6.3])   # half windows 1 to 16
+def test_block_shapes_agree(sS):
+    """A crop's outputs, whose windows lie inside it, are those of the large frame: blocks of
+    8, 16 and 32 rows, one and two groups of columns.  (Crops start at a multiple of the four
+    rows a thread owns: which rows of a window pair up follows the row's number.)"""
+    rng = np.random.default_rng(11)
+    W, H, w, h = 1024, 352, 96, 72
+    U = (rng.normal(0, 0.4, (H, W)) + np.linspace(-9, 9, W)[None, :]).astype(np.float32)
+    V = rng.normal(3, 0.4, (H, W)).astype(np.float32)
+    I = random_image(rng, W, H)
+    s = _half_window(sS)
+    big = _refine(U, V, I, sS)
+    for x0, y0 in ((101, 64), (700, 132)):
+        part = _refine(*(a[y0:y0 + h, x0:x0 + w] for a in (U, V, I)), sS)
+        inner = (slice(None), slice(s, h - s), slice(s, w - s))
+        assert np.array_equal(part[inner], big[:, y0:y0 + h, x0:x0 + w][inner])
+    for r0 in (0, 171, H - 2):
+        eu, ev = trilateral_f64(U, V, U, V, I, r0, 2, s, 0.4, 0.1, sS)
+        assert np.abs(big[0, r0:r0 + 2] - eu).max() <= 1e-5 and np.abs(big[1, r0:r0 + 2] - ev).max() <= 1e-5
