@@ -139,6 +139,7 @@ def _declare(lib):
         "bm_batch_autotune": (c.c_int, [c.c_void_p, c.c_char_p, c.c_int, c.c_char_p, c.c_size_t]),
         "bm_selftest_barrier": (c.c_int, [c.c_uint32, c.c_uint32, c.c_uint64, P(c.c_int)]),
         "bm_debug_fail_alloc": (None, [c.c_uint64]),
+        "bm_debug_alloc_limit": (None, [c.c_uint64]),
         "bm_debug_alloc_count": (c.c_uint64, []),
         "bm_debug_live_allocs": (c.c_int64, []),
         "bm_debug_guard_bands": (None, [c.c_int]),

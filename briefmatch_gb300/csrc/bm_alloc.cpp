@@ -1,10 +1,11 @@
 // bm_alloc.cpp -- the engine's device allocator and its test hooks.
 //
 // Every device allocation of the contexts, batches and proposal networks goes
-// through device_malloc / device_free.  Two host-only test hooks sit on that path,
+// through device_malloc / device_free.  Three host-only test hooks sit on that path,
 // both off unless a test turns them on:
 //  - bm_debug_fail_alloc(k): the k-th allocation from then on fails as if the device
 //    were out of memory (the path a real cudaMalloc failure takes);
+//  - bm_debug_alloc_limit(bytes): larger allocations fail in the same way;
 //  - bm_debug_guard_bands(on): allocations made while it is on carry 256-byte guard
 //    bands before and after the buffer, filled with a known byte; bm_debug_check_guards
 //    reads every live band back and reports the first one a kernel overwrote.
@@ -27,20 +28,21 @@ constexpr unsigned char kGuardByte = 0xA5;
 std::atomic<uint64_t> g_allocs{0};
 std::atomic<int64_t> g_live{0};           // allocations made and not yet freed
 std::atomic<uint64_t> g_fail_at{0};       // absolute allocation number that fails, 0 = none
+std::atomic<uint64_t> g_limit{0};         // largest allocation that works, 0 = any
 std::atomic<int> g_guard_on{0};
 std::mutex g_mu;
 std::map<void*, size_t> g_guarded;        // user pointer -> user bytes
 
 }  // namespace
 
-namespace bmk {
+namespace {
 
-cudaError_t device_malloc(void** p, size_t bytes)
+// One attempt at one allocation.
+cudaError_t attempt(void** p, size_t bytes)
 {
     *p = nullptr;
-    const uint64_t k = ++g_allocs;
-    const uint64_t fail = g_fail_at.load();
-    if (fail && k == fail) return cudaErrorMemoryAllocation;
+    const uint64_t limit = g_limit.load();
+    if (limit && bytes > limit) return cudaErrorMemoryAllocation;
     if (!g_guard_on.load()) {
         const cudaError_t e = cudaMalloc(p, bytes);
         if (e == cudaSuccess) ++g_live;
@@ -65,6 +67,32 @@ cudaError_t device_malloc(void** p, size_t bytes)
     return cudaSuccess;
 }
 
+}  // namespace
+
+namespace bmk {
+
+cudaError_t device_malloc_or(void** p, size_t bytes, size_t least, size_t* got)
+{
+    *p = nullptr;
+    *got = bytes;
+    const uint64_t k = ++g_allocs;
+    const uint64_t fail = g_fail_at.load();
+    if (fail && k == fail) return cudaErrorMemoryAllocation;
+    cudaError_t e = attempt(p, bytes);
+    if (e == cudaErrorMemoryAllocation && least < bytes) {
+        cudaGetLastError();   // (the next launch's check would find the failure)
+        *got = least;
+        e = attempt(p, least);
+    }
+    return e;
+}
+
+cudaError_t device_malloc(void** p, size_t bytes)
+{
+    size_t got = 0;
+    return device_malloc_or(p, bytes, bytes, &got);
+}
+
 void device_free(void* p)
 {
     if (!p) return;
@@ -86,6 +114,8 @@ void device_free(void* p)
 extern "C" {
 
 void bm_debug_fail_alloc(uint64_t k) { g_fail_at = k ? g_allocs.load() + k : 0; }
+
+void bm_debug_alloc_limit(uint64_t bytes) { g_limit = bytes; }
 
 uint64_t bm_debug_alloc_count(void) { return g_allocs.load(); }
 

@@ -78,15 +78,19 @@ struct bm_ctx {
     float* d_up = nullptr;   // dense up-sampled image (BM_BUF_UP), filled on request
     // working up-sampled image with an edge-replicated margin of up_margin pixels on
     // every side (at least the pattern's largest offset), row pitch up_pitch(), followed
-    // by its key image (upad_keys())
+    // by its key image (upad_keys()) unless the device had no room for one
     float* d_upad = nullptr;
+    bool upad_keyed = false;
     int up_margin = 0;
     bool upad_valid = false;   // d_upad holds the current frame
     bool upad_use = false;     // frames are re-sampled and the pattern fits the key image
     int up_pitch() const { return (int)prm.sx + 2 * up_margin; }
     size_t upad_count(size_t m) const { return (prm.sx + 2 * m) * (prm.sy + 2 * m); }
     float* upad_origin() const { return d_upad + (size_t)up_margin * up_pitch() + up_margin; }
-    uint32_t* upad_keys() const { return reinterpret_cast<uint32_t*>(d_upad + upad_count(up_margin)); }
+    uint32_t* upad_keys() const
+    {
+        return upad_keyed ? reinterpret_cast<uint32_t*>(d_upad + upad_count(up_margin)) : nullptr;
+    }
     uint32_t* d_feat[2] = {nullptr, nullptr};
     int feat1 = 0;                           // d_feat[feat1] is FEAT1, d_feat[feat1^1] FEAT2
     uint32_t* d_flow[2] = {nullptr, nullptr};
@@ -451,15 +455,19 @@ bm_status set_pattern_impl(bm_ctx* c, const float* h_pattern)
     // working image stay in effect)
     if (use && (!c->d_upad || rmax > c->up_margin)) {
         float* fresh = nullptr;
-        const bm_status st = dev_alloc(&fresh, 2 * c->upad_count(rmax));
-        if (st != BM_OK) return st;
-        const cudaError_t e = cudaStreamSynchronize(c->stream);
+        const size_t image = c->upad_count(rmax) * sizeof(float);
+        size_t got = 0;
+        cudaError_t e = bmk::device_malloc_or((void**)&fresh, 2 * image, image, &got);
+        if (e != cudaSuccess)
+            return fail(BM_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", image, cudaGetErrorString(e));
+        e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) {
             bmk::device_free(fresh);
             return fail(BM_ERR_CUDA, "bm_set_pattern: %s", cudaGetErrorString(e));
         }
         if (c->d_upad) bmk::device_free(c->d_upad);
         c->d_upad = fresh;
+        c->upad_keyed = got > image;
         c->up_margin = rmax;
         c->upad_valid = false;
     }

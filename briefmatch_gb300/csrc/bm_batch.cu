@@ -41,7 +41,8 @@ struct PairDev {
     const uint8_t* frame[2];
     float* guide;          // frame 0 as float (the trilateral guide)
     float* up;             // up-sampled frame: dense sx*sy, or edge-replicated (below)
-    int up_margin;         // margin the up buffer has room for: (sx+2m)*(sy+2m) floats, then as many key words
+    int up_margin;         // margin the up buffer has room for: (sx+2m)*(sy+2m) floats
+    uint32_t* keys;        // its key image, as large; null where memory is short and for pairs not re-sampled
     uint32_t* F[2];
     uint32_t* flow[2];
     uint16_t* cost;
@@ -422,10 +423,9 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
     const bool padded = resample && d.rmax <= d.up_margin && key_image_fits(d.up_margin, pitch);
     for (int which = 0; which < 2; which++) {
         if (padded) {
-            uint32_t* keys = reinterpret_cast<uint32_t*>(d.up + (size_t)pitch * (d.sy + 2 * d.up_margin));
-            BB_CUDA(upsample_u8_pad(d.frame[which], which == 0 ? d.guide : nullptr, d.up, keys, pitch, d.up_margin,
+            BB_CUDA(upsample_u8_pad(d.frame[which], which == 0 ? d.guide : nullptr, d.up, d.keys, pitch, d.up_margin,
                                     d.sx_in, d.sy_in, d.sx, d.sy, d.lx, d.ix, d.ly, d.iy, st));
-            BB_CUDA(features_keys(keys, d.up, pitch, d.F[which], d.sx, d.sy, (int)b->nsp, b->pattern_off_pad[j], rev,
+            BB_CUDA(features_keys(d.keys, d.up, pitch, d.F[which], d.sx, d.sy, (int)b->nsp, b->pattern_off_pad[j], rev,
                                   false, st));
         } else {
             if (which == 0) BB_CUDA(u8_to_f32(d.frame[0], d.guide, ni, st));
@@ -832,7 +832,7 @@ bm_status bm_batch_create(const bm_params* pairs, uint32_t count, bm_batch** out
 
     // layout
     struct Off {
-        size_t frame[2], guide, up, F[2], flow[2], cost, fin, fmed, fout, tmp, pat, off, taps, lx, ix, ly, iy, nnx, nny;
+        size_t frame[2], guide, up, keys, F[2], flow[2], cost, fin, fmed, fout, tmp, pat, off, taps, lx, ix, ly, iy, nnx, nny;
     };
     std::vector<Off> offs(count);
     size_t cursor = 0;
@@ -879,7 +879,7 @@ bm_status bm_batch_create(const bm_params* pairs, uint32_t count, bm_batch** out
         const size_t n = (size_t)p.sx * p.sy, ni = (size_t)p.sx_in * p.sy_in;
         Off& o = offs[i];
         o.guide = take(ni * 4);
-        o.up = take(2 * (p.sx + 2 * (size_t)margin[i]) * (p.sy + 2 * (size_t)margin[i]) * 4);
+        o.up = take((p.sx + 2 * (size_t)margin[i]) * (p.sy + 2 * (size_t)margin[i]) * 4);
         o.F[0] = take(n * b->nsp * 4);
         o.F[1] = take(n * b->nsp * 4);
         o.flow[0] = take(n * 4);
@@ -898,12 +898,19 @@ bm_status bm_batch_create(const bm_params* pairs, uint32_t count, bm_batch** out
         o.nnx = take((size_t)p.sx_in * 4);
         o.nny = take((size_t)p.sy_in * 4);
     }
-    b->arena_bytes = cursor;
-    cudaError_t e = bmk::device_malloc((void**)&b->arena, b->arena_bytes);
+    // the key images last: a device without room for them takes the batch without
+    const size_t unkeyed = cursor;
+    for (uint32_t i = 0; i < count; i++) {
+        const bm_params& p = pairs[i];
+        if (p.sx != p.sx_in || p.sy != p.sy_in)
+            offs[i].keys = take((p.sx + 2 * (size_t)margin[i]) * (p.sy + 2 * (size_t)margin[i]) * 4);
+    }
+    cudaError_t e = bmk::device_malloc_or((void**)&b->arena, cursor, unkeyed, &b->arena_bytes);
     if (e != cudaSuccess) {
         delete b;
-        return bfail(BM_ERR_NOMEM, "bm_batch_create: cudaMalloc of %zu bytes failed: %s", cursor, cudaGetErrorString(e));
+        return bfail(BM_ERR_NOMEM, "bm_batch_create: cudaMalloc of %zu bytes failed: %s", unkeyed, cudaGetErrorString(e));
     }
+    const bool keyed = b->arena_bytes == cursor;
     e = cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         bmk::device_free(b->arena);
@@ -955,6 +962,7 @@ bm_status bm_batch_create(const bm_params* pairs, uint32_t count, bm_batch** out
         d.guide = reinterpret_cast<float*>(A + o.guide);
         d.up = reinterpret_cast<float*>(A + o.up);
         d.up_margin = margin[i];
+        d.keys = keyed && (d.sx != d.sx_in || d.sy != d.sy_in) ? reinterpret_cast<uint32_t*>(A + o.keys) : nullptr;
         d.F[0] = reinterpret_cast<uint32_t*>(A + o.F[0]);
         d.F[1] = reinterpret_cast<uint32_t*>(A + o.F[1]);
         d.flow[0] = reinterpret_cast<uint32_t*>(A + o.flow[0]);

@@ -15,6 +15,8 @@ void set_error_text(const char* msg);
 // The engine's device allocator (bm_alloc.cpp): cudaMalloc/cudaFree behind the test
 // hooks bm_debug_fail_alloc and bm_debug_guard_bands.
 cudaError_t device_malloc(void** p, size_t bytes);
+// `bytes`, or `least` where the device has no room for more; *got is the one it was.
+cudaError_t device_malloc_or(void** p, size_t bytes, size_t least, size_t* got);
 void device_free(void* p);
 
 // Random-search stream position for one launch (briefmatch_cuda.cu:237-241).
@@ -49,8 +51,8 @@ cudaError_t upsample_u8(const uint8_t* in, float* out, int sxi, int syi, int sxo
 // Up-sampling into an image with an edge-replicated margin of m pixels on every
 // side; `out` is the start of the (sxo + 2m) x (syo + 2m) buffer, row pitch `pitch`.
 // `keys`, of the same shape, receives the 16-bit keys the descriptors compare first: per
-// word the pixel's key and that of the pixel below it.  `frame`, unless null, receives the
-// input frame as float.
+// word the pixel's key and that of the pixel below it (null: no keys).  `frame`, unless
+// null, receives the input frame as float.
 cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_t* keys, int pitch, int m, int sxi,
                             int syi, int sxo, int syo, const float* lx, const int* ix, const float* ly, const int* iy,
                             cudaStream_t st);
@@ -83,7 +85,8 @@ bool key_image_fits(int m, int pitch);
 // (the stages of one frame in a row); this one may then start under its last blocks.
 
 // Descriptors from an edge-replicated image and its keys (upsample_u8_pad): both point
-// at the start of the margin, which is no narrower than the largest pattern offset.
+// at the start of the margin, which is no narrower than the largest pattern offset.  Without
+// keys (null) every pair is compared on the float image.
 cudaError_t features_keys(const uint32_t* keys, const float* up, int pitch, uint32_t* F, int sx, int sy, int nsp,
                           const KeyOffsets& ko, int rev, bool chained, cudaStream_t st);
 

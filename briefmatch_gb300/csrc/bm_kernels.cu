@@ -90,8 +90,9 @@ __global__ void __launch_bounds__(256) k_upsample(const T* __restrict__ in, floa
 //
 // Beside the float image the kernel writes the key image the descriptors read: a word
 // per pixel with the 16-bit key (sample_key) of the pixel in its low half and of the
-// pixel below it in its high half.  A thread pairs the keys of its own rows; the word
-// that spans two threads' rows is written as two halves.  Beside that
+// pixel below it in its high half (if it has one: it may be missing where memory is short).
+// A thread pairs the keys of its own rows; the word that spans two threads' rows is written
+// as two halves.  Beside that
 // the threads write the frame itself as float into `frame` (if any), for the refinement:
 // 2 us at 1024x436 where a launch of its own took 4 to 6.  (Extra blocks for it: as fast
 // on large frames, 4 us slower on small ones.)
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(TX * TY, 2) k_upsample_pad_rows(const uint8_t*
         const size_t o = X + (size_t)Y * pitch;
         out[o] = val;
         const uint32_t key = sample_key(val);
+        if (!keys) continue;
         if (r > 0)
             keys[o - pitch] = key_above | (key << 16);
         else if (Y > 0)
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(256) k_features(const float* __restrict__ I, u
 // pair in a thousand ties and each lane repairs its own; saturated or flat parts tie
 // throughout, and there (a lane with more than MANY_TIES) the warp goes sample by
 // sample, and past FLAT_TIES samples of a word reads the next words of the chunk from
-// the float image outright.
+// the float image outright (as it does throughout when there is no key image).
 //
 // Reading two keys per 4 bytes halves the load requests that bound the float form
 // (70 % of the load unit's rate, and 13 % of its instructions branches around the
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(256, 6) k_features_keys(const uint32_t* W, con
 #pragma unroll 1
     for (int c = 0; c < NSP / CW; c++) {
         uint32_t word[2][CW];
-        bool flat = false;
+        bool flat = W == nullptr;
 #pragma unroll
         for (int wd = 0; wd < CW; wd++) {
             const int w = c * CW + wd;

@@ -295,6 +295,8 @@ bm_status bm_selftest_barrier(uint32_t blocks, uint32_t expect, uint64_t spin_li
 /* The k-th device allocation of the library from now on fails as if the device were
  * out of memory (k = 0: none fails). */
 void bm_debug_fail_alloc(uint64_t k);
+/* Allocations of more than `bytes` fail in the same way (0 = off). */
+void bm_debug_alloc_limit(uint64_t bytes);
 /* Device allocations made so far, and those made and not yet freed. */
 uint64_t bm_debug_alloc_count(void);
 int64_t bm_debug_live_allocs(void);
