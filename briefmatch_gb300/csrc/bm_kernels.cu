@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(256) k_upsample(const T* __restrict__ in, floa
 // the threads write the frame itself as float into `frame` (if any), for the refinement:
 // 2 us at 1024x436 where a launch of its own took 4 to 6.  (Extra blocks for it: as fast
 // on large frames, 4 us slower on small ones.)
-template <int UP_R>
+template <int UP_R, bool KEYS>
 __global__ void __launch_bounds__(TX * TY, 2) k_upsample_pad_rows(const uint8_t* __restrict__ in, float* __restrict__ frame,
                                                                float* __restrict__ out,
                                                                uint32_t* __restrict__ keys, int pitch, int m, int sxi,
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(TX * TY, 2) k_upsample_pad_rows(const uint8_t*
         const size_t o = X + (size_t)Y * pitch;
         out[o] = val;
         const uint32_t key = sample_key(val);
-        if (!keys) continue;
+        if constexpr (!KEYS) continue;
         if (r > 0)
             keys[o - pitch] = key_above | (key << 16);
         else if (Y > 0)
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256) k_features(const float* __restrict__ I, u
 // pair in a thousand ties and each lane repairs its own; saturated or flat parts tie
 // throughout, and there (a lane with more than MANY_TIES) the warp goes sample by
 // sample, and past FLAT_TIES samples of a word reads the next words of the chunk from
-// the float image outright (as it does throughout when there is no key image).
+// the float image outright.
 //
 // Reading two keys per 4 bytes halves the load requests that bound the float form
 // (70 % of the load unit's rate, and 13 % of its instructions branches around the
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(256, 6) k_features_keys(const uint32_t* W, con
 #pragma unroll 1
     for (int c = 0; c < NSP / CW; c++) {
         uint32_t word[2][CW];
-        bool flat = W == nullptr;
+        bool flat = false;
 #pragma unroll
         for (int wd = 0; wd < CW; wd++) {
             const int w = c * CW + wd;
@@ -320,6 +320,35 @@ __global__ void __launch_bounds__(256, 6) k_features_keys(const uint32_t* W, con
         }
         store_desc<CW>(F + ((size_t)y * sx + x) * NSP + c * CW, word[0]);
         if (second) store_desc<CW>(F + ((size_t)(y + 1) * sx + x) * NSP + c * CW, word[1]);
+    }
+}
+
+// The same without a key image (memory is short): every pair on the float image.  A kernel
+// of its own, as another branch to the float image costs the one above 1-3 % of its time.
+template <int NSP>
+__global__ void __launch_bounds__(256) k_features_float(const float* I, int pitch, uint32_t* __restrict__ F, int sx, int sy,
+                                                        const __grid_constant__ KeyOffsets po, int rev)
+{
+    chain_wait();
+    chain_trigger();
+    int bx = blockIdx.x, by = blockIdx.y;
+    if (rev) {
+        bx = gridDim.x - 1 - bx;
+        by = gridDim.y - 1 - by;
+    }
+    const int x = bx * TX + threadIdx.x, y = by * TY + threadIdx.y;
+    if (x >= sx || y >= sy) return;
+    const char* base = reinterpret_cast<const char*>(I + ((size_t)y * pitch + x));
+    uint32_t* out = F + ((size_t)y * sx + x) * NSP;
+#pragma unroll 1
+    for (int w = 0; w < NSP; w++) {
+        uint32_t bits = 0;
+#pragma unroll
+        for (int b = 0; b < 32; b++) {
+            const uint2 o = po.off[w * 32 + b];
+            if (*reinterpret_cast<const float*>(base + o.x) > *reinterpret_cast<const float*>(base + o.y)) bits |= 1u << b;
+        }
+        out[w] = bits;
     }
 }
 
@@ -638,9 +667,10 @@ cudaError_t upsample_u8_pad(const uint8_t* in, float* frame, float* out, uint32_
         kernel<<<g, dim3(TX, TY), 0, st>>>(in, frame, out, keys, pitch, m, sxi, syi, sxo, syo, lx, ix, ly, iy);
     };
     const long columns = (sxo + 2 * m + TX - 1) / TX, eights = (syo + 2 * m + TY - 1) / TY;
-    if (columns * eights >= 8L * sms) rows(k_upsample_pad_rows<8>, 8);
-    else if (columns * eights >= 4L * sms) rows(k_upsample_pad_rows<4>, 4);
-    else rows(k_upsample_pad_rows<2>, 2);
+    if (!keys) rows(k_upsample_pad_rows<8, false>, 8);   // memory is short
+    else if (columns * eights >= 8L * sms) rows(k_upsample_pad_rows<8, true>, 8);
+    else if (columns * eights >= 4L * sms) rows(k_upsample_pad_rows<4, true>, 4);
+    else rows(k_upsample_pad_rows<2, true>, 2);
     return cudaGetLastError();
 }
 
@@ -683,6 +713,9 @@ void key_offsets(KeyOffsets& ko, const int4* pat, int N, int m, int pitch)
 cudaError_t features_keys(const uint32_t* keys, const float* up, int pitch, uint32_t* F, int sx, int sy, int nsp,
                           const KeyOffsets& ko, int rev, bool chained, cudaStream_t st)
 {
+    if (!keys) {
+        BM_DISPATCH_NSP(nsp, return launch(k_features_float<NSP>, grid2d(sx, sy), dim3(TX, TY), 0, chained, st, up, pitch, F, sx, sy, ko, rev));
+    }
     const dim3 g((sx + TX - 1) / TX, (sy + 2 * TY - 1) / (2 * TY));
     BM_DISPATCH_NSP(nsp, return launch(k_features_keys<NSP>, g, dim3(TX, TY), 0, chained, st, keys, up, pitch, F, sx, sy, ko, rev));
     return cudaSuccess;
