@@ -449,7 +449,7 @@ bm_status set_pattern_impl(bm_ctx* c, const float* h_pattern)
     }
     // the working up-sampled image's margin must cover the largest offset
     const bm_params& p = c->prm;
-    const bool use = (p.sx != p.sx_in || p.sy != p.sy_in) &&
+    const bool use = (p.sx != p.sx_in || p.sy != p.sy_in) && bmk::rows_slide((int)p.sy_in, (int)p.sy) &&
                      bmk::key_image_fits(std::max(rmax, c->up_margin), (int)p.sx + 2 * std::max(rmax, c->up_margin));
     // (the new image is allocated first: if that fails, the previous pattern and
     // working image stay in effect)

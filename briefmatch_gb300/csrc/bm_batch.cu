@@ -420,7 +420,7 @@ bm_status enqueue_pair(bm_batch* b, const bm_batch_schedule& s, int j, cudaStrea
     // descriptors from the edge-replicated up-sampled image while the pair's pattern
     // fits the margin its buffer was laid out with; from the dense image otherwise
     const int pitch = d.sx + 2 * d.up_margin;
-    const bool padded = resample && d.rmax <= d.up_margin && key_image_fits(d.up_margin, pitch);
+    const bool padded = resample && d.rmax <= d.up_margin && rows_slide(d.sy_in, d.sy) && key_image_fits(d.up_margin, pitch);
     for (int which = 0; which < 2; which++) {
         if (padded) {
             BB_CUDA(upsample_u8_pad(d.frame[which], which == 0 ? d.guide : nullptr, d.up, d.keys, pitch, d.up_margin,

@@ -79,6 +79,11 @@ void key_offsets(KeyOffsets& ko, const int4* pat, int N, int m, int pitch);
 // Whether every sample stays within 32-bit byte offsets (a margin of tens of thousands of
 // pixels does not); the dense image serves the others.
 bool key_image_fits(int m, int pitch);
+// Whether upsample_u8_pad's rows share most of their windows: where frames are reduced to less
+// than a seventh of their rows, every output's window is new, and sliding to it row by row
+// loads more than the window (1920x1080 u0.1 and u0.12: 40 and 34 us with the frame's
+// conversion, 16 and 16 by the dense image; at u0.15 sliding takes 25 and at u0.2 18).
+inline bool rows_slide(int syi, int syo) { return syi < 7 * (long)syo; }
 
 // `chained` in a launcher: the launch before it on the stream is a kernel that either was
 // launched unchained or itself waits for its predecessor before it lets the next start
