@@ -345,9 +345,9 @@ __device__ __forceinline__ void init_px(const uint32_t* F1, const uint32_t* F2,
 // temporal candidate when !first, exactly as init_px), then the network's proposal
 // for this pixel -- pred is [h4][w4][3] (u, v in quarter-resolution input pixels,
 // confidence logit) -- where its confidence logit reaches logit_min; the proposal
-// replaces the plain vector only if its Hamming cost is strictly lower.  Descriptors are
-// read through L2 (chained launch, as init_px).
-template <int NSP>
+// replaces the plain vector only if its Hamming cost is strictly lower.  CHAINED: as
+// init_px.
+template <int NSP, bool CHAINED>
 __device__ __forceinline__ void seed_px(const uint32_t* F1, const uint32_t* F2,
                                         const uint32_t* __restrict__ flow_prev, uint32_t* __restrict__ flow_out,
                                         uint16_t* __restrict__ cost, int sx, int sy, int first, int x, int y,
@@ -365,8 +365,8 @@ __device__ __forceinline__ void seed_px(const uint32_t* F1, const uint32_t* F2,
         ny = min(max(hi16(t), -y), sy - y - 1);
     }
     uint32_t f1[NSP];
-    load_desc<NSP, true>(f1, F1 + pix * NSP);
-    int h = hamming<NSP, true>(f1, F2 + (pix + nx + (long)ny * sx) * NSP);
+    load_desc<NSP, CHAINED>(f1, F1 + pix * NSP);
+    int h = hamming<NSP, CHAINED>(f1, F2 + (pix + nx + (long)ny * sx) * NSP);
     // quarter-resolution cell of this up-sampled pixel (scale = up-sampled px per
     // quarter-resolution px, inv = its reciprocal from the host, so the cell index
     // is one IEEE add and multiply: no approximate division)
@@ -377,7 +377,7 @@ __device__ __forceinline__ void seed_px(const uint32_t* F1, const uint32_t* F2,
         const int sxv = min(max(__float2int_rn(pr[0] * scale_x), -x), sx - x - 1);
         const int syv = min(max(__float2int_rn(pr[1] * scale_y), -y), sy - y - 1);
         if (sxv != nx || syv != ny) {
-            const int hs = hamming<NSP, true>(f1, F2 + (pix + sxv + (long)syv * sx) * NSP);
+            const int hs = hamming<NSP, CHAINED>(f1, F2 + (pix + sxv + (long)syv * sx) * NSP);
             if (hs < h) {
                 h = hs;
                 nx = sxv;
