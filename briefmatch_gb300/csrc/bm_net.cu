@@ -1382,9 +1382,11 @@ struct bm_net {
     CUtensorMap map_wf[NL];
     CUtensorMap map_wb[NL];
     uint32_t map_B = 0, map_h = 0, map_w = 0;
+    CUtensorMap map_fwd[NL];      // source rows of each layer's input
+    bool map_all = false;         // the following are encoded too (training, fused launch)
     CUtensorMap map_in;
     CUtensorMap map_act[NL - 1];
-    CUtensorMap map_fwd[NL], map_dy[NL];   // source rows of each layer's input and of its output gradient
+    CUtensorMap map_dy[NL];       // source rows of each layer's output gradient
     int num_sms = 1;
 };
 
@@ -1438,21 +1440,28 @@ bm_status check_dims(bm_net* n, uint32_t B, uint32_t h, uint32_t w)
 // backward pass alternates.
 constexpr int dy_slot(int l) { return (NL - 1 - l) & 1; }
 
-// Tensor maps of the activation buffers for a (B, h, w) call (host-side encoding only).
-bool ensure_act_maps(bm_net* n, uint32_t B, uint32_t h, uint32_t w)
+// Tensor maps of the activation buffers for a (B, h, w) call (host-side encoding only, about
+// 50 ns each): the six that a forward pass by layers reads, or `all` eighteen.
+bool ensure_act_maps(bm_net* n, uint32_t B, uint32_t h, uint32_t w, bool all)
 {
-    if (n->map_B == B && n->map_h == h && n->map_w == w) return true;
     const int Bi = (int)B, hi = (int)h, wi = (int)w;
-    bool ok = act_map(&n->map_in, n->d_in, Bi, hi, wi);
+    bool ok = true;
+    if (n->map_B != B || n->map_h != h || n->map_w != w) {
+        n->map_B = 0;
+        n->map_all = false;
+        for (int l = 0; ok && l < NL; l++) ok = row_map(&n->map_fwd[l], l ? n->d_act[l - 1] : n->d_in, Bi, hi, wi, DIL[l]);
+        if (!ok) return false;
+        n->map_B = B;
+        n->map_h = h;
+        n->map_w = w;
+    }
+    if (!all || n->map_all) return true;
+    ok = act_map(&n->map_in, n->d_in, Bi, hi, wi);
     for (int l = 0; ok && l < NL - 1; l++) ok = act_map(&n->map_act[l], n->d_act[l], Bi, hi, wi);
-    for (int l = 0; ok && l < NL; l++) ok = row_map(&n->map_fwd[l], l ? n->d_act[l - 1] : n->d_in, Bi, hi, wi, DIL[l]);
     for (int l = 0; ok && l < NL; l++)
         ok = row_map(&n->map_dy[l], n->d_dy[dy_slot(l)], Bi, hi, wi, DIL[l], l == NL - 1 ? 16 : 32);
-    if (!ok) return false;
-    n->map_B = B;
-    n->map_h = h;
-    n->map_w = w;
-    return true;
+    n->map_all = ok;
+    return ok;
 }
 
 bm_status forward(bm_net* n, uint32_t B, uint32_t h, uint32_t w, cudaStream_t st)
@@ -1463,7 +1472,7 @@ bm_status forward(bm_net* n, uint32_t B, uint32_t h, uint32_t w, cudaStream_t st
     }
     const int Bi = (int)B, hi = (int)h, wi = (int)w;
     if (n->umma) {
-        if (!ensure_act_maps(n, B, h, w)) return nfail(BM_ERR_CUDA, "bm_net: tensor map encoding failed");
+        if (!ensure_act_maps(n, B, h, w, n->fused)) return nfail(BM_ERR_CUDA, "bm_net: tensor map encoding failed");
         if (n->fused) {
             NetFusedArgs a;
             for (int l = 0; l < NL; l++) {
@@ -1802,6 +1811,7 @@ bm_status bm_net_train_step(bm_net* n, uint32_t B, uint32_t h, uint32_t w, const
     cudaStream_t st = (cudaStream_t)stream;
     s = forward(n, B, h, w, st);
     if (s != BM_OK) return s;
+    if (n->umma && !ensure_act_maps(n, B, h, w, true)) return nfail(BM_ERR_CUDA, "bm_net: tensor map encoding failed");
     const size_t px = (size_t)B * h * w;
     const int Bi = (int)B, hi = (int)h, wi = (int)w;
     BN_CUDA(cudaMemsetAsync(n->d_grad, 0, n->nparam * 4, st));
