@@ -35,7 +35,7 @@ using namespace bmk::dev;
 struct PairDev {
     int sx, sy, sx_in, sy_in;
     int P, fsize, tri_s, rmax;
-    float dist, mx, my, cE, cI, cS;
+    float dist, mx, my;
     int first_up_tile_x;   // tiles per row on the up-sampled grid
     int first_in_tile_x;   // tiles per row at input resolution (32x8)
     const uint8_t* frame[2];
@@ -947,10 +947,6 @@ bm_status bm_batch_create(const bm_params* pairs, uint32_t count, bm_batch** out
         d.dist = std::sqrt(std::ceil((float)p.sx * 0.5f / 3.0f));
         d.mx = (float)p.sx_in / (float)p.sx;
         d.my = (float)p.sy_in / (float)p.sy;
-        const TriCoef tc = tri_coef(p.sEPE * p.sEPE, p.sI * p.sI, p.sS * p.sS);
-        d.cE = tc.cE;
-        d.cI = tc.cI;
-        d.cS = tc.cS;
         d.first_up_tile_x = (d.sx + TX - 1) / TX;
         d.first_in_tile_x = (d.sx_in + TX - 1) / TX;
         b->pre_up[j + 1] = b->pre_up[j] + (unsigned)(d.first_up_tile_x * ((d.sy + TY - 1) / TY));
