@@ -1080,6 +1080,7 @@ bm_status bm_batch_set_pattern(bm_batch* b, uint32_t pair, const float* h_patter
         off[s] = make_int2(v[0] + v[1] * sx, v[2] + v[3] * sx);
     }
     d.rmax = rmax;
+    destroy_graph(b);   // the offsets are parameters of the captured launches
     if (b->pattern_off.size() != b->count) b->pattern_off.resize(b->count);
     if (b->pattern_off_pad.size() != b->count) b->pattern_off_pad.resize(b->count);
     std::memcpy(b->pattern_off[j].off, off.data(), sizeof(b->pattern_off[j].off));
