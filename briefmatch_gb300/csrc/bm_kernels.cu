@@ -552,25 +552,35 @@ __global__ void __launch_bounds__(256) k_trilateral_global(const float* __restri
     if (x >= sx || y >= sy) return;
     const size_t o = (size_t)x + (size_t)y * sx;
     const float um0 = Um[o], vm0 = Vm[o], I0 = I[o];
-    // sums relative to the centre, as trilateral_block's
-    const float bu = fabsf(um0) <= TRI_FAR ? um0 : 0.0f, bv = fabsf(vm0) <= TRI_FAR ? vm0 : 0.0f;
+    // sums of the differences to the centre, as trilateral_block's; of the flow itself where
+    // that is far
+    const bool far_u = fabsf(um0) > TRI_FAR, far_v = fabsf(vm0) > TRI_FAR;
     float uf = 0.0f, vf = 0.0f, W = 0.0f;
-    for (int i = -s; i < s; i++) {
-        const int gx = min(sx - 1, max(0, x + i));
-        const float si = (float)(i * i) * cS;
-        for (int j = -s; j < s; j++) {
-            const size_t g = (size_t)gx + (size_t)min(sy - 1, max(0, y + j)) * sx;
-            const float u1 = __ldg(U + g), v1 = __ldg(V + g);
-            const float dI = __ldg(I + g) - I0;
-            const float du = u1 - um0, dv = v1 - vm0;
-            const float e = du * du + dv * dv;
-            const float sp = si + (float)(j * j) * cS;
-            const float w = exp2f(fmaf(e, -cE, fmaf(dI * dI, -cI, -sp)));
-            uf = fmaf(w, u1 - bu, uf);
-            vf = fmaf(w, v1 - bv, vf);
-            W += w;
+    auto walk = [&](auto flow) {
+        constexpr bool FLOW = decltype(flow)::value;
+        for (int i = -s; i < s; i++) {
+            const int gx = min(sx - 1, max(0, x + i));
+            const float si = (float)(i * i) * cS;
+            for (int j = -s; j < s; j++) {
+                const size_t g = (size_t)gx + (size_t)min(sy - 1, max(0, y + j)) * sx;
+                const float u1 = __ldg(U + g), v1 = __ldg(V + g);
+                const float dI = __ldg(I + g) - I0;
+                const float du = u1 - um0, dv = v1 - vm0;
+                const float e = du * du + dv * dv;
+                const float sp = si + (float)(j * j) * cS;
+                const float w = exp2f(fmaf(e, -cE, fmaf(dI * dI, -cI, -sp)));
+                uf = fmaf(w, FLOW && far_u ? u1 : du, uf);
+                vf = fmaf(w, FLOW && far_v ? v1 : dv, vf);
+                W += w;
+            }
         }
+    };
+    walk(std::false_type{});
+    if (far_u || far_v) {
+        uf = vf = W = 0.0f;
+        walk(std::true_type{});
     }
+    const float bu = far_u ? 0.0f : um0, bv = far_v ? 0.0f : vm0;
     Uo[o] = W < 1e-5f ? fmaf(bu, W, uf) / 1e-5f : bu + uf / W;
     Vo[o] = W < 1e-5f ? fmaf(bv, W, vf) / 1e-5f : bv + vf / W;
 }

@@ -122,3 +122,24 @@ def test_block_shapes_agree(sS):
     for r0 in (0, 171, H - 2):
         eu, ev = trilateral_f64(U, V, U, V, I, r0, 2, s, 0.4, 0.1, sS)
         assert np.abs(big[0, r0:r0 + 2] - eu).max() <= 1e-5 and np.abs(big[1, r0:r0 + 2] - ev).max() <= 1e-5
+
+
+def test_window_without_a_tile():
+    """Half windows past the largest tile: small flows beside fast ones, and far centres."""
+    W, H, sS = 150, 110, 21.5
+    rng = np.random.default_rng(5)
+    obj = _bad(W, H, 2)
+    U = np.where(obj, 500.0, 0.01 + rng.uniform(-0.005, 0.005, (H, W))).astype(np.float32)
+    V = np.where(obj, -40.0, 0.01 + rng.uniform(-0.005, 0.005, (H, W))).astype(np.float32)
+    I = random_image(rng, W, H)
+    s = _half_window(sS)
+    assert s > 52
+    out = _refine(U, V, I, sS)
+    eu, ev = trilateral_f64(U, V, U, V, I, 54, 3, s, 0.4, 0.1, sS)
+    back = ~obj[54:57]
+    # the sums run over the whole window, 11,000 taps one after the other: 2^-24 each at worst
+    tol = 2.0 ** -24 * 0.02 + 11000 * 2.0 ** -24 * 0.01
+    assert np.abs(out[0, 54:57] - eu)[back].max() <= tol and np.abs(out[1, 54:57] - ev)[back].max() <= tol
+    U[55, 70] = 2e38
+    out = _refine(U, V, I, sS)
+    assert out[0, 55, 70] == np.float32(2e38) and np.isfinite(out).all()
