@@ -500,10 +500,9 @@ __device__ __forceinline__ void jump_candidates(const uint32_t* flow_in, uint32_
 // Descriptors of up to 16 bytes: one thread reads its pixel's descriptor and its
 // candidates' whole; a thread without a live candidate reads none.  The level is bound
 // by the L1 data pipe (a gather of 32 scattered 16-byte vectors takes ~18 wavefronts)
-// with the integer pipe next to it: 32-bit indices, clamps on 16-bit pairs and gathers
-// without zero-fill took the integer pipe from 74 % to 52 % and a level at 1024x436
-// u2.9 N128 from 42.0 to 36.8 us (67.1 to 56.9 with the random search, whose state
-// now stays in registers).
+// with the integer pipe next to it: 32-bit indices and clamps on 16-bit pairs took the
+// integer pipe from 74 % to 52 % and a level at 1024x436 u2.9 N128 from 42.0 to 36.8 us
+// (67.1 to 56.9 with the random search, whose state now stays in registers).
 template <int NSP, bool RS, bool INLAUNCH = false>
 __device__ __forceinline__ void jump_px(const uint32_t* __restrict__ F1, const uint32_t* __restrict__ F2,
                                         const uint32_t* flow_in, uint32_t* flow_out, uint16_t* cost, int sx, int sy,
@@ -876,20 +875,21 @@ __device__ __forceinline__ void median2_px(const float* in, float* __restrict__ 
 // packed f32x2 registers hold the two rows, so a sample pair is used as it is read from
 // shared memory (the tile is stored column by column) and serves all four outputs.
 // TRI_G = 2 groups of TX x TY threads share a tile, each taking half of the window's
-// columns; their sums meet in shared memory (small windows: one group, G = 1).  The neighbourhood is staged with
-// clamp-to-edge addressing, `smem` must hold tri_smem_bytes(s, TY).
+// columns; their sums meet in shared memory (small windows: one group, G = 1).  The
+// neighbourhood is staged with clamp-to-edge addressing, `smem` must hold
+// tri_smem_bytes(s, TY).
 //
 // The three Gaussians are one exp2 of the summed exponents:
 // q = du^2 + dv^2 + dI^2 + j^2 cS over scaled differences (kE = sqrt(cE), kI = sqrt(cI)).
 // What is summed are the weighted differences du and dv to the output's own median value,
 // which is added back to the quotient: the sums are of small numbers whatever the flow is,
 // and a value depends on nothing outside its window.  The scaled centre's rounding is known
-// (one FMA) and taken off the quotient.  Against 64 bits that leaves an error of about half
-// a unit in the last place of the pixel's own flow: 3.0e-8 of the norm of a 1920x1080 field
-// (sums of the flow itself 2.1e-7).  Sums relative to one reference flow per block reach
-// 3.4e-8 there, but are up to 3e-4 px off at small flows beside a fast object (float32
-// restatement; these: 6e-10 px).  The column factor exp2(-cS i^2) is applied once per
-// column.  Nine FP32 lane operations per tap and output.
+// (one FMA) and taken off the quotient; what it moves the weights by stays.  Against 64 bits
+// that leaves an error of about half a unit in the last place of the pixel's own flow: 3.0 to
+// 3.8e-8 of the norm of 1920x1080 fields (sums of the flow itself 2.2e-7).  Sums relative to
+// one reference flow per block reach 3.1 to 3.5e-8 there, but are up to 3e-4 px off at small
+// flows beside a fast object (float32 restatement; these: 6e-10 px).  The column factor
+// exp2(-cS i^2) is applied once per column.  Nine FP32 lane operations per tap and output.
 //
 // What bounds it is the FP32 pipe's operand reads: a packed FMA with three different
 // 64-bit operands takes three cycles, with two it takes two (measured).  So differences
