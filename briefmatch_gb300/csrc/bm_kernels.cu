@@ -553,8 +553,8 @@ __global__ void __launch_bounds__(256) k_trilateral_global(const float* __restri
     const size_t o = (size_t)x + (size_t)y * sx;
     const float um0 = Um[o], vm0 = Vm[o], I0 = I[o];
     // sums of the differences to the centre, as trilateral_block's; of the flow itself where
-    // that is far
-    const bool far_u = fabsf(um0) > TRI_FAR, far_v = fabsf(vm0) > TRI_FAR;
+    // that is far or NaN (an empty window gives 0 all the same)
+    const bool far_u = !(fabsf(um0) <= TRI_FAR), far_v = !(fabsf(vm0) <= TRI_FAR);
     float uf = 0.0f, vf = 0.0f, W = 0.0f;
     auto walk = [&](auto flow) {
         constexpr bool FLOW = decltype(flow)::value;

@@ -143,3 +143,12 @@ def test_window_without_a_tile():
     U[55, 70] = 2e38
     out = _refine(U, V, I, sS)
     assert out[0, 55, 70] == np.float32(2e38) and np.isfinite(out).all()
+
+
+def test_empty_window():
+    """A spatial sigma whose square underflows leaves no taps: every sum is 0, and so is the
+    quotient with the floor of the weights, also at NaN and infinite centres."""
+    rng = np.random.default_rng(6)
+    U, V = (rng.normal(0, 3, (20, 35)).astype(np.float32) for _ in range(2))
+    U[3, 4], V[5, 6], U[7, 8] = np.nan, np.inf, 1e35
+    assert not _refine(U, V, random_image(rng, 35, 20), 1e-30).any()
