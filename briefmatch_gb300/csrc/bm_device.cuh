@@ -152,6 +152,7 @@ __device__ __forceinline__ f2x pk2(float a, float b) { f2x r; asm("mov.b64 %0, {
 __device__ __forceinline__ float lo2(f2x v) { return __uint_as_float((unsigned int)(v & 0xffffffffull)); }
 __device__ __forceinline__ float hi2(f2x v) { return __uint_as_float((unsigned int)(v >> 32)); }
 __device__ __forceinline__ f2x add2(f2x a, f2x b) { f2x d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f2x mul2(f2x a, f2x b) { f2x d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ f2x fma2(f2x a, f2x b, f2x c)
 {
     f2x d;
@@ -879,25 +880,31 @@ __device__ __forceinline__ void median2_px(const float* in, float* __restrict__ 
 // neighbourhood is staged with clamp-to-edge addressing, `smem` must hold
 // tri_smem_bytes(s, TY).
 //
-// The three Gaussians are one exp2 of the summed exponents:
-// q = du^2 + dv^2 + dI^2 + j^2 cS over scaled differences (kE = sqrt(cE), kI = sqrt(cI)).
+// The three Gaussians are one exp2 of the summed exponents,
+// r q = r (du^2 + dv^2 + dI^2 + j^2 cS / r) over scaled differences: kE is the power of two
+// nearest sqrt(cE), r = cE / kE^2 the factor that leaves, kI = sqrt(cI / r).  With it a flow's
+// scaled difference is exact but for one rounding: a scale that rounds, kE = sqrt(cE) and no
+// factor, saves the multiplication, but puts an error of q's size into the weights far from
+// the centre, and where only such are left (a sum of weights under the floor of 1e-5) the
+// output was up to 4e-4 px off at flows of 18 px.
+//
 // What is summed are the weighted differences du and dv to the output's own median value,
 // which is added back to the quotient: the sums are of small numbers whatever the flow is,
-// and a value depends on nothing outside its window.  The scaled centre's rounding is known
-// (one FMA) and taken off the quotient; what it moves the weights by stays.  Against 64 bits
-// that leaves an error of about half a unit in the last place of the pixel's own flow: 3.0 to
-// 3.8e-8 of the norm of 1920x1080 fields (sums of the flow itself 2.2e-7).  Sums relative to
-// one reference flow per block reach 3.1 to 3.5e-8 there, but are up to 3e-4 px off at small
-// flows beside a fast object (float32 restatement; these: 6e-10 px).  The column factor
-// exp2(-cS i^2) is applied once per column.  Nine FP32 lane operations per tap and output.
+// and a value depends on nothing outside its window.  Error against 64 bits: 2.6e-8 of the
+// norm of a 1920x1080 field, which is the rounding of the result (sums of the flow itself
+// 2.2e-7; sums relative to one reference flow per block 3.1 to 5.0e-8, but up to 3e-4 px off
+// at small flows beside a fast object, where these stay at 6e-10).  The column factor
+// exp2(-cS i^2) is applied once per column.  Ten FP32 lane operations per tap and output.
 //
 // What bounds it is the FP32 pipe's operand reads: a packed FMA with three different
-// 64-bit operands takes three cycles, with two it takes two (measured).  So differences
-// are additions, squares read one register twice, and only the two weighted sums need
-// three operands: 20 cycles per pair of taps, 18 by operation count.  1920x1080 with a
-// 94 x 94 window: 7.16 -> 5.61 ms; 1024x436 (48 x 48): 400 -> 344 us.  The tile's loads are
-// eight in flight per thread, the medians' before them; one after the other they took 0.1 ms
-// of the former, and half the time of small windows.
+// 64-bit registers takes three cycles, with two it takes two (measured; an operand that is
+// the same for the whole grid does not count).  So flow differences are additions, the
+// intensity's an FMA with the grid's scale, squares read one register twice, and only the two
+// weighted sums need three registers: 22 cycles per pair of taps, 20 by operation count.
+// 1920x1080 with a 94 x 94 window: 7.16 -> 6.12 ms; 1024x436 (48 x 48): 400 -> 372 us (without
+// the factor r 5.61 and 342).  The tile's loads are eight in flight per thread, the medians'
+// before them; one after the other they took 0.1 ms of the former, and half the time of
+// small windows.
 //
 // Flows beyond TRI_FAR of a standard deviation (and infinite ones) as a centre: the sums
 // over differences would meet 0 * inf, so such an output takes its sums over the flow.
@@ -925,11 +932,34 @@ __host__ __device__ inline size_t tri_smem_bytes(int s, int ty)
 }
 
 constexpr float TRI_FAR = 1e30f;
-// A sample times its scale; a finite one stays finite.
-__device__ __forceinline__ float tri_scaled(float k, float v)
+// A finite flow held where its scaled difference stays finite.
+__device__ __forceinline__ float tri_held(float v, float most)
 {
-    const float big = 3.402823466e38f, t = __fmul_rn(k, v);
-    return fabsf(t) > big && fabsf(v) <= big ? copysignf(big, t) : t;
+    return fabsf(v) > most && fabsf(v) <= 3.402823466e38f ? copysignf(most, v) : v;
+}
+
+// Exponent scales of the trilateral weights: exp(-d/(2 sigma2)) = exp2(-d * c)
+// with intensities divided by 255 folded into cI; kE, r and kI as trilateral_block has them.
+struct TriCoef {
+    float cE, cI, cS;
+    float kE, r, kI, cSr;   // cSr = cS / r
+    bool scaled;            // kE and r are ordinary numbers (cE is neither 0 nor infinite)
+};
+inline TriCoef tri_coef(float sigmaEPE2, float sigmaI2, float sigmaS2)
+{
+    const float LOG2E = 1.4426950408889634f;
+    TriCoef t;
+    t.cE = LOG2E / (2.0f * sigmaEPE2);
+    t.cI = LOG2E / (2.0f * sigmaI2 * 255.0f * 255.0f);
+    t.cS = LOG2E / (2.0f * sigmaS2);
+    t.scaled = t.cE > 0.0f && t.cE < 3.0e38f;
+    const double cE = t.scaled ? (double)t.cE : 1.0;
+    const double kE = __builtin_exp2(__builtin_rint(0.5 * __builtin_log2(cE))), r = cE / (kE * kE);
+    t.kE = (float)kE;
+    t.r = (float)r;
+    t.kI = (float)__builtin_sqrt((double)t.cI / r);
+    t.cSr = (float)((double)t.cS / r);
+    return t;
 }
 
 // 2^-x per half.  The negation is spelled without .ftz, which makes it a modifier of the
@@ -947,9 +977,10 @@ template <int TY, int G>
 __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, const float* __restrict__ V,
                                                  const float* Um, const float* Vm,
                                                  const float* __restrict__ I, float* __restrict__ Uo,
-                                                 float* __restrict__ Vo, int sx, int sy, int s, float kE, float kI,
-                                                 float cS, int bx0, int by0, float4* smem4)
+                                                 float* __restrict__ Vo, int sx, int sy, int s, const TriCoef& tc,
+                                                 int bx0, int by0, float4* smem4)
 {
+    const float kE = tc.kE, kI = tc.kI;
     const int TW = TX + 2 * s, TH = tri_rows(TY) + 2 * s, P = tri_pitch(s, TY);
     // row terms of pair p: outputs 0 (.x .y: rows 2p, 2p + 1) and 1 (.z .w: rows 2p - 1,
     // 2p); outputs 2 and 3 use pair p - 1's
@@ -958,6 +989,7 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
     float* sV = sU + TW * P;
     float* sI = sV + TW * P;
     const int x0 = bx0 - s, y0 = by0 - s;
+    const float most = kE > 1.0f ? 1e38f / kE : 3.402823466e38f;
     const int x = bx0 + threadIdx.x;
     const int yb = by0 + threadIdx.y * TRI_R;
     // (pixels outside the image compute on clamped centres and store nothing)
@@ -993,15 +1025,15 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
                 for (int h = 0; h < 2; h++)
                     if (r0 + k * STEP < TH && h < cols) {
                         const int at = (c0 + h * TX) * P + r0 + k * STEP;
-                        sU[at] = tri_scaled(kE, a[k][h]);
-                        sV[at] = tri_scaled(kE, b[k][h]);
-                        sI[at] = __fmul_rn(kI, i[k][h]);
+                        sU[at] = __fmul_rn(kE, tri_held(a[k][h], most));
+                        sV[at] = __fmul_rn(kE, tri_held(b[k][h], most));
+                        sI[at] = i[k][h];
                     }
         }
     }
     for (int p = threadIdx.y * TX + threadIdx.x; p <= s; p += TX * TY) {
         auto term = [&](int n) {
-            return n >= 0 && n < 2 * s ? (float)((n - s) * (n - s)) * cS : __int_as_float(0x7f800000);
+            return n >= 0 && n < 2 * s ? (float)((n - s) * (n - s)) * tc.cSr : __int_as_float(0x7f800000);
         };
         rowf[p] = make_float4(term(2 * p), term(2 * p + 1), term(2 * p - 1), term(2 * p));
     }
@@ -1009,13 +1041,14 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
 
 #pragma unroll
     for (int r = 0; r < TRI_R; r++) {
-        const float i0 = -sI[(threadIdx.x + s) * P + threadIdx.y * TRI_R + r + s];
+        const float i0 = __fmul_rn(-kI, sI[(threadIdx.x + s) * P + threadIdx.y * TRI_R + r + s]);
         ic[r] = pk2(i0, i0);
     }
     float su[TRI_R], sv[TRI_R], sw[TRI_R];
 #pragma unroll
     for (int r = 0; r < TRI_R; r++) su[r] = sv[r] = sw[r] = 0.0f;
 
+    const f2x kII = pk2(kI, kI), rr = pk2(tc.r, tc.r);
     struct Pair {
         f2x u, v, i;
     };
@@ -1034,8 +1067,8 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
             return t;
         };
         auto sums = [&](int r, const Pair& t, f2x row) {
-            const f2x du = add2(t.u, um[r]), dv = add2(t.v, vm[r]), dI = add2(t.i, ic[r]);
-            const f2x w = ex2n_2(fma2(dI, dI, fma2(dv, dv, fma2(du, du, row))));
+            const f2x du = add2(t.u, um[r]), dv = add2(t.v, vm[r]), dI = fma2(t.i, kII, ic[r]);
+            const f2x w = ex2n_2(mul2(fma2(dI, dI, fma2(dv, dv, fma2(du, du, row))), rr));
             au[r] = fma2(w, du, au[r]);
             av[r] = fma2(w, dv, av[r]);
             aw[r] = add2(aw[r], w);
@@ -1090,7 +1123,7 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
         t = load(s + 1);                              // row 2s + 2
         h = lower(t);
         sums(3, h, last);
-        const float wi = exp2f(-(float)(i * i) * cS);
+        const float wi = exp2f(-(float)(i * i) * tc.cS);
 #pragma unroll
         for (int r = 0; r < TRI_R; r++) {
             su[r] = __fmaf_rn(wi, lo2(au[r]) + hi2(au[r]), su[r]);
@@ -1153,54 +1186,32 @@ __device__ __forceinline__ void trilateral_block(const float* __restrict__ U, co
         const float mv = sv[r] + other_v[r];
         if (yb + r < sy) {
             const size_t o = (size_t)x + (size_t)(yb + r) * sx;
-            // sum of w u over max(1e-5, sum of w): with u = a + (d - e) / kE, a the centre, d
-            // the summed difference and e what the scaled centre was rounded by
-            auto quotient = [&](float centre, float neg, float m) {
-                const float e = __fmaf_rn(kE, centre, neg);
-                const bool none = w < 1e-5f;
-                const float q = __fdiv_rn(none ? __fmaf_rn(centre, w, __fmaf_rn(-e, w, m) * inv_k) : m, none ? 1e-5f : w);
-                return none ? q : __fmaf_rn(q - e, inv_k, centre);
+            // sum of w u over max(1e-5, sum of w), with u = centre + scaled difference / kE
+            auto quotient = [&](float centre, float m) {
+                return w < 1e-5f ? __fdiv_rn(__fmaf_rn(centre, w, m * inv_k), 1e-5f)
+                                 : __fmaf_rn(__fdiv_rn(m, w), inv_k, centre);
             };
-            float u = quotient(a[r], lo2(um[r]), mu), v = quotient(b[r], lo2(vm[r]), mv);
-            const bool far_u = fabsf(lo2(um[r])) > TRI_FAR, far_v = fabsf(lo2(vm[r])) > TRI_FAR;
-            if (far_u || far_v) {
+            float u = quotient(a[r], mu), v = quotient(b[r], mv);
+            if (fabsf(lo2(um[r])) > TRI_FAR || fabsf(lo2(vm[r])) > TRI_FAR) {
                 float fu = 0.0f, fv = 0.0f, fw = 0.0f;
 #pragma unroll 1
                 for (int k = 0; k < 4 * s * s; k++) {
                     const int i = k / (2 * s) - s, j = k % (2 * s) - s;
                     const size_t g = (size_t)min(sx - 1, max(0, x + i)) + (size_t)min(sy - 1, max(0, yb + r + j)) * sx;
-                    const float du = tri_scaled(kE, U[g]) + lo2(um[r]), dv = tri_scaled(kE, V[g]) + lo2(vm[r]);
-                    const float dI = __fmul_rn(kI, I[g]) + lo2(ic[r]);
-                    const float f = exp2f(-(du * du + dv * dv + dI * dI + (float)(i * i + j * j) * cS));
+                    const float du = __fmaf_rn(kE, U[g], lo2(um[r])), dv = __fmaf_rn(kE, V[g], lo2(vm[r]));
+                    const float dI = __fmaf_rn(kI, I[g], lo2(ic[r]));
+                    const float f = exp2f(-(tc.r * (du * du + dv * dv + dI * dI) + (float)(i * i + j * j) * tc.cS));
                     fu = __fmaf_rn(f, U[g], fu);
                     fv = __fmaf_rn(f, V[g], fv);
                     fw += f;
                 }
-                if (far_u) u = __fdiv_rn(fu, fmaxf(1e-5f, fw));
-                if (far_v) v = __fdiv_rn(fv, fmaxf(1e-5f, fw));
+                u = __fdiv_rn(fu, fmaxf(1e-5f, fw));
+                v = __fdiv_rn(fv, fmaxf(1e-5f, fw));
             }
             Uo[o] = u;
             Vo[o] = v;
         }
     }
-}
-
-// Exponent scales of the trilateral weights: exp(-d/(2 sigma2)) = exp2(-d * c)
-// with intensities divided by 255 folded into cI.
-struct TriCoef {
-    float cE, cI, cS;
-    float kE, kI;   // sqrt(cE), sqrt(cI)
-};
-inline TriCoef tri_coef(float sigmaEPE2, float sigmaI2, float sigmaS2)
-{
-    const float LOG2E = 1.4426950408889634f;
-    TriCoef t;
-    t.cE = LOG2E / (2.0f * sigmaEPE2);
-    t.cI = LOG2E / (2.0f * sigmaI2 * 255.0f * 255.0f);
-    t.cS = LOG2E / (2.0f * sigmaS2);
-    t.kE = (float)__builtin_sqrt((double)t.cE);
-    t.kI = (float)__builtin_sqrt((double)t.cI);
-    return t;
 }
 
 }  // namespace dev

@@ -531,13 +531,13 @@ __global__ void __launch_bounds__(TX * TY * G, 16 / (TY * G)) k_trilateral(const
                                                                        const float* Vm,
                                                                        const float* __restrict__ I,
                                                                        float* __restrict__ Uo, float* __restrict__ Vo,
-                                                                       int sx, int sy, int s, float kE, float kI, float cS)
+                                                                       int sx, int sy, int s,
+                                                                       const __grid_constant__ TriCoef tc)
 {
     chain_wait();
     chain_trigger();
     extern __shared__ float4 smem4[];
-    trilateral_block<TY, G>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, kE, kI, cS, blockIdx.x * TX, blockIdx.y * tri_rows(TY),
-                         smem4);
+    trilateral_block<TY, G>(U, V, Um, Vm, I, Uo, Vo, sx, sy, s, tc, blockIdx.x * TX, blockIdx.y * tri_rows(TY), smem4);
 }
 
 __global__ void __launch_bounds__(256) k_trilateral_global(const float* __restrict__ U, const float* __restrict__ V,
@@ -878,9 +878,9 @@ static int trilateral_rows(int sx, int sy, int s, int sms)
 // Half windows up to TRI_SMALL_S on a grid several waves deep take blocks of four warps
 // without the groups' exchange: a window this small is over before the next block's loads
 // arrive, so four blocks share an SM (with the medians, 1920x1080, s = 2, 4 and 8: 84, 122 and
-// 256 us by blocks of 8 rows, 66, 99 and 228 by these; s = 12: 467 and 439, where the larger
-// block is ahead from s = 16 on smaller frames).  A half window of 1 needs no tile: four taps
-// a pixel from memory, 42 us instead of 56.
+// 256 us by blocks of 8 rows, 66, 99 and 228 by these, 66, 103 and 242 with the exponent's
+// factor; s = 12: 467 and 439, where the larger block is ahead from s = 16 on smaller frames).
+// A half window of 1 needs no tile: four taps a pixel from memory, 42 us instead of 56.
 constexpr int TRI_SMALL_S = 8;
 
 cudaError_t trilateral(const float* U, const float* V, const float* Um, const float* Vm,
@@ -889,13 +889,13 @@ cudaError_t trilateral(const float* U, const float* V, const float* Um, const fl
 {
     const TriCoef tc = tri_coef(sigmaEPE2, sigmaI2, sigmaS2);
     const float cE = tc.cE, cI = tc.cI, cS = tc.cS;
-    if (s > 1 && s <= TRI_MAX_S) {
+    if (s > 1 && s <= TRI_MAX_S && tc.scaled) {
         cudaError_t e = ensure_trilateral_smem(s);
         if (e != cudaSuccess) return e;
         auto by_rows = [&](auto kernel, int ty, int groups) {
             dim3 g((sx + TX - 1) / TX, (sy + tri_rows(ty) - 1) / tri_rows(ty));
             return launch(kernel, g, dim3(TX, ty, groups), tri_smem_bytes(s, ty), chained, st, U, V, Um, Vm, I, Uo, Vo, sx,
-                          sy, s, tc.kE, tc.kI, cS);
+                          sy, s, tc);
         };
         int sms = 0;
         e = sm_count(&sms);
